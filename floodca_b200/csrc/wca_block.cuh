@@ -1,0 +1,750 @@
+// The FP32 step on column pairs for all-LAND grids, one CTA per row range.
+//
+// The same arithmetic as sweep_segment (FloodCA src/kernels/physics.h and
+// src/common/model.c:321-605), organised as passes of BLK_ROWS rows by a CTA
+// of BLK_ROWS warps. In a pass warp w holds row i = first + w of a strip of
+// 64 columns (two adjacent columns per lane, one packed f32x2 pair) and runs
+//
+//     A  the faces of row i (x) and between rows i-1 and i (y, diagonals)
+//     C  outflow and limiter of row i-1
+//     D  depth update of row i-2, hmax, tmax
+//     E  the next step's stable velocity of row i-3, when the pass has a
+//        candidate for it
+//
+// with a CTA barrier after A, C and D. What a phase leaves for other rows
+// (face discharges X, Y, E, W, limiter S, new level L) goes through shared
+// memory; the rows of z, h, n and hmax come by TMA, one tile a field and pass,
+// BLK_STAGES - 1 passes ahead.
+//
+// What bounds it, and why this split. A sweep in which each warp carries its
+// rows from A to E in registers needs every phase's state at once: 128
+// registers, 16 warps per SM, 709 warp instructions per 64-column row. With a
+// barrier between the phases each phase's registers die with it (64
+// registers, 32 warps per SM), the row ring is a fixed address distance
+// instead of register moves, and rows are shared by the CTA, so a range costs
+// six rows of halo per CTA instead of per warp. 446 warp instructions per row
+// at 64 % of the issue slots. Measured on a B200, microseconds a step, warm
+// grids, one warp per row range (before) and this: 4096^2 350 and 220, 2048^2
+// 112 and 70, 1024^2 51.5 and 27.8, 256^2 20.1 and 18.2, 1003 x 1498 with
+// K = 8 104 and 64. Bound by issue slots and the barriers; HBM is at 24 %.
+#pragma once
+
+#include <cstddef>
+
+#include "wca_f2.cuh"
+#include "wca_tma.cuh"
+
+namespace fcab {
+
+constexpr int BLK_ROWS = 8;                 // rows per pass = warps per CTA
+constexpr int BLK_THREADS = 32 * BLK_ROWS;
+constexpr int BLK_STAGES = 3;               // tile stages: the pass at work and those ahead
+constexpr uint32_t BLK_ROW_B = 256;         // bytes of a strip row
+
+// Shared memory, in bytes from a 1024-byte boundary. Tile stage: rows
+// first-2 .. first+7 of z, h, n and rows first-2 .. first+5 of hmax, so that a
+// warp's rows i, i-1, i-2 sit at fixed distances from one address. Rings: two
+// buffers per phase value, each of BLK_ROWS + 2 slots; warp w leaves its row
+// in slot w + 2 and finds the two rows above in slots w + 1 and w. The last
+// two warps write their rows to slots 0 and 1 of the other buffer as well,
+// where the next pass looks for them.
+constexpr uint32_t BLK_TILE_B = (BLK_ROWS + 2) * BLK_ROW_B;
+constexpr uint32_t BLK_Z = 0, BLK_H = BLK_TILE_B, BLK_N = 2 * BLK_TILE_B, BLK_M = 3 * BLK_TILE_B;
+constexpr uint32_t BLK_STAGE_B = 3 * BLK_TILE_B + BLK_ROWS * BLK_ROW_B;
+constexpr uint32_t BLK_RINGS = BLK_STAGES * BLK_STAGE_B;
+constexpr uint32_t BLK_X = 0, BLK_Y = BLK_TILE_B, BLK_S = 2 * BLK_TILE_B, BLK_L = 3 * BLK_TILE_B;
+constexpr uint32_t BLK_E = 4 * BLK_TILE_B, BLK_W = 5 * BLK_TILE_B;      // K = 8
+template <int K>
+__host__ __device__ constexpr uint32_t blk_buf()
+{
+    return (K == 8 ? 6 : 4) * BLK_TILE_B;
+}
+template <int K>
+__host__ __device__ constexpr uint32_t blk_tail()
+{
+    return BLK_RINGS + 2 * blk_buf<K>();
+}
+
+// Packed per-step constants. Products with a negated constant replace the
+// negations of the Newton and Markstein corrections.
+struct BlkK {
+    f2 dx, nrdx, dd, nrdd, w, A, nA, invA, gK, dt, rain;
+    f2 rden, nden;                      // RN(1/(2K dt)), -(2K dt)
+    float tau_l, tau_h;
+};
+
+// After the rings: what every thread of the CTA reads (so that no phase holds
+// it in registers) and the CTA's rare sums.
+template <typename AccT>
+struct BlkTail {
+    unsigned long long bar[BLK_STAGES];
+    BlkK c;
+    StepVals<float> sv;
+    AccT a_clamp, a_bnd;        // clamped volume, open-edge outflow
+    long long rain_cells;       // LAND output cells (uniform rain)
+    unsigned vmax;              // bits of the CTA's largest next-step velocity
+    int bad;
+    int unit[2];                // next unit of the CTA, by unit parity
+};
+template <int K>
+__host__ __device__ constexpr int blk_smem_bytes()
+{
+    return 1024 + (int)blk_tail<K>() + (int)sizeof(BlkTail<double>);
+}
+
+// Shared memory by 32-bit shared address.
+__device__ __forceinline__ f2 sld(uint32_t a)
+{
+    f2 v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v.u) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float slf(uint32_t a)
+{
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sst(uint32_t a, f2 v)
+{
+    asm volatile("st.shared.b64 [%0], %1;" ::"r"(a), "l"(v.u) : "memory");
+}
+// Sign changes and magnitudes by halves: packed instructions take the sign
+// change as an operand modifier.
+__device__ __forceinline__ f2 ng2(f2 a) { return mk2(-lo2(a), -hi2(a)); }
+__device__ __forceinline__ f2 ab2(f2 a) { return mk2(fabsf(lo2(a)), fabsf(hi2(a))); }
+// magnitude of a with the sign of s, one three-input logic operation a half
+__device__ __forceinline__ float csign(float a, float s)
+{
+    float r;
+    asm("lop3.b32 %0, %1, %2, 0x7fffffff, 0xe4;" : "=f"(r) : "f"(a), "f"(s));
+    return r;
+}
+// -(u*u) per half, rounded (scalar products: never contracted into a sum)
+__device__ __forceinline__ f2 nsq2(f2 u)
+{
+    return mk2(__fmul_rn(-lo2(u), lo2(u)), __fmul_rn(-hi2(u), hi2(u)));
+}
+// RN(a / c) given rc = RN(1/c), nc = -c (Markstein, as div2_mk)
+__device__ __forceinline__ f2 div2_c(f2 a, f2 rc, f2 nc)
+{
+    const f2 q = mul2(a, rc);
+    return fma2(fma2(q, nc, a), rc, q);
+}
+
+// hf^(2/3) per half as cbrt_sq2; `unsure` is raised when either half needs
+// the exact scalar function (cbrt_sq_rn).
+__device__ __forceinline__ f2 cbrt_sq2n(f2 hf, bool &unsure)
+{
+    const f2 l = lg2_2(hf);
+    const f2 u0 = ex2_2(mul2(l, bc2(0.333333343f)));
+    const f2 p = nsq2(u0);                                  // -s_hi
+    const f2 s_lo = fma2(u0, u0, p);
+    const f2 nr = fma2(ng2(s_lo), u0, fma2(p, u0, hf));     // hf - u0^3
+    const f2 c2 = mul2(nr, rcp_2(mul2(bc2(1.5f), p)));      // 2 (u0 - u)
+    const f2 t = fma2(ng2(u0), c2, s_lo);
+    const f2 y = sub2(t, p);
+    const f2 e = sub2(t, add2(p, y));
+    const f2 chk = fma2(e, bc2(1.00048828125f), y);
+    unsure = unsure || lo2(chk) != lo2(y) || hi2(chk) != hi2(y) || !(fabsf(lo2(l)) <= 20.0f) ||
+             !(fabsf(hi2(l)) <= 20.0f);
+    return y;
+}
+
+static __device__ __noinline__ float blk_cbrt(float hf) { return cbrt_sq_rn(hf); }
+static __device__ __noinline__ float blk_vcr(float g, float hf) { return sqrt_prod_rn(g, hf); }
+
+// One face pair between evaluation and use. A half that carries no flow
+// (|dL| < tau_l or hf < tau_h) continues with dL = 0 and hf = 1: it raises no
+// flag, and its volume cap is zero, so its discharge is.
+struct BlkFace {
+    f2 dL, hf, cb, v, rs;
+};
+
+// Faces a -> b in the steps of face2_v / face2_crit / face2_q (see there for
+// the formulas), on the constants at shared address kc (a BlkK).
+// blk_face_v: everything up to the factors of the Manning velocity
+// v * cb * rs = (1/nf) * hf^(2/3) * sqrt(S); `unsure`: a cube root of the lane
+// must be settled by the exact scalar function.
+template <int MATH>
+__device__ __forceinline__ BlkFace blk_face_v(f2 La, f2 Lb, f2 za, f2 zb, f2 na, f2 nb, f2 d,
+                                              f2 nrd, float tau_l, float tau_h, bool &unsure)
+{
+    BlkFace f;
+    const f2 dL = sub2(La, Lb);
+    const f2 hf = sub2(max2(La, Lb), max2(za, zb));
+    const bool live0 = fabsf(lo2(dL)) >= tau_l && lo2(hf) >= tau_h;
+    const bool live1 = fabsf(hi2(dL)) >= tau_l && hi2(hf) >= tau_h;
+    f.dL = sel2(live0, live1, dL, bc2(0.0f));
+    f.hf = sel2(live0, live1, hf, bc2(1.0f));
+    const f2 nf = max2(mul2(bc2(0.5f), add2(na, nb)), bc2(1e-12f));
+    if constexpr (MATH == MATH_EXACT) {
+        f.v = rcp_2(nf);
+        f.v = fma2(fma2(ng2(nf), f.v, bc2(1.0f)), f.v, f.v);
+        const f2 q = mul2(ab2(f.dL), nrd);                      // -RN(|dL| rd)
+        const f2 nS = fma2(fma2(q, d, ab2(f.dL)), nrd, q);      // -RN(|dL|/d)
+        const f2 y = rsqrt_2(ng2(nS));
+        const f2 s = mul2(nS, y);
+        f.rs = fma2(ng2(fma2(s, s, nS)), mul2(bc2(0.5f), y), ng2(s));
+        f.cb = cbrt_sq2n(f.hf, unsure);
+    } else {
+        const f2 S = mul2(ab2(f.dL), ng2(nrd));
+        f.rs = mul2(S, rsqrt_2(S));
+        f.cb = ex2_2(mul2(lg2_2(f.hf), bc2(0.666666687f)));
+        f.v = rcp_2(nf);
+    }
+    return f;
+}
+
+// v = (1/nf) cb sqrt(S); `crit`: a half may reach the critical velocity
+// sqrt(g hf) (a dead half's v is NaN and raises nothing)
+__device__ __forceinline__ void blk_face_m(BlkFace &f, f2 gK, bool &crit)
+{
+    f.v = mul2(mul2(f.v, f.cb), f.rs);
+    const f2 v2 = mul2(f.v, f.v);
+    // exact: v^2 < g hf (1 - 1e-6) leaves v surely below the critical velocity
+    const f2 pm = mul2(gK, f.hf);
+    crit = crit || lo2(v2) >= lo2(pm) || hi2(v2) >= hi2(pm);
+}
+
+// v = min(v, RN(sqrt(g hf))) on the halves that may exceed it
+template <int MATH>
+__device__ __forceinline__ void blk_face_crit(BlkFace &f, f2 gK, float g)
+{
+    const f2 v2 = mul2(f.v, f.v);
+    const f2 pm = mul2(gK, f.hf);
+    const bool cr0 = lo2(v2) >= lo2(pm), cr1 = hi2(v2) >= hi2(pm);
+    f2 vcr;
+    if constexpr (MATH == MATH_EXACT) {
+        bool u0, u1;
+        vcr = vcrit2(bc2(g), f.hf, u0, u1);
+        if (cr0 && u0)
+            vcr = mk2(blk_vcr(g, lo2(f.hf)), hi2(vcr));
+        if (cr1 && u1)
+            vcr = mk2(lo2(vcr), blk_vcr(g, hi2(f.hf)));
+    } else {
+        const f2 p = mul2(bc2(g), f.hf);
+        vcr = mul2(p, rsqrt_2(p));
+    }
+    f.v = sel2(cr0, cr1, min2(f.v, vcr), f.v);
+}
+
+// sign(dL) min(v hf w, RN(RN(|dL| A)/(2K dt))); caps: plus the number of
+// halves whose volume cap binds
+template <int MATH>
+__device__ __forceinline__ f2 blk_face_q(const BlkFace &f, f2 w, f2 A, f2 rden, f2 nden,
+                                         unsigned &caps)
+{
+    const f2 Qm = mul2(mul2(f.v, f.hf), w);
+    const f2 num = mul2(ab2(f.dL), A);
+    f2 Qc;
+    if constexpr (MATH == MATH_EXACT)
+        Qc = div2_c(num, rden, nden);
+    else
+        Qc = mul2(num, rden);
+    if (lo2(Qc) < lo2(Qm))
+        caps += 1u;
+    if (hi2(Qc) < hi2(Qm))
+        caps += 1u;
+    const f2 Q = min2(Qm, Qc);
+    return mk2(csign(lo2(Q), lo2(f.dL)), csign(hi2(Q), hi2(f.dL)));
+}
+
+// Q s of the upwind cell (s_down for Q < 0): one of the products is zero.
+__device__ __forceinline__ f2 upwind2(f2 Q, f2 s_up, f2 s_down)
+{
+    const f2 z0 = bc2(0.0f);
+    return fma2(min2(Q, z0), s_down, mul2(max2(Q, z0), s_up));
+}
+
+template <typename AccT, int K, int MATH, bool RAINF>
+struct BlockSweep {
+    using SS = StepSums<float, AccT>;
+    using Tail = BlkTail<AccT>;
+    static constexpr int NF = K == 8 ? 4 : 2;
+    static constexpr uint32_t TAIL = blk_tail<K>();
+    static constexpr uint32_t KC = TAIL + (uint32_t)offsetof(Tail, c);
+    static constexpr uint32_t SV = TAIL + (uint32_t)offsetof(Tail, sv);
+#define FCAB_KC(m) sld(sb + KC + (uint32_t)offsetof(BlkK, m))
+#define FCAB_SV(m) slf(sb + SV + (uint32_t)offsetof(StepVals<float>, m))
+
+    // Per-CTA state that persists over units: the count of tile passes so far
+    // decides stages, barrier parities and ring buffers.
+    struct Cta {
+        uint32_t sb;                // shared address of the CTA's memory (1024-byte aligned)
+        Tail *tail;
+        unsigned pass;
+    };
+
+    // Once per CTA: barriers, cleared rings (rows above a unit's first row
+    // are read, and their results dropped).
+    static __device__ __forceinline__ void init(Cta &T, char *sm)
+    {
+        T.sb = smem_addr(sm);
+        T.tail = reinterpret_cast<Tail *>(sm + TAIL);
+        T.pass = 0;
+        for (uint32_t o = BLK_RINGS + threadIdx.x * 16; o < TAIL; o += BLK_THREADS * 16)
+            *reinterpret_cast<uint4 *>(sm + o) = make_uint4(0u, 0u, 0u, 0u);
+        if (threadIdx.x == 0) {
+            for (int q = 0; q < BLK_STAGES; q++)
+                mbar_init1(smem_addr(&T.tail->bar[q]));
+            T.tail->bad = 0;
+            fence_proxy_async_smem();
+        }
+    }
+
+    // Once per step (one thread; a barrier follows): constants and sums.
+    static __device__ __forceinline__ void begin(Cta &T, const GridD<float> &g,
+                                                 const RunK<float> &rk, const Ctl *ctl)
+    {
+        Tail &t = *T.tail;
+        const StepVals<float> sv = step_vals<float, K>(g, rk, ctl);
+        const StepK<float> &k = sv.k;
+        t.sv = sv;
+        t.a_clamp = t.a_bnd = 0;
+        t.vmax = 0u;
+        t.rain_cells = 0;
+        BlkK &c = t.c;
+        c.dx = bc2(k.dx);
+        c.nrdx = bc2(-k.rdx);
+        c.dd = bc2(k.d_diag);
+        c.nrdd = bc2(-k.rdd);
+        c.w = bc2(k.w);
+        c.A = bc2(k.A);
+        c.nA = bc2(-k.A);
+        c.invA = bc2(k.inv_A);
+        c.gK = bc2(k.g * (MATH == MATH_EXACT ? 0.999999f : 1.0f));
+        c.dt = bc2(sv.dt);
+        c.rain = bc2(sv.rainv);
+        c.rden = bc2(k.rden);
+        c.nden = bc2(-k.den);
+        c.tau_l = k.tau_l;
+        c.tau_h = k.tau_h;
+    }
+
+    // one thread: the tiles of a pass (from row y0, two above the pass's
+    // first) into its stage
+    static __device__ __forceinline__ void issue(uint32_t sb, const CUtensorMap *tm,
+                                                 const CUtensorMap *th, int tx, int y0,
+                                                 unsigned pass)
+    {
+        const unsigned st = pass % BLK_STAGES;
+        const uint32_t bar = sb + TAIL + 8u * st, dst = sb + st * BLK_STAGE_B;
+        fence_proxy_async_smem();
+        mbar_arrive_tx(bar, BLK_STAGE_B);
+        tma_load_tile(dst + BLK_Z, tm, bar, tx, y0);
+        tma_load_tile(dst + BLK_H, th, bar, tx, y0);
+        tma_load_tile(dst + BLK_N, tm + 1, bar, tx, y0);
+        tma_load_tile(dst + BLK_M, tm + 4, bar, tx, y0);
+    }
+    // one thread: waits for the tiles of a pass
+    static __device__ __forceinline__ void arrived(const Cta &T, unsigned pass)
+    {
+        if (!mbar_wait_bounded(T.sb + TAIL + 8u * (pass % BLK_STAGES), (pass / BLK_STAGES) & 1u))
+            T.tail->bad = 1;
+    }
+    // a row of a phase value: into slot w + 2, and for the last two warps
+    // into the other buffer's slot w - 6 (`over`: the distance to it)
+    static __device__ __forceinline__ void keep(uint32_t at, f2 v, bool last2, uint32_t over)
+    {
+        sst(at + 2 * BLK_ROW_B, v);
+        if (last2)
+            sst(at + over, v);
+    }
+
+    // whether a row of the strip has open edges (all of its cells, or its end)
+    static __device__ __forceinline__ bool open_row(int edges, int r, int nr)
+    {
+        return (edges & 12) || (r == 0 && (edges & 1)) || (r == nr - 1 && (edges & 2));
+    }
+
+    // The velocity below which no cell can raise the step's maximum: the CTA's
+    // largest so far, or the seed; and the depth below which no cell reaches it
+    // (g h <= thr^2 (1 - 1e-6)).
+    static __device__ __forceinline__ float threshold(const Tail &t)
+    {
+        const float vm = __uint_as_float(*(const volatile unsigned *)&t.vmax);
+        return vm > t.sv.vseed ? vm : t.sv.vseed;
+    }
+    static __device__ __forceinline__ float height_cut(const Tail &t, float thr)
+    {
+        return fmaxf(thr * thr * 0.999998f * __frcp_rn(t.sv.k.g), t.sv.k.tau_h);
+    }
+
+    // Rows [r0, r1) of one strip, by the whole CTA. wp: the warp's index, as a
+    // warp-uniform value.
+    static __device__ __forceinline__ void run(Cta &T, const GridD<float> &g,
+                                               const RunK<float> &rk, int strip, int r0, int r1,
+                                               int wp, int lane, SS &ss)
+    {
+        using Gm = Geom<2>;
+        Tail &tl = *T.tail;
+        const uint32_t sb = T.sb;
+        const f2 z0 = bc2(0.0f);
+        const int nr = g.nr, nc = g.nc, pitch = (int)g.pitch;
+        const int c_first = strip * Gm::OW - Gm::HL;
+        const int cbase = c_first + lane * 2;
+        const bool out_lane = lane * 2 >= Gm::HL && lane * 2 < Gm::HL + Gm::OW;
+        // open edges (bit 0 north, 1 south, 2 west, 3 east) this strip has
+        const int edges = !rk.open ? 0
+                                   : (rk.edge_n ? 1 : 0) | (rk.edge_s ? 2 : 0) |
+                                         (rk.edge_w && c_first <= 0 ? 4 : 0) |
+                                         (rk.edge_e && c_first + Gm::SW > nc - 1 ? 8 : 0);
+        // strips with a column outside the grid, column 0 or nc-1, or the
+        // inflow cell: their rows take the special branches
+        const bool spec_strip = c_first <= 0 || c_first + Gm::SW > nc - 1 ||
+                                (rk.inflow_c >= c_first && rk.inflow_c < c_first + Gm::SW);
+        const int H = r1 - r0;
+        const int np = (H + 6 + BLK_ROWS - 1) / BLK_ROWS;           // passes
+        const CUtensorMap *tm = g.tmap;
+        const CUtensorMap *th = tm + (tl.sv.hin == g.h1 ? 3 : 2);
+        const int tx = c_first + PADC;                              // a multiple of 4 floats
+        const int ty = r0 - 5 + PADR;
+        const unsigned pass0 = T.pass;
+        if (wp == 0 && lane == 0) {
+            for (int b = 0; b < min(np, BLK_STAGES - 1); b++)
+                issue(sb, tm, th, tx, ty + b * BLK_ROWS, pass0 + b);
+            arrived(T, pass0);
+        }
+        float hcut = height_cut(tl, threshold(tl));
+        __syncthreads();
+
+        const bool last2 = wp >= BLK_ROWS - 2;
+        const uint32_t sl = sb + lane * 8 + wp * BLK_ROW_B;
+        uint32_t rb = sl + BLK_RINGS;                               // this pass's rings
+        uint32_t turn = blk_buf<K>();                               // to the other buffer
+        if (pass0 & 1u) {
+            rb += turn;
+            turn = 0u - turn;
+        }
+        uint32_t tb = sl + pass0 % BLK_STAGES * BLK_STAGE_B;        // this pass's tiles
+        const uint32_t tb_end = sl + BLK_STAGES * BLK_STAGE_B;
+        int rel = wp - 5;                   // row i-2 relative to r0
+        int off2 = (r0 + rel + PADR) * pitch + cbase + PADC;        // its element
+        bool prev_cand = false;
+
+        for (int b = 0; b < np; b++) {
+            if (wp == 0 && lane == 0 && b + BLK_STAGES - 1 < np)
+                // the stage's rows were last read in pass b-1, before its last barrier
+                issue(sb, tm, th, tx, ty + (b + BLK_STAGES - 1) * BLK_ROWS,
+                      pass0 + b + BLK_STAGES - 1);
+            const uint32_t over = turn - (BLK_ROWS - 2) * BLK_ROW_B;
+            const int r = r0 + rel;                                 // row i-2
+            const bool own2 = (unsigned)rel < (unsigned)H;          // written
+            // rows i-1, i-2 on or outside the grid's first and last rows
+            const bool spec = spec_strip || r < 1 || r + 2 >= nr;
+
+            // ---- A: x faces of row i; y (and diagonal) faces of rows i-1, i
+            f2 Y1, E1 = z0, W1 = z0;
+            {
+                const f2 z = sld(tb + BLK_Z + 2 * BLK_ROW_B), n = sld(tb + BLK_N + 2 * BLK_ROW_B);
+                const f2 L = add2(z, sld(tb + BLK_H + 2 * BLK_ROW_B));
+                const f2 zp = sld(tb + BLK_Z + BLK_ROW_B), npv = sld(tb + BLK_N + BLK_ROW_B);
+                const f2 Lp = add2(zp, sld(tb + BLK_H + BLK_ROW_B));
+                const f2 zr = right2(z), Lr = right2(L), nrr = right2(n);
+                const f2 dx = FCAB_KC(dx), nrdx = FCAB_KC(nrdx);
+                const float tau_l = slf(sb + KC + (uint32_t)offsetof(BlkK, tau_l));
+                const float tau_h = slf(sb + KC + (uint32_t)offsetof(BlkK, tau_h));
+                BlkFace f[NF];
+                bool unsure = false, crit = false;
+                f[0] = blk_face_v<MATH>(L, Lr, z, zr, n, nrr, dx, nrdx, tau_l, tau_h, unsure);
+                f[1] = blk_face_v<MATH>(Lp, L, zp, z, npv, n, dx, nrdx, tau_l, tau_h, unsure);
+                if constexpr (K == 8) {
+                    const f2 zpr = right2(zp), Lpr = right2(Lp), npr = right2(npv);
+                    const f2 dd = FCAB_KC(dd), nrdd = FCAB_KC(nrdd);
+                    f[2] = blk_face_v<MATH>(Lp, Lr, zp, zr, npv, nrr, dd, nrdd, tau_l, tau_h,
+                                            unsure);
+                    f[3] = blk_face_v<MATH>(Lpr, L, zpr, z, npr, n, dd, nrdd, tau_l, tau_h,
+                                            unsure);
+                }
+                if constexpr (MATH == MATH_EXACT) {
+                    if (__any_sync(0xffffffffu, unsure)) {
+                        if (unsure) {
+#pragma unroll
+                            for (int q = 0; q < NF; q++)
+                                f[q].cb = mk2(blk_cbrt(lo2(f[q].hf)), blk_cbrt(hi2(f[q].hf)));
+                        }
+                    }
+                }
+                const f2 gK = FCAB_KC(gK);
+#pragma unroll
+                for (int q = 0; q < NF; q++)
+                    blk_face_m(f[q], gK, crit);
+                if (__any_sync(0xffffffffu, crit)) {
+                    const float gr = FCAB_SV(k.g);
+#pragma unroll
+                    for (int q = 0; q < NF; q++)
+                        blk_face_crit<MATH>(f[q], gK, gr);
+                }
+                // volume caps are counted by the cell that holds the face: x
+                // faces by row i, the others by row i-1
+                unsigned cx = 0u, cy = 0u;
+                const f2 w = FCAB_KC(w), A = FCAB_KC(A), rden = FCAB_KC(rden), nden = FCAB_KC(nden);
+                const f2 X = blk_face_q<MATH>(f[0], w, A, rden, nden, cx);
+                Y1 = blk_face_q<MATH>(f[1], w, A, rden, nden, cy);
+                keep(rb + BLK_X, X, last2, over);
+                keep(rb + BLK_Y, Y1, last2, over);
+                if constexpr (K == 8) {
+                    E1 = blk_face_q<MATH>(f[2], w, A, rden, nden, cy);
+                    W1 = blk_face_q<MATH>(f[3], w, A, rden, nden, cy);
+                    keep(rb + BLK_E, E1, last2, over);
+                    keep(rb + BLK_W, W1, last2, over);
+                }
+                if ((unsigned)(rel + 2) < (unsigned)H)
+                    ss.capn += cx;
+                if ((unsigned)(rel + 1) < (unsigned)H)
+                    ss.capn += cy;
+            }
+            __syncthreads();
+
+            // ---- C: outflow volume and limiter of row i-1 (model.c:180-238,
+            //      489-502), in the reference order +x, -x, +y, -y, d1+, d1-,
+            //      d2+, d2-, open slots
+            f2 Y2, S1 = bc2(1.0f), E2 = z0, W2 = z0;
+            {
+                const f2 X1 = sld(rb + BLK_X + BLK_ROW_B);
+                Y2 = sld(rb + BLK_Y + BLK_ROW_B);
+                f2 out = sub2(max2(X1, z0), min2(left2(X1), z0));
+                out = add2(out, max2(Y1, z0));
+                out = sub2(out, min2(Y2, z0));
+                if constexpr (K == 8) {
+                    E2 = sld(rb + BLK_E + BLK_ROW_B);
+                    W2 = sld(rb + BLK_W + BLK_ROW_B);
+                    out = add2(out, max2(E1, z0));
+                    out = sub2(out, min2(left2(E2), z0));
+                    out = add2(out, max2(left2(W1), z0));
+                    out = sub2(out, min2(W2, z0));
+                }
+                const f2 hp = sld(tb + BLK_H + BLK_ROW_B);
+                if (spec && open_row(edges, r + 1, nr)) {
+                    const bool own = out_lane && (unsigned)(rel + 1) < (unsigned)H;
+                    const OpenFaces o = open_faces2(sld(tb + BLK_Z + BLK_ROW_B), hp,
+                                                    sld(tb + BLK_N + BLK_ROW_B), r + 1, cbase, nr,
+                                                    nc, g.r_lo, g.r_hi, edges, own, own,
+                                                    &tl.sv.k);
+                    ss.capn += o.cap;
+                    out = add2(out, o.add);
+                }
+                const f2 ov = mul2(out, FCAB_KC(dt));
+                const f2 hold = mul2(hp, FCAB_KC(A));
+                const f2 hz = max2(hold, z0);
+                const bool l0 = lo2(ov) > lo2(hz), l1 = hi2(ov) > hi2(hz);
+                if (__any_sync(0xffffffffu, l0 || l1)) {
+                    const f2 o = sel2(l0, l1, ov, bc2(1.0f));
+                    f2 q;
+                    if constexpr (MATH == MATH_EXACT)
+                        q = div2_mk(hold, o, rcp2_nr(o));
+                    else
+                        q = mul2(hold, rcp_2(o));
+                    S1 = sel2(l0, l1, q, S1);
+                }
+                keep(rb + BLK_S, S1, last2, over);
+            }
+            __syncthreads();
+
+            // ---- D: net inflow of row i-2 from the upwind-scaled
+            //      discharges, depth update, clamp, inflow, hmax and tmax
+            //      (model.c:511-597)
+            bool cand = false;
+            {
+                const f2 S2 = sld(rb + BLK_S + BLK_ROW_B), S3 = sld(rb + BLK_S);
+                const f2 sr = right2(S2);
+                const f2 Qsx = upwind2(sld(rb + BLK_X), S2, sr);
+                f2 net = sub2(left2(Qsx), Qsx);
+                net = sub2(net, upwind2(Y2, S2, S1));
+                net = add2(net, upwind2(sld(rb + BLK_Y), S3, S2));
+                if constexpr (K == 8) {
+                    net = sub2(net, upwind2(E2, S2, right2(S1)));
+                    net = add2(net, left2(upwind2(sld(rb + BLK_E), S3, sr)));
+                    net = sub2(net, left2(upwind2(W2, sr, S1)));
+                    net = add2(net, upwind2(sld(rb + BLK_W), right2(S3), S2));
+                }
+                const f2 h = sld(tb + BLK_H);
+                if (spec && open_row(edges, r, nr)) {
+                    // open-edge outflow scaled by the cell's own limiter
+                    // (model.c:553-559), summed over its open slots
+                    const OpenFaces o = open_faces2(sld(tb + BLK_Z), h, sld(tb + BLK_N), r, cbase,
+                                                    nr, nc, g.r_lo, g.r_hi, edges, false, false,
+                                                    &tl.sv.k);
+                    float qb[2];
+#pragma unroll
+                    for (int j = 0; j < 2; j++)
+                        qb[j] = open_sum<float>(get2(o.qo, j) * get2(S2, j),
+                                                __popc((o.ko >> (4 * j)) & 15u));
+                    net = sub2(net, mk2(qb[0], qb[1]));
+                    const float dt = FCAB_SV(dt);
+                    if (own2 && out_lane && (o.ko & 15u))
+                        atomicAdd(&tl.a_bnd, acc_mul<AccT, float>(dt, qb[0]));
+                    if (own2 && out_lane && (o.ko >> 4))
+                        atomicAdd(&tl.a_bnd, acc_mul<AccT, float>(dt, qb[1]));
+                }
+                f2 rain;
+                if constexpr (RAINF) {
+                    // rows r0-1 and r1 too: stage E reads their new levels
+                    rain = (unsigned)(rel + 1) <= (unsigned)(H + 1) ? ld2(g.cr + off2) : z0;
+                    rain = mul2_sep(rain, bc2(FCAB_SV(F)));
+                } else {
+                    rain = FCAB_KC(rain);
+                }
+                f2 dq;
+                if constexpr (MATH == MATH_EXACT)
+                    dq = div2_c(net, FCAB_KC(invA), FCAB_KC(nA));
+                else
+                    dq = mul2(net, FCAB_KC(invA));
+                f2 hu = add2(h, add2(mul2_sep(FCAB_KC(dt), dq), rain));
+                if (__any_sync(0xffffffffu, lo2(hu) < 0.0f || hi2(hu) < 0.0f)) {
+                    float a0 = lo2(hu), a1 = hi2(hu);
+                    const bool own = own2 && out_lane;
+                    const float A = FCAB_SV(A);
+                    if (a0 < 0.0f) {
+                        if (own && cbase >= 0 && cbase < nc)
+                            atomicAdd(&tl.a_clamp, acc_mul<AccT, float>(-a0, A));
+                        a0 = 0.0f;
+                    }
+                    if (a1 < 0.0f) {
+                        if (own && cbase + 1 >= 0 && cbase + 1 < nc)
+                            atomicAdd(&tl.a_clamp, acc_mul<AccT, float>(-a1, A));
+                        a1 = 0.0f;
+                    }
+                    hu = mk2(a0, a1);
+                }
+                const f2 z = sld(tb + BLK_Z);
+                f2 Ln = add2(z, hu);
+                if (spec) {
+                    const bool rin = r >= g.r_lo && r < g.r_hi;
+                    const bool in0 = rin && cbase >= 0 && cbase < nc;
+                    const bool in1 = rin && cbase + 1 >= 0 && cbase + 1 < nc;
+                    if (r == rk.inflow_r) {
+                        const int d = rk.inflow_c - cbase;
+                        const float dh = FCAB_SV(inflow_dh);
+                        if (d == 0)
+                            hu = mk2(lo2(hu) + dh, hi2(hu));
+                        else if (d == 1)
+                            hu = mk2(lo2(hu), hi2(hu) + dh);
+                        Ln = add2(z, hu);
+                    }
+                    // cells outside the grid: no level for stage E, no rain,
+                    // and they keep their padding depth of zero
+                    Ln = sel2(in0, in1, Ln, bc2(__int_as_float(0x7fc00000)));
+                    hu = sel2(in0, in1, hu, h);
+                    rain = sel2(in0, in1, rain, z0);
+                }
+                keep(rb + BLK_L, Ln, last2, over);
+                if (own2 && out_lane) {
+                    if constexpr (sizeof(AccT) == 4) {
+                        const float A = FCAB_SV(A);
+                        ss.a_rain += A * lo2(rain) + A * hi2(rain);
+                    } else if constexpr (RAINF) {
+                        ss.rain_sum += (double)lo2(rain) + (double)hi2(rain);
+                    }
+                    // a cell that could raise the velocity maximum
+                    cand = lo2(hu) >= hcut || hi2(hu) >= hcut;
+                    const f2 hm = sld(tb + BLK_M);                  // hmax of row i-2
+                    const uint64_t ho = sld(sb + SV + (uint32_t)offsetof(StepVals<float>, hout)).u;
+                    st2(reinterpret_cast<float *>(ho) + off2, hu);
+                    st2(g.hmax + off2, max2(hu, hm));
+                    float *const tmx = g.tmax + off2;
+                    const float tv = FCAB_SV(tmax_val);
+                    if (lo2(hu) > lo2(hm))
+                        tmx[0] = tv;
+                    if (hi2(hu) > hi2(hm))
+                        tmx[1] = tv;
+                }
+            }
+            if (wp == 0 && lane == 0 && b + 1 < np)
+                arrived(T, pass0 + b + 1);
+            const bool any_cand = __syncthreads_or(cand) != 0;
+
+            // ---- E: next step's stable velocity of row i-3 from the new
+            //      levels of rows i-4..i-2 (physics.h:158-217). A candidate
+            //      of this pass sits in rows i-3 of this pass or, for the
+            //      last warp's row, of the next one.
+            if (any_cand || prev_cand) {
+                const float thr = threshold(tl);
+                hcut = height_cut(tl, thr);
+                if (tl.sv.want_v && (unsigned)(rel - 1) < (unsigned)H)
+                    velocity_row(tl, g, sld(rb + BLK_L + BLK_ROW_B),
+                                 sld(rb + BLK_L + 2 * BLK_ROW_B), sld(rb + BLK_L), r - 1, cbase,
+                                 open_row(edges, r - 1, nr) ? edges : 0,
+                                 out_lane && cbase >= 0 && cbase < nc,
+                                 out_lane && cbase + 1 >= 0 && cbase + 1 < nc, off2 - pitch, thr,
+                                 hcut);
+            }
+            prev_cand = any_cand;
+
+            rb += turn;
+            turn = 0u - turn;
+            tb += BLK_STAGE_B;
+            if (tb == tb_end)
+                tb = sl;
+            rel += BLK_ROWS;
+            off2 += BLK_ROWS * pitch;
+        }
+        T.pass += np;
+        // uniform rain on LAND output cells
+        if constexpr (sizeof(AccT) == 8 && !RAINF) {
+            if (wp == 0 && lane == 0)
+                tl.rain_cells += (long long)H * (min(nc, c_first + Gm::HL + Gm::OW) -
+                                                 (c_first + Gm::HL));
+        }
+    }
+
+    // Stage E of one row: candidates are the output cells whose new depth
+    // reaches hcut; a multiply-only bound v^6 <= h^4 S^3 / n^6 against thr^6
+    // goes first, the exact velocity only where it could exceed thr.
+    static __device__ __forceinline__ void velocity_row(Tail &tl, const GridD<float> &g, f2 la,
+                                                        f2 lb, f2 lt, int r, int cbase, int edges,
+                                                        bool in0, bool in1, int off, float thr,
+                                                        float hcut)
+    {
+        const StepVals<float> &sv = tl.sv;
+        const f2 z0 = bc2(0.0f);
+        f2 mo = max2(abs2(sub2(la, right2(la))), abs2(sub2(la, left2(la))));
+        mo = max2(mo, max2(abs2(sub2(la, lb)), abs2(sub2(la, lt))));
+        mo = max2(mo, z0);
+        f2 md = z0;
+        if constexpr (K == 8) {
+            md = max2(abs2(sub2(la, right2(lb))), abs2(sub2(la, left2(lb))));
+            md = max2(md, max2(abs2(sub2(la, right2(lt))), abs2(sub2(la, left2(lt)))));
+            md = max2(md, z0);
+        }
+        // a candidate's new depth was stored by this CTA before the last barrier
+        const f2 hv = in0 || in1 ? ld2_rw(sv.hout + off) : z0;
+        const bool e0 = in0 && lo2(hv) >= hcut, e1 = in1 && hi2(hv) >= hcut;
+        if (!(e0 || e1))
+            return;
+        if (edges) {
+            // the open virtual neighbour z - S_bnd*dx, h = 0 (physics.h:183-189)
+            const bool erow = (r == 0 && (edges & 1)) || (r == g.nr - 1 && (edges & 2));
+            const f2 zz = ld2(g.z + off);
+            const f2 dv = abs2(sub2(la, sub2(zz, bc2(sv.k.S_bnd * sv.k.dx))));
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int cc = cbase + j;
+                if (erow || (cc == 0 && (edges & 4)) || (cc == g.nc - 1 && (edges & 8)))
+                    put2(mo, j, fmaxf(get2(mo, j), get2(dv, j)));
+            }
+        }
+        const f2 nv = ld2(g.n + off);
+        const f2 n2 = mul2(nv, nv);
+        f2 S = mul2(mo, bc2(sv.k.rdx));
+        if constexpr (K == 8)
+            S = max2(S, mul2(md, bc2(sv.k.rdd)));
+        const f2 h2 = mul2(hv, hv);
+        const f2 lhs = mul2(mul2(h2, h2), mul2(mul2(S, S), S));
+        const float t2 = thr * thr;
+        // 0 when thr < 1e-6: every velocity is at least 1e-6 (physics.h:214-216)
+        const float T6 = thr >= 1e-6f ? t2 * t2 * t2 * 0.9998f : 0.0f;
+        const f2 rhs = mul2(mul2(mul2(n2, n2), n2), bc2(T6));
+        const bool x0 = e0 && (lo2(lhs) >= lo2(rhs) || lo2(lhs) < 1e-30f);
+        const bool x1 = e1 && (hi2(lhs) >= hi2(rhs) || hi2(lhs) < 1e-30f);
+        if (x0 || x1) {
+            const float vm = pair_velocity<K, MATH>(0.0f, x0, x1, mo, md, hv, nv, &sv.k);
+            atomicMax(&tl.vmax, __float_as_uint(vm));
+        }
+    }
+#undef FCAB_KC
+#undef FCAB_SV
+};
+
+}  // namespace fcab

@@ -16,12 +16,14 @@ struct VariantKey {
     int math;   // MATH_*
     int rainf;  // per-cell rain field
     int landonly; // every cell LAND (mask not read, padding at PAD_Z)
+    int blk = 0;  // FP32 all-LAND: the block sweep (needs the session's row maps)
 };
 
 // Type-erased launchers; `g`, `rk` point at GridD<T>/RunK<T> of the variant's T.
 struct Launchers {
-    cudaError_t (*step)(const void *g, const void *rk, const TimeCfg &tc, Ctl *ctl,
-                        int warps_total, int grid, cudaStream_t s, int smem);
+    // split: warps of the whole grid (sweeps by warp), or rows of a unit (block sweep)
+    cudaError_t (*step)(const void *g, const void *rk, const TimeCfg &tc, Ctl *ctl, int split,
+                        int grid, cudaStream_t s, int smem);
     // full velocity pass + step control: the first step's dt, or
     // (only_if_needed) a dt deferred by a step whose pruned maximum fell
     // below its seed
@@ -30,6 +32,7 @@ struct Launchers {
     const void *step_fn;   // __global__ symbol, for occupancy queries
     int threads;           // threads per CTA of the step kernel
     int tma_smem;          // dynamic shared memory of its TMA row source (0: none)
+    int blk;               // the block sweep: `grid` CTAs share the rows
 };
 
 // Batched-ensemble launchers (FP32 state, FP64 accumulation).
@@ -104,6 +107,30 @@ Launchers make_launchers()
     L.step_fn = (const void *)&k_step<T, AccT, K, CPL, MATH, RAINF, LAND>;
     L.threads = step_threads<CPL, MATH>();
     L.tma_smem = use_pair_sweep<T, K, CPL, LAND>() ? tma_smem_bytes(L.threads / 32) : 0;
+    L.blk = 0;
+    return L;
+}
+
+template <typename AccT, int K, int MATH, bool RAINF>
+cudaError_t launch_step_blk(const void *g, const void *rk, const TimeCfg &tc, Ctl *ctl, int seg,
+                            int grid, cudaStream_t s, int smem)
+{
+    k_step_blk<AccT, K, MATH, RAINF><<<grid, BLK_THREADS, smem, s>>>(
+        *static_cast<const GridD<float> *>(g), *static_cast<const RunK<float> *>(rk), tc, ctl,
+        seg);
+    return cudaGetLastError();
+}
+
+template <typename AccT, int K, int MATH, bool RAINF>
+Launchers make_launchers_blk()
+{
+    Launchers L;
+    L.step = &launch_step_blk<AccT, K, MATH, RAINF>;
+    L.init = &launch_init<float, K, MATH>;
+    L.step_fn = (const void *)&k_step_blk<AccT, K, MATH, RAINF>;
+    L.threads = BLK_THREADS;
+    L.tma_smem = blk_smem_bytes<K>();
+    L.blk = 1;
     return L;
 }
 
@@ -111,6 +138,17 @@ Launchers make_launchers()
 template <typename T, typename AccT, int MATH>
 bool lookup_kcr(const VariantKey &k, Launchers *out)
 {
+    if constexpr (sizeof(T) == 4) {
+        if (k.blk && k.landonly) {
+            if (k.K == 4)
+                *out = k.rainf ? make_launchers_blk<AccT, 4, MATH, true>()
+                               : make_launchers_blk<AccT, 4, MATH, false>();
+            else
+                *out = k.rainf ? make_launchers_blk<AccT, 8, MATH, true>()
+                               : make_launchers_blk<AccT, 8, MATH, false>();
+            return true;
+        }
+    }
 #define FCAB_CASE(KK, CC, RR)                                                    \
     if (k.K == KK && k.cpl == CC && (k.rainf != 0) == RR) {                      \
         *out = k.landonly ? make_launchers<T, AccT, KK, CC, MATH, RR, true>()   \

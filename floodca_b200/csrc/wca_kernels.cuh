@@ -100,6 +100,7 @@ struct Ctl {
     // velocity seed of the next step's dt pruning (float or double bits, 0:
     // none) and the deferred-dt handshake with the full velocity pass
     unsigned long long vseed_bits;
+    unsigned int next_unit;     // block sweep: units handed out beyond the first per CTA
     int need_v;                 // the step's pruned maximum fell below the seed
     int pause_carry;            // progress pause decided before the deferral
     long long full_passes;      // deferred dts completed by the full pass
@@ -1147,6 +1148,7 @@ __device__ __forceinline__ void publish_sums(StepSums<T, AccT> &ss, const StepVa
 
 #include "wca_sweep_f2.cuh"
 #include "wca_sweep_f4.cuh"
+#include "wca_block.cuh"
 
 namespace fcab {
 
@@ -1247,11 +1249,112 @@ __host__ __device__ constexpr int step_blocks_per_sm()
                      : step_min_blocks<K, CPL, MATH>();
 }
 
+// Resident CTAs of the block sweep the register allocation aims for.
+#ifndef FCAB_BLK_CTAS
+#define FCAB_BLK_CTAS 4
+#endif
+#ifndef FCAB_BLK_CTAS_K8
+#define FCAB_BLK_CTAS_K8 3
+#endif
+template <int K>
+__host__ __device__ constexpr int blk_ctas_per_sm()
+{
+    return K == 8 ? FCAB_BLK_CTAS_K8 : FCAB_BLK_CTAS;
+}
+
 template <typename T, int K, int MATH>
 __global__ void k_init_dt(GridD<T> g, RunK<T> rk, TimeCfg tc, Ctl *ctl, int only_if_needed);
 
 // CTAs of the full velocity pass (grid-stride over every cell; 256 threads)
 constexpr int VPASS_GRID = 148 * 8;
+
+// ---- the last CTA to finish prepares the next step
+template <typename T, int K, int MATH>
+__device__ __forceinline__ void step_tail(const GridD<T> &g, const RunK<T> &rk, const TimeCfg &tc,
+                                          Ctl *ctl)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned prev = atomicAdd(&ctl->ctas_done, 1u);
+        if (prev == gridDim.x - 1) {
+            __threadfence();
+            ctl->h_cur ^= 1;
+            ctl->launches += 1;
+            ctl->next_unit = 0u;
+            if (tc.split) {
+                ctl->fin_pending = 1;
+                ctl->ctas_done = 0u;
+            } else {
+                finalize<T>(ctl, tc, rk, true);
+                // a missed seed defers this step's dt to the full velocity
+                // pass: launched from here into the tail of the stream, so
+                // it runs before the next step and only when needed
+                if (tc.tail_vpass && ctl->need_v) {
+                    k_init_dt<T, K, MATH><<<VPASS_GRID, 256, 0, cudaStreamTailLaunch>>>(g, rk, tc,
+                                                                                      ctl, 1);
+                    if (cudaGetLastError() != cudaSuccess)
+                        ctl->err = 2;   // the host's poll runs the pass instead
+                }
+            }
+        }
+    }
+}
+
+// The block sweep's step: CTAs take units of `seg` rows of a strip.
+template <typename AccT, int K, int MATH, bool RAINF>
+__global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
+    k_step_blk(GridD<float> g, RunK<float> rk, TimeCfg tc, Ctl *ctl, int seg)
+{
+    using Sweep = BlockSweep<AccT, K, MATH, RAINF>;
+    using G = Geom<2>;
+    if (ctl->active == 0)
+        return;
+    extern __shared__ __align__(1024) unsigned char fcab_dsm[];
+    char *const sm = reinterpret_cast<char *>(fcab_dsm) +
+                     ((1024u - (smem_addr(fcab_dsm) & 1023u)) & 1023u);
+    int lane;       // volatile: held in a register, not read again from the special register
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+    StepSums<float, AccT> ss;
+    typename Sweep::Cta T;
+    Sweep::init(T, sm);
+    if (threadIdx.x == 0) {
+        Sweep::begin(T, g, rk, ctl);
+        fence_proxy_async_smem();
+    }
+    __syncthreads();
+    // units of `seg` rows of a strip, taken from the step's counter (the first
+    // one by the CTA's index)
+    const int nr = g.nr, nstrips = (g.nc + G::OW - 1) / G::OW;
+    const int nblk = (nr + seg - 1) / seg, units = nstrips * nblk;
+    const int wp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    int par = 0;
+    for (int u = blockIdx.x; u < units; par ^= 1) {
+        if (threadIdx.x == 0)
+            T.tail->unit[par] = units > (int)gridDim.x
+                                    ? (int)(gridDim.x + atomicAdd(&ctl->next_unit, 1u))
+                                    : units;
+        const int r0 = u % nblk * seg;
+        Sweep::run(T, g, rk, u / nblk, r0, min(nr, r0 + seg), wp, lane, ss);
+        __syncthreads();
+        u = T.tail->unit[par];
+    }
+    // halo lanes evaluate faces that other strips own
+    if (!(lane * 2 >= G::HL && lane * 2 < G::HL + G::OW))
+        ss.capn = 0u;
+    if (threadIdx.x == 0) {
+        if (T.tail->bad)
+            ctl->err = 3;           // a row tile never arrived; the host reports it
+        ss.a_clamp = T.tail->a_clamp;
+        ss.a_bnd = T.tail->a_bnd;
+        ss.vmax = __uint_as_float(T.tail->vmax);
+        ss.rain_cells = T.tail->rain_cells;
+    }
+    const StepVals<float> &sv = T.tail->sv;
+    publish_sums<float, AccT, RAINF>(ss, sv, ctl, lane,
+                                     (int)((blockIdx.x * BLK_ROWS + wp) & (NSLOT - 1)));
+    step_tail<float, K, MATH>(g, rk, tc, ctl);
+}
 
 template <typename T, typename AccT, int K, int CPL, int MATH, bool RAINF, bool LANDONLY>
 __global__ void __launch_bounds__(step_threads<CPL, MATH>(),
@@ -1333,32 +1436,7 @@ __global__ void __launch_bounds__(step_threads<CPL, MATH>(),
     }
 
     publish_sums<T, AccT, RAINF>(ss, sv, ctl, lane, wid & (NSLOT - 1));
-    // ---- the last CTA to finish prepares the next step
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned prev = atomicAdd(&ctl->ctas_done, 1u);
-        if (prev == gridDim.x - 1) {
-            __threadfence();
-            ctl->h_cur ^= 1;
-            ctl->launches += 1;
-            if (tc.split) {
-                ctl->fin_pending = 1;
-                ctl->ctas_done = 0u;
-            } else {
-                finalize<T>(ctl, tc, rk, true);
-                // a missed seed defers this step's dt to the full velocity
-                // pass: launched from here into the tail of the stream, so
-                // it runs before the next step and only when needed
-                if (tc.tail_vpass && ctl->need_v) {
-                    k_init_dt<T, K, MATH><<<VPASS_GRID, 256, 0, cudaStreamTailLaunch>>>(g, rk, tc,
-                                                                                      ctl, 1);
-                    if (cudaGetLastError() != cudaSuccess)
-                        ctl->err = 2;   // the host's poll runs the pass instead
-                }
-            }
-        }
-    }
+    step_tail<T, K, MATH>(g, rk, tc, ctl);
 }
 
 // --------------------------------------------------------------------------

@@ -146,21 +146,23 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
     return fn;
 }
 
-// Row-tile maps of the padded FP32 fields z, n, h0, h1 for the pair sweep's
-// TMA row source: 2-D [rows][pitch] floats, boxes of 64 columns x TMA_RB
-// rows; rows past the array read as zeros (never used).
+// Row-tile maps of the padded FP32 fields z, n, h0, h1, hmax for the block
+// sweep: 2-D [rows][pitch] floats, boxes of 64 columns and the rows of a pass
+// (z, n, h: and two more above); rows past the array read as zeros (never
+// used).
 bool make_row_maps(FcabSim *s)
 {
     auto fn = tensor_map_encoder();
     if (!fn || s->esize != 4)
         return false;
-    CUtensorMap maps[4];
-    const void *fields[4] = {s->z, s->n, s->h0, s->h1};
+    CUtensorMap maps[5];
+    const void *fields[5] = {s->z, s->n, s->h0, s->h1, s->hmax};
     cuuint64_t dims[2] = {(cuuint64_t)s->pitch, (cuuint64_t)s->rows_alloc};
     cuuint64_t strides[1] = {(cuuint64_t)s->pitch * 4};
-    cuuint32_t box[2] = {64, (cuuint32_t)TMA_RB};
+    cuuint32_t box[2] = {64, 0};
     cuuint32_t es[2] = {1, 1};
-    for (int q = 0; q < 4; q++) {
+    for (int q = 0; q < 5; q++) {
+        box[1] = q == 4 ? (cuuint32_t)BLK_ROWS : (cuuint32_t)BLK_ROWS + 2;
         if (((uintptr_t)fields[q] & 15) ||
             fn(&maps[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, (void *)fields[q], dims, strides, box,
                es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -172,14 +174,6 @@ bool make_row_maps(FcabSim *s)
         return false;
     return cudaMemcpyAsync(s->tmaps, maps, sizeof(maps), cudaMemcpyHostToDevice, s->stream) ==
            cudaSuccess;
-}
-
-// Row source of the FP32 pair sweep: FCAB_ROW_SOURCE=tma streams rows by
-// TMA into shared memory, anything else (the default) by plain loads.
-bool want_tma_rows()
-{
-    const char *e = getenv("FCAB_ROW_SOURCE");
-    return e && strcmp(e, "tma") == 0;
 }
 
 }  // namespace
@@ -297,6 +291,35 @@ long long fcab::step_warps(const FcabConfig &c, int cpl, int nsm, int per_sm, in
     return warps < 1 ? 1 : warps;
 }
 
+int fcab::blk_seg(const FcabConfig &c, int nsm, int per_sm)
+{
+    if (c.seg_rows > 0)
+        return c.seg_rows;
+    // One unit per CTA in one wave, blocks per strip chosen by the passes a
+    // unit takes (its rows and six halo rows, BLK_ROWS a pass) times what a
+    // pass costs with that many CTAs on an SM. Measured on a B200: a pass
+    // takes about 1.4, 1.9, 2.5 and 3.0 us with 1..4 CTAs per SM.
+    const long long strips = (c.ncols + Geom<2>::OW - 1) / Geom<2>::OW;
+    const long long slots = (long long)nsm * (per_sm > 0 ? per_sm : 1);
+    if (strips > slots) {
+        // more strips than CTAs: about four units a CTA from the step's queue
+        const long long nb = (4 * slots + strips - 1) / strips;
+        return (int)((c.nrows + nb - 1) / nb);
+    }
+    double best = 0.0;
+    long long best_seg = c.nrows;
+    for (long long nb = 1; nb * strips <= slots && nb <= c.nrows; nb++) {
+        const long long seg = (c.nrows + nb - 1) / nb;
+        const long long per = (strips * nb + nsm - 1) / nsm;
+        const double cost = (double)((seg + 6 + BLK_ROWS - 1) / BLK_ROWS) * (0.8 + 0.55 * per);
+        if (nb == 1 || cost < best) {
+            best = cost;
+            best_seg = seg;
+        }
+    }
+    return (int)best_seg;
+}
+
 // Rejects configurations the step cannot run: unknown enumerations, a dt
 // reuse count below 1, non-positive or non-finite cell size, gravity,
 // Courant factor or dt bounds (a zero dt never advances the clock), negative
@@ -393,7 +416,7 @@ extern "C" int fcab_sim_create(FcabSim **out, const FcabConfig *cfg, void *strea
         fcab_sim_destroy(s);
         return fail(FCAB_ERR_CUDA, "allocation: %s", cudaGetErrorString(e));
     }
-    if (cfg->precision != FCAB_PREC_F64 && want_tma_rows())
+    if (cfg->precision != FCAB_PREC_F64)
         s->use_tma = make_row_maps(s);
     if (cfg->precision == FCAB_PREC_F64)
         fill_runk<double>(s->rkd, *cfg);
@@ -678,6 +701,12 @@ static int resolve_variant(FcabSim *s)
     if (s->esize == 4 && key.landonly && (key.cpl == 2 || key.cpl == 4) &&
         (long long)(s->cfg.nrows + s->hn + s->hs + 2 * PADR) * s->pitch >= (1ll << 31))
         key.cpl = s->cpl = 1;
+    // FP32 all-LAND grids run the block sweep (two columns per lane) unless
+    // one or four columns per lane are asked for
+    key.blk = s->use_tma && key.landonly && (key.cpl == 2 || s->cfg.cols_per_lane == 0) &&
+              (long long)(s->cfg.nrows + s->hn + s->hs + 2 * PADR) * s->pitch < (1ll << 31);
+    if (key.blk)
+        key.cpl = s->cpl = 2;
     bool ok = key.prec == FCAB_PREC_F32 ? lookup_f32(key, &s->L)
               : key.prec == FCAB_PREC_F32_ALL ? lookup_f32all(key, &s->L)
                                                : lookup_f64(key, &s->L);
@@ -696,7 +725,15 @@ static int resolve_variant(FcabSim *s)
     if (per_sm < 1)
         per_sm = 1;
     const int wpb = s->L.threads / 32;     // warps per CTA
-    s->grid = (int)((step_warps(s->cfg, s->cpl, nsm, per_sm, wpb) + wpb - 1) / wpb);
+    if (s->L.blk) {
+        s->split = blk_seg(s->cfg, nsm, per_sm);
+        const long long units = (long long)((s->cfg.ncols + Geom<2>::OW - 1) / Geom<2>::OW) *
+                                ((s->cfg.nrows + s->split - 1) / s->split);
+        s->grid = (int)std::min<long long>(units, (long long)nsm * per_sm);
+    } else {
+        s->grid = (int)((step_warps(s->cfg, s->cpl, nsm, per_sm, wpb) + wpb - 1) / wpb);
+        s->split = s->grid * wpb;
+    }
     s->warps_total = s->grid * wpb;
     s->occupancy = per_sm;
     if (s->graph) {
@@ -746,7 +783,7 @@ static cudaError_t launch_one(FcabSim *s)
     if (s->esize == 8) {
         GridD<double> g;
         grid_view(s, g);
-        e = s->L.step(&g, &s->rkd, s->tc, s->ctl, s->warps_total, s->grid, s->stream,
+        e = s->L.step(&g, &s->rkd, s->tc, s->ctl, s->split, s->grid, s->stream,
                       step_smem(s));
         if (e == cudaSuccess && s->tc.vseed_on && !s->tc.tail_vpass)
             e = s->L.init(&g, &s->rkd, s->tc, s->ctl, full_grid, s->stream, 1);
@@ -754,7 +791,7 @@ static cudaError_t launch_one(FcabSim *s)
     }
     GridD<float> g;
     grid_view(s, g);
-    e = s->L.step(&g, &s->rkf, s->tc, s->ctl, s->warps_total, s->grid, s->stream,
+    e = s->L.step(&g, &s->rkf, s->tc, s->ctl, s->split, s->grid, s->stream,
                   step_smem(s));
     if (e == cudaSuccess && s->tc.vseed_on && !s->tc.tail_vpass)
         e = s->L.init(&g, &s->rkf, s->tc, s->ctl, full_grid, s->stream, 1);
@@ -1224,12 +1261,12 @@ extern "C" int fcab_sim_slab_step(FcabSim *s)
     if (s->esize == 8) {
         GridD<double> g;
         grid_view(s, g);
-        CUDA_TRY(s->L.step(&g, &s->rkd, s->tc, s->ctl, s->warps_total, s->grid, s->stream,
+        CUDA_TRY(s->L.step(&g, &s->rkd, s->tc, s->ctl, s->split, s->grid, s->stream,
                            step_smem(s)));
     } else {
         GridD<float> g;
         grid_view(s, g);
-        CUDA_TRY(s->L.step(&g, &s->rkf, s->tc, s->ctl, s->warps_total, s->grid, s->stream,
+        CUDA_TRY(s->L.step(&g, &s->rkf, s->tc, s->ctl, s->split, s->grid, s->stream,
                            step_smem(s)));
     }
     s->launches += 1;

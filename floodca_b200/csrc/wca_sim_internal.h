@@ -22,14 +22,15 @@ struct FcabSim {
     fcab::Ctl *ctl = nullptr;    // device control block
     void *ctl_host = nullptr;    // pinned mirror
     void *scratch = nullptr;     // 64 bytes of device scratch
-    void *tmaps = nullptr;       // row-tile tensor maps of z, n, h0, h1 (device memory)
-    bool use_tma = false;        // FP32 pair sweep rows by TMA
+    void *tmaps = nullptr;       // row-tile tensor maps of z, n, h0, h1, hmax (device memory)
+    bool use_tma = false;        // the FP32 fields have row maps (block sweep)
     fcab::RunK<float> rkf;
     fcab::RunK<double> rkd;
     fcab::TimeCfg tc;
     bool rain_field = false;
     bool landonly = false;       // mask-free kernel variant (all cells LAND)
     int cpl = 2, grid = 1, warps_total = 4, occupancy = 1;
+    int split = 4;               // how the grid shares the rows (Launchers::step)
     fcab::Launchers L;
     bool have_variant = false, variant_dirty = true;
     cudaGraphExec_t graph = nullptr;
@@ -55,6 +56,8 @@ int pick_cpl(const FcabConfig &c);
 // per_sm CTAs of wpb warps) with segments of cfg.seg_rows rows when set,
 // else an even split, at least 4 rows per warp (wca_sim.cu).
 long long step_warps(const FcabConfig &c, int cpl, int nsm, int per_sm, int wpb);
+// Rows of a work unit of the block sweep (cfg.seg_rows when set).
+int blk_seg(const FcabConfig &c, int nsm, int per_sm);
 // Run constants of an FP32 configuration (defined in wca_sim.cu).
 void make_run_params_f32(const FcabConfig &cfg, RunK<float> *rk, TimeCfg *tc);
 // Row-block copies between dense pageable host rows and pitched device rows
