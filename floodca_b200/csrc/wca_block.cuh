@@ -40,8 +40,13 @@ constexpr int BLK_ROWS = 8;                 // rows per pass = warps per CTA
 constexpr int BLK_THREADS = 32 * BLK_ROWS;
 constexpr int BLK_STAGES = 3;               // tile stages: the pass at work and those ahead
 constexpr uint32_t BLK_ROW_B = 256;         // bytes of a strip row
+// Cells up to which the step's last CTA does a missed seed's velocity pass
+// alone: it reads the depths (4 B a cell) and evaluates the few cells deep
+// enough to matter. One step in a hundred needs it; a launch that could
+// launch the pass costs 1.3 us on every step.
+constexpr long long BLK_SOLO = 1ll << 18;
 
-// Shared memory, in bytes from a 1024-byte boundary. Tile stage: rows
+// Shared memory, in bytes from a 128-byte boundary. Tile stage: rows
 // first-2 .. first+7 of z, h, n and rows first-2 .. first+5 of hmax, so that a
 // warp's rows i, i-1, i-2 sit at fixed distances from one address. Rings: two
 // buffers per phase value, each of BLK_ROWS + 2 slots; warp w leaves its row
@@ -80,8 +85,10 @@ struct BlkTail {
     unsigned long long bar[BLK_STAGES];
     BlkK c;
     StepVals<float> sv;
-    AccT a_clamp, a_bnd;        // clamped volume, open-edge outflow
+    TimePre pre;
+    AccT a_clamp, a_bnd, a_rain;    // clamped volume, open-edge outflow, rain
     long long rain_cells;       // LAND output cells (uniform rain)
+    unsigned cap;               // faces whose volume cap bound
     unsigned vmax;              // bits of the CTA's largest next-step velocity
     int bad;
     int unit[2];                // next unit of the CTA, by unit parity
@@ -89,7 +96,7 @@ struct BlkTail {
 template <int K>
 __host__ __device__ constexpr int blk_smem_bytes()
 {
-    return 1024 + (int)blk_tail<K>() + (int)sizeof(BlkTail<double>);
+    return 128 + (int)blk_tail<K>() + (int)sizeof(BlkTail<double>);
 }
 
 // Shared memory by 32-bit shared address.
@@ -233,7 +240,7 @@ __device__ __forceinline__ void blk_face_crit(BlkFace &f, f2 gK, float g)
 // halves whose volume cap binds
 template <int MATH>
 __device__ __forceinline__ f2 blk_face_q(const BlkFace &f, f2 w, f2 A, f2 rden, f2 nden,
-                                         unsigned &caps)
+                                         unsigned &caps, bool &c0, bool &c1)
 {
     const f2 Qm = mul2(mul2(f.v, f.hf), w);
     const f2 num = mul2(ab2(f.dL), A);
@@ -242,12 +249,69 @@ __device__ __forceinline__ f2 blk_face_q(const BlkFace &f, f2 w, f2 A, f2 rden, 
         Qc = div2_c(num, rden, nden);
     else
         Qc = mul2(num, rden);
-    if (lo2(Qc) < lo2(Qm))
+    c0 = lo2(Qc) < lo2(Qm);
+    c1 = hi2(Qc) < hi2(Qm);
+    if (c0)
         caps += 1u;
-    if (hi2(Qc) < hi2(Qm))
+    if (c1)
         caps += 1u;
     const f2 Q = min2(Qm, Qc);
     return mk2(csign(lo2(Q), lo2(f.dL)), csign(hi2(Q), hi2(f.dL)));
+}
+
+// Discharges of two cells across an open edge, to the virtual neighbour
+// z - S_bnd*dx, h = 0, same n, clipped at zero (FloodCA
+// src/common/model.c:166-177); cap: bit per half whose volume cap binds. The
+// cells' z, h and n lie at shared address `row` (a tile's row), the step's
+// constants at kc and sv. Evaluated on the pair like any other face: the
+// scalar formula, called for each cell from both phases that need it, took
+// half of a 61 x 93 grid's step.
+struct OpenPair {
+    f2 q;
+    unsigned cap;
+};
+static __device__ __noinline__ OpenPair open_pair(uint32_t row, uint32_t kc, uint32_t sv)
+{
+    const f2 z = sld(row + BLK_Z), n = sld(row + BLK_N);
+    const f2 L = add2(z, sld(row + BLK_H));
+    const float S = slf(sv + (uint32_t)offsetof(StepVals<float>, k.S_bnd));
+    const float dxs = slf(sv + (uint32_t)offsetof(StepVals<float>, k.dx));
+    const float g = slf(sv + (uint32_t)offsetof(StepVals<float>, k.g));
+    const f2 lv = sub2(z, bc2(__fmul_rn(S, dxs)));
+    bool unsure = false, crit = false;
+    BlkFace f = blk_face_v<MATH_EXACT>(L, lv, z, lv, n, n, bc2(dxs),
+                                       sld(kc + (uint32_t)offsetof(BlkK, nrdx)),
+                                       slf(kc + (uint32_t)offsetof(BlkK, tau_l)),
+                                       slf(kc + (uint32_t)offsetof(BlkK, tau_h)), unsure);
+    if (unsure)
+        f.cb = mk2(blk_cbrt(lo2(f.hf)), blk_cbrt(hi2(f.hf)));
+    const f2 gK = bc2(g * 0.999999f);
+    blk_face_m(f, gK, crit);
+    if (crit)
+        blk_face_crit<MATH_EXACT>(f, gK, g);
+    unsigned caps = 0u;
+    OpenPair o;
+    bool c0, c1;
+    o.q = blk_face_q<MATH_EXACT>(f, sld(kc + (uint32_t)offsetof(BlkK, w)),
+                                 sld(kc + (uint32_t)offsetof(BlkK, A)),
+                                 sld(kc + (uint32_t)offsetof(BlkK, rden)),
+                                 sld(kc + (uint32_t)offsetof(BlkK, nden)), caps, c0, c1);
+    o.cap = (c0 ? 1u : 0u) | (c1 ? 2u : 0u);
+    o.q = max2(o.q, bc2(0.0f));
+    return o;
+}
+
+// Open sides of the cells (r, c) and (r, c+1); edges as in BlockSweep::run.
+__device__ __forceinline__ void open_sides(int r, int c, int nr, int nc, int r_lo, int r_hi,
+                                           int edges, int &k0, int &k1)
+{
+    const int rows = (r == 0 && (edges & 1)) + (r == nr - 1 && (edges & 2));
+    const bool rin = r >= r_lo && r < r_hi;
+    k0 = rin && c >= 0 && c < nc ? rows + (c == 0 && (edges & 4)) + (c == nc - 1 && (edges & 8))
+                                 : 0;
+    k1 = rin && c + 1 >= 0 && c + 1 < nc
+             ? rows + (c + 1 == 0 && (edges & 4)) + (c + 1 == nc - 1 && (edges & 8))
+             : 0;
 }
 
 // Q s of the upwind cell (s_down for Q < 0): one of the products is zero.
@@ -271,26 +335,27 @@ struct BlockSweep {
     // Per-CTA state that persists over units: the count of tile passes so far
     // decides stages, barrier parities and ring buffers.
     struct Cta {
-        uint32_t sb;                // shared address of the CTA's memory (1024-byte aligned)
+        uint32_t sb;                // shared address of the CTA's memory (128-byte aligned)
         Tail *tail;
         unsigned pass;
     };
 
-    // Once per CTA: barriers, cleared rings (rows above a unit's first row
-    // are read, and their results dropped).
-    static __device__ __forceinline__ void init(Cta &T, char *sm)
+    // What a unit reads of a row above its first one, from rings that no
+    // phase has written yet, only reaches rows that are dropped: the rings
+    // need no clearing.
+    static __device__ __forceinline__ void attach(Cta &T, char *sm)
     {
         T.sb = smem_addr(sm);
         T.tail = reinterpret_cast<Tail *>(sm + TAIL);
         T.pass = 0;
-        for (uint32_t o = BLK_RINGS + threadIdx.x * 16; o < TAIL; o += BLK_THREADS * 16)
-            *reinterpret_cast<uint4 *>(sm + o) = make_uint4(0u, 0u, 0u, 0u);
-        if (threadIdx.x == 0) {
-            for (int q = 0; q < BLK_STAGES; q++)
-                mbar_init1(smem_addr(&T.tail->bar[q]));
-            T.tail->bad = 0;
-            fence_proxy_async_smem();
-        }
+    }
+    // one thread, once per CTA
+    static __device__ __forceinline__ void init_barriers(Cta &T)
+    {
+        for (int q = 0; q < BLK_STAGES; q++)
+            mbar_init1(T.sb + TAIL + 8u * q);
+        T.tail->bad = 0;
+        fence_proxy_async_smem();
     }
 
     // Once per step (one thread; a barrier follows): constants and sums.
@@ -301,8 +366,8 @@ struct BlockSweep {
         const StepVals<float> sv = step_vals<float, K>(g, rk, ctl);
         const StepK<float> &k = sv.k;
         t.sv = sv;
-        t.a_clamp = t.a_bnd = 0;
-        t.vmax = 0u;
+        t.a_clamp = t.a_bnd = t.a_rain = 0;
+        t.vmax = t.cap = 0u;
         t.rain_cells = 0;
         BlkK &c = t.c;
         c.dx = bc2(k.dx);
@@ -336,6 +401,16 @@ struct BlockSweep {
         tma_load_tile(dst + BLK_H, th, bar, tx, y0);
         tma_load_tile(dst + BLK_N, tm + 1, bar, tx, y0);
         tma_load_tile(dst + BLK_M, tm + 4, bar, tx, y0);
+    }
+    // one thread: the tiles of a unit's first passes
+    static __device__ __forceinline__ void first_tiles(const Cta &T, const GridD<float> &g,
+                                                       int h_cur, int strip, int r0, int r1)
+    {
+        using Gm = Geom<2>;
+        const int np = (r1 - r0 + 6 + BLK_ROWS - 1) / BLK_ROWS;
+        for (int b = 0; b < min(np, BLK_STAGES - 1); b++)
+            issue(T.sb, g.tmap, g.tmap + (h_cur ? 3 : 2), strip * Gm::OW - Gm::HL + PADC,
+                  r0 - 5 + PADR + b * BLK_ROWS, T.pass + b);
     }
     // one thread: waits for the tiles of a pass
     static __device__ __forceinline__ void arrived(const Cta &T, unsigned pass)
@@ -371,11 +446,57 @@ struct BlockSweep {
         return fmaxf(thr * thr * 0.999998f * __frcp_rn(t.sv.k.g), t.sv.k.tau_h);
     }
 
-    // Rows [r0, r1) of one strip, by the whole CTA. wp: the warp's index, as a
-    // warp-uniform value.
+    // The CTA's sums and velocity maximum to the control block.
+    static __device__ __forceinline__ void publish(Cta &T, const SS &ss, Ctl *ctl, int lane,
+                                                   int slot)
+    {
+        using Gm = Geom<2>;
+        Tail &t = *T.tail;
+        // halo lanes evaluate faces that other strips own
+        const bool out = lane * 2 >= Gm::HL && lane * 2 < Gm::HL + Gm::OW;
+        const unsigned cap = __reduce_add_sync(0xffffffffu, out ? ss.capn : 0u);
+        if (lane == 0 && cap)
+            atomicAdd(&t.cap, cap);
+        if constexpr (sizeof(AccT) == 4) {
+            const AccT r = warp_sum(ss.a_rain);
+            if (lane == 0)
+                atomicAdd(&t.a_rain, r);
+        } else if constexpr (RAINF) {
+            const double r = warp_sum(ss.rain_sum);
+            if (lane == 0)
+                atomicAdd(&t.a_rain, (double)t.sv.A * r);
+        }
+        __syncthreads();
+        // the sums are read by the host only: warp 1 adds them, so that warp
+        // 0's fence does not wait for them
+        if (threadIdx.x == 32) {
+            AccT rain = t.a_rain;
+            if constexpr (sizeof(AccT) == 8 && !RAINF)
+                rain = (double)t.rain_cells * ((double)t.sv.A * (double)t.sv.rainv);
+            AccT *const acc = sizeof(AccT) == 8 ? (AccT *)&ctl->accd[0][slot]
+                                                : (AccT *)&ctl->accf[0][slot];
+            if (rain != 0)
+                atomicAdd(acc, rain);
+            if (t.a_clamp != 0)
+                atomicAdd(acc + NSLOT, t.a_clamp);
+            if (t.a_bnd != 0)
+                atomicAdd(acc + 3 * NSLOT, t.a_bnd);
+            if (t.cap)
+                atomicAdd(&ctl->cap[slot], (unsigned long long)t.cap);
+        }
+        if (threadIdx.x == 0) {
+            if (t.sv.want_v && t.vmax)
+                atomicMax(&ctl->vmax_bits, (unsigned long long)t.vmax);
+            if (t.bad)
+                ctl->err = 3;       // a row tile never arrived; the host reports it
+        }
+    }
+
+    // Rows [r0, r1) of one strip, by the whole CTA; its first tiles are on
+    // their way (first_tiles). wp: the warp's index, as a warp-uniform value.
     static __device__ __forceinline__ void run(Cta &T, const GridD<float> &g,
-                                               const RunK<float> &rk, int strip, int r0, int r1,
-                                               int wp, int lane, SS &ss)
+                                               const RunK<float> &rk, int h_cur, int strip,
+                                               int r0, int r1, int wp, int lane, SS &ss)
     {
         using Gm = Geom<2>;
         Tail &tl = *T.tail;
@@ -397,15 +518,12 @@ struct BlockSweep {
         const int H = r1 - r0;
         const int np = (H + 6 + BLK_ROWS - 1) / BLK_ROWS;           // passes
         const CUtensorMap *tm = g.tmap;
-        const CUtensorMap *th = tm + (tl.sv.hin == g.h1 ? 3 : 2);
+        const CUtensorMap *th = tm + (h_cur ? 3 : 2);
         const int tx = c_first + PADC;                              // a multiple of 4 floats
         const int ty = r0 - 5 + PADR;
         const unsigned pass0 = T.pass;
-        if (wp == 0 && lane == 0) {
-            for (int b = 0; b < min(np, BLK_STAGES - 1); b++)
-                issue(sb, tm, th, tx, ty + b * BLK_ROWS, pass0 + b);
+        if (wp == 0 && lane == 0)
             arrived(T, pass0);
-        }
         float hcut = height_cut(tl, threshold(tl));
         __syncthreads();
 
@@ -479,14 +597,15 @@ struct BlockSweep {
                 // volume caps are counted by the cell that holds the face: x
                 // faces by row i, the others by row i-1
                 unsigned cx = 0u, cy = 0u;
+                bool c0, c1;
                 const f2 w = FCAB_KC(w), A = FCAB_KC(A), rden = FCAB_KC(rden), nden = FCAB_KC(nden);
-                const f2 X = blk_face_q<MATH>(f[0], w, A, rden, nden, cx);
-                Y1 = blk_face_q<MATH>(f[1], w, A, rden, nden, cy);
+                const f2 X = blk_face_q<MATH>(f[0], w, A, rden, nden, cx, c0, c1);
+                Y1 = blk_face_q<MATH>(f[1], w, A, rden, nden, cy, c0, c1);
                 keep(rb + BLK_X, X, last2, over);
                 keep(rb + BLK_Y, Y1, last2, over);
                 if constexpr (K == 8) {
-                    E1 = blk_face_q<MATH>(f[2], w, A, rden, nden, cy);
-                    W1 = blk_face_q<MATH>(f[3], w, A, rden, nden, cy);
+                    E1 = blk_face_q<MATH>(f[2], w, A, rden, nden, cy, c0, c1);
+                    W1 = blk_face_q<MATH>(f[3], w, A, rden, nden, cy, c0, c1);
                     keep(rb + BLK_E, E1, last2, over);
                     keep(rb + BLK_W, W1, last2, over);
                 }
@@ -517,13 +636,13 @@ struct BlockSweep {
                 }
                 const f2 hp = sld(tb + BLK_H + BLK_ROW_B);
                 if (spec && open_row(edges, r + 1, nr)) {
-                    const bool own = out_lane && (unsigned)(rel + 1) < (unsigned)H;
-                    const OpenFaces o = open_faces2(sld(tb + BLK_Z + BLK_ROW_B), hp,
-                                                    sld(tb + BLK_N + BLK_ROW_B), r + 1, cbase, nr,
-                                                    nc, g.r_lo, g.r_hi, edges, own, own,
-                                                    &tl.sv.k);
-                    ss.capn += o.cap;
-                    out = add2(out, o.add);
+                    const OpenPair o = open_pair(tb + BLK_ROW_B, sb + KC, sb + SV);
+                    int k0, k1;
+                    open_sides(r + 1, cbase, nr, nc, g.r_lo, g.r_hi, edges, k0, k1);
+                    if ((unsigned)(rel + 1) < (unsigned)H)
+                        ss.capn += (o.cap & 1u ? k0 : 0) + (o.cap & 2u ? k1 : 0);
+                    out = add2(out, mk2(open_sum<float>(lo2(o.q), k0),
+                                        open_sum<float>(hi2(o.q), k1)));
                 }
                 const f2 ov = mul2(out, FCAB_KC(dt));
                 const f2 hold = mul2(hp, FCAB_KC(A));
@@ -563,20 +682,20 @@ struct BlockSweep {
                 if (spec && open_row(edges, r, nr)) {
                     // open-edge outflow scaled by the cell's own limiter
                     // (model.c:553-559), summed over its open slots
-                    const OpenFaces o = open_faces2(sld(tb + BLK_Z), h, sld(tb + BLK_N), r, cbase,
-                                                    nr, nc, g.r_lo, g.r_hi, edges, false, false,
-                                                    &tl.sv.k);
-                    float qb[2];
-#pragma unroll
-                    for (int j = 0; j < 2; j++)
-                        qb[j] = open_sum<float>(get2(o.qo, j) * get2(S2, j),
-                                                __popc((o.ko >> (4 * j)) & 15u));
-                    net = sub2(net, mk2(qb[0], qb[1]));
+                    const OpenPair o = open_pair(tb, sb + KC, sb + SV);
+                    int k0, k1;
+                    open_sides(r, cbase, nr, nc, g.r_lo, g.r_hi, edges, k0, k1);
+                    const f2 qs = mul2_sep(o.q, S2);
+                    const float q0 = open_sum<float>(lo2(qs), k0);
+                    const float q1 = open_sum<float>(hi2(qs), k1);
+                    net = sub2(net, mk2(q0, q1));
                     const float dt = FCAB_SV(dt);
-                    if (own2 && out_lane && (o.ko & 15u))
-                        atomicAdd(&tl.a_bnd, acc_mul<AccT, float>(dt, qb[0]));
-                    if (own2 && out_lane && (o.ko >> 4))
-                        atomicAdd(&tl.a_bnd, acc_mul<AccT, float>(dt, qb[1]));
+                    AccT bnd = 0;
+                    if (own2 && out_lane)
+                        bnd = acc_mul<AccT, float>(dt, q0) + acc_mul<AccT, float>(dt, q1);
+                    bnd = warp_sum(bnd);
+                    if (lane == 0 && bnd != 0)
+                        atomicAdd(&tl.a_bnd, bnd);
                 }
                 f2 rain;
                 if constexpr (RAINF) {

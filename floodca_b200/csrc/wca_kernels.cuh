@@ -136,13 +136,21 @@ __device__ __forceinline__ double tri_f(double t, double T, double tp)
     return T - tp <= 0.0 ? 0.0 : (2.0 / T) * ((T - t) / (T - tp));
 }
 
+// RN(x / c) given rc = RN(1/c) (Markstein's correction; see div_mk): a third
+// of the latency of the division.
+__device__ __forceinline__ double div_const(double x, double c, double rc)
+{
+    const double q = x * rc;
+    return fma(fma(-q, c, x), rc, q);
+}
+
 __device__ inline double hyeto_integral(const TimeCfg &c, double t, double dt)
 {
     if (dt <= 0.0)
         return 0.0;
     double t1 = t + dt;
     if (c.hyeto == 1)
-        return dt / 86400.0;
+        return div_const(dt, 86400.0, 1.0 / 86400.0);
     double T = c.D_h * 3600.0, tp = c.phi * T, sum = 0.0, a;
     if (t1 <= 0.0 || t >= T)
         return 0.0;
@@ -208,54 +216,94 @@ __device__ inline double inflow_volume(const TimeCfg &c, double t, double dt)
     return sum;
 }
 
-// Prepares ctl for the step after the one just taken (after_step) or for
-// the first step. Runs on one thread once every CTA's atomics are visible.
-template <typename T>
-__device__ void finalize(Ctl *c, const TimeCfg &tc, const RunK<T> &rk, bool after_step)
+// What the next step's clock needs from the step now running, none of which
+// depends on the new depths: known as soon as that step starts, so the block
+// sweep works it out while its first tiles are in flight.
+struct TimePre {
+    double t, t_next;           // time after the step, next event after that
+    double dt_base, V_in;       // the held dt; inflow volume after the step
+    unsigned long long seed;
+    long long hits, full_passes;
+    int step, done, pause, rain_on, inflow_off;
+};
+
+__device__ inline TimePre time_pre(const Ctl *c, const TimeCfg &tc, bool after_step)
 {
+    TimePre p;
     double t = c->t;
     int step = c->step;
+    const double dt = c->dt, t_next = c->t_next, wend = c->window_end;
+    const int hit = c->hit, force_day = c->force_day, carry = c->pause_carry;
+    const double V_in_step = c->V_in_step;
+    p.V_in = c->V_in;
+    p.dt_base = c->dt_base;
+    p.seed = c->vseed_bits;
+    p.hits = c->dt_min_hits;
+    p.full_passes = c->full_passes;
+    p.inflow_off = c->inflow_off;
     if (after_step) {
-        if (c->hit)
-            t = c->t_next;
+        p.V_in += V_in_step;
+        if (hit)
+            t = t_next;
         else if (tc.time_f32)
-            t = (double)((float)c->t + (float)c->dt);
+            t = (double)((float)t + (float)dt);
         else
-            t = c->t + c->dt;
+            t = t + dt;
         step += 1;
-        c->V_in += c->V_in_step;
     }
-    bool done = tc.max_steps > 0 ? step >= tc.max_steps : t >= tc.T_sim - 1e-15;
+    const bool done = tc.max_steps > 0 ? step >= tc.max_steps : t >= tc.T_sim - 1e-15;
     int pause = 0;
     if (!done && tc.n_force_days > 0) {
         int d = t < 0.0 ? 0 : (int)floor(t / 86400.0);
         if (d >= tc.n_force_days)
             d = tc.n_force_days - 1;
-        if (d != c->force_day)
+        if (d != force_day)
             pause = 1;              // the host loads the day's Rday, then resumes
     }
     if (!done && after_step && tc.progress_every > 0 && step % tc.progress_every == 0)
         pause = 1;
-    if (!done && c->pause_carry)
+    if (!done && carry)
         pause = 1;                  // decided before a deferred dt
-    if (!done && c->window_end > 0.0 && t >= c->window_end - 1e-9)
+    if (!done && wend > 0.0 && t >= wend - 1e-9)
         pause = 1;                  // end of an output window
-    T dt_base = (T)c->dt_base;
+    p.t = t;
+    p.step = step;
+    p.done = done;
+    p.pause = pause;
+    p.t_next = done ? 0.0 : next_event(tc, t);
+    p.rain_on = tc.rain_end <= 0.0 || tc.rain_end - t >= 1e-9;
+    return p;
+}
+
+// Prepares ctl for the step after the one just taken (after_step) or for
+// the first step. Runs on one thread once every CTA's atomics are visible.
+// Of the control block it reads the velocity maximum alone, the rest comes
+// with `pre`: a chain of loads through global memory costs about 300 cycles a
+// link.
+template <typename T>
+__device__ void finalize(Ctl *c, const TimeCfg &tc, const RunK<T> &rk, bool after_step,
+                         const TimePre &pre)
+{
+    const unsigned long long vbits = *(volatile unsigned long long *)&c->vmax_bits;
+    const unsigned long long sbits = pre.seed;
+    const double t = pre.t;
+    const int step = pre.step, pause = pre.pause;
+    bool done = pre.done != 0;
+    c->V_in = pre.V_in;
+    T dt_base = (T)pre.dt_base;
     if (!done && step % tc.U == 0) {
-        T vmax;
-        if (sizeof(T) == 4)
-            vmax = (T)__uint_as_float((unsigned)c->vmax_bits);
-        else
-            vmax = (T)__longlong_as_double((long long)c->vmax_bits);
-        T seed;
-        if (sizeof(T) == 4)
-            seed = (T)__uint_as_float((unsigned)c->vseed_bits);
-        else
-            seed = (T)__longlong_as_double((long long)c->vseed_bits);
+        T vmax, seed;
+        if (sizeof(T) == 4) {
+            vmax = (T)__uint_as_float((unsigned)vbits);
+            seed = (T)__uint_as_float((unsigned)sbits);
+        } else {
+            vmax = (T)__longlong_as_double((long long)vbits);
+            seed = (T)__longlong_as_double((long long)sbits);
+        }
         if (after_step && tc.vseed_on && vmax < seed) {
-            c->full_passes += 1;
             // cells pruned against the seed may hold the maximum: keep the
-            // time advance, defer dt to the full velocity pass (k_init_dt)
+            // time advance, defer dt to the full velocity pass
+            c->full_passes = pre.full_passes + 1;
             c->t = t;
             c->step = step;
             c->pause_carry = pause;
@@ -285,7 +333,7 @@ __device__ void finalize(Ctl *c, const TimeCfg &tc, const RunK<T> &rk, bool afte
         }
         if (dtm < rk.dt_min) {
             dtm = rk.dt_min;
-            c->dt_min_hits += 1;
+            c->dt_min_hits = pre.hits + 1;
         }
         if (dtm > rk.dt_max)
             dtm = rk.dt_max;
@@ -296,7 +344,7 @@ __device__ void finalize(Ctl *c, const TimeCfg &tc, const RunK<T> &rk, bool afte
     int hit = 0;
     double F = 0.0, V_in = 0.0;
     if (!done) {
-        t_next = next_event(tc, t);
+        t_next = pre.t_next;
         double remain = t_next - t;
         if (remain <= (double)dt) {
             if (remain < 0.0)
@@ -308,9 +356,8 @@ __device__ void finalize(Ctl *c, const TimeCfg &tc, const RunK<T> &rk, bool afte
             done = true;            // the reference loop stops advancing here
     }
     if (!done) {
-        bool rain_on = tc.rain_end <= 0.0 || tc.rain_end - t >= 1e-9;
-        F = rain_on ? hyeto_integral(tc, t, (double)dt) : 0.0;
-        V_in = c->inflow_off ? 0.0 : inflow_volume(tc, t, (double)dt);
+        F = pre.rain_on ? hyeto_integral(tc, t, (double)dt) : 0.0;
+        V_in = pre.inflow_off ? 0.0 : inflow_volume(tc, t, (double)dt);
     }
     c->t = t;
     c->step = step;
@@ -319,7 +366,7 @@ __device__ void finalize(Ctl *c, const TimeCfg &tc, const RunK<T> &rk, bool afte
     c->t_next = t_next;
     c->hit = hit;
     c->F = F;
-    c->inflow_dh = (double)(T)(V_in / (double)rk.k.A);
+    c->inflow_dh = V_in != 0.0 ? (double)(T)(V_in / (double)rk.k.A) : 0.0;
     c->V_in_step = V_in;
     if (tc.time_f32)
         c->tmax_val = (double)((float)t + (float)dt);
@@ -333,6 +380,14 @@ __device__ void finalize(Ctl *c, const TimeCfg &tc, const RunK<T> &rk, bool afte
     c->active = (!done && !pause) ? 1 : 0;
     c->vmax_bits = 0ull;
     c->ctas_done = 0u;
+}
+
+template <typename T>
+__device__ __forceinline__ void finalize(Ctl *c, const TimeCfg &tc, const RunK<T> &rk,
+                                         bool after_step)
+{
+    const TimePre pre = time_pre(c, tc, after_step);
+    finalize<T>(c, tc, rk, after_step, pre);
 }
 
 // --------------------------------------------------------------------------
@@ -1301,59 +1356,160 @@ __device__ __forceinline__ void step_tail(const GridD<T> &g, const RunK<T> &rk, 
     }
 }
 
+// Stable velocity of cell (r, c) on the current depth h (0: not a wet LAND
+// cell, or not above the depth hcut).
+template <typename T, int K, int MATH>
+__device__ __forceinline__ T velocity_at(const GridD<T> &g, const RunK<T> &rk, const T *h, int r,
+                                         int c, T hcut)
+{
+    const StepK<T> &k = rk.k;
+    const long long a = (long long)(r + PADR) * g.pitch + c + PADC;
+    const T ha = h[a];
+    if (!(ha >= hcut) || g.m[a] != M_LAND)
+        return T(0);
+    const T la = g.z[a] + ha;
+    T mo = T(0), md = T(0);
+    const long long nb[8] = {a + 1, a - 1, a + g.pitch, a - g.pitch,
+                             a + g.pitch + 1, a + g.pitch - 1, a - g.pitch + 1,
+                             a - g.pitch - 1};
+#pragma unroll
+    for (int q = 0; q < (K == 8 ? 8 : 4); q++) {
+        const uint32_t mb = g.m[nb[q]];
+        if (mb == M_WALL)
+            continue;
+        const T lb = mb == M_SEA ? k.z_sea : g.z[nb[q]] + h[nb[q]];
+        const T d = fabs(la - lb);
+        if (q < 4)
+            mo = fmax(mo, d);
+        else
+            md = fmax(md, d);
+    }
+    if (rk.open && ((c == 0 && rk.edge_w) || (c == g.nc - 1 && rk.edge_e) ||
+                    (r == 0 && rk.edge_n) || (r == g.nr - 1 && rk.edge_s)))
+        mo = fmax(mo, fabs(la - (g.z[a] - k.S_bnd * k.dx)));
+    T Smax = Mth<T, MATH>::div(mo, k.dx);
+    if (K == 8) {
+        const T Sd = Mth<T, MATH>::div(md, k.d_diag);
+        if (Sd > Smax)
+            Smax = Sd;
+    }
+    return cell_velocity<T, MATH>(ha, g.n[a], Smax, k);
+}
+
 // The block sweep's step: CTAs take units of `seg` rows of a strip.
-template <typename AccT, int K, int MATH, bool RAINF>
+//
+// A step on a small grid is latency: of the 14.5 us a 61 x 93 step took, 2.7
+// were the launch of a kernel that can launch others (1.2 without), 1.6 the
+// constants and the first tiles one after the other, 5 the scalar open-edge
+// formula on cold code, 1.9 the clock at the end. So the first tiles leave
+// before anything else is computed, the constants and the clock are worked
+// out by two other warps meanwhile, and on grids of up to BLK_SOLO cells
+// (TAILV = false) the last CTA does a missed seed's velocity pass itself
+// instead of launching it. Measured, us a step: 61 x 93 14.5 -> 9.0, 256^2
+// 18.2 -> 11.1, 512^2 19.3 -> 14.3, 1024^2 27.8 -> 25.2.
+template <typename AccT, int K, int MATH, bool RAINF, bool TAILV>
 __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
     k_step_blk(GridD<float> g, RunK<float> rk, TimeCfg tc, Ctl *ctl, int seg)
 {
     using Sweep = BlockSweep<AccT, K, MATH, RAINF>;
     using G = Geom<2>;
-    if (ctl->active == 0)
+    const int active = ctl->active, h_cur = ctl->h_cur;
+    if (active == 0)
         return;
     extern __shared__ __align__(1024) unsigned char fcab_dsm[];
     char *const sm = reinterpret_cast<char *>(fcab_dsm) +
-                     ((1024u - (smem_addr(fcab_dsm) & 1023u)) & 1023u);
+                     ((128u - (smem_addr(fcab_dsm) & 127u)) & 127u);
     int lane;       // volatile: held in a register, not read again from the special register
     asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
-    StepSums<float, AccT> ss;
-    typename Sweep::Cta T;
-    Sweep::init(T, sm);
-    if (threadIdx.x == 0) {
-        Sweep::begin(T, g, rk, ctl);
-        fence_proxy_async_smem();
-    }
-    __syncthreads();
+    const int wp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
     // units of `seg` rows of a strip, taken from the step's counter (the first
     // one by the CTA's index)
     const int nr = g.nr, nstrips = (g.nc + G::OW - 1) / G::OW;
     const int nblk = (nr + seg - 1) / seg, units = nstrips * nblk;
-    const int wp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    typename Sweep::Cta T;
+    Sweep::attach(T, sm);
+    if (lane == 0) {
+        if (wp == 0) {
+            Sweep::init_barriers(T);
+            const int r0 = blockIdx.x % nblk * seg;
+            Sweep::first_tiles(T, g, h_cur, blockIdx.x / nblk, r0, min(nr, r0 + seg));
+            T.tail->unit[0] = units > (int)gridDim.x
+                                  ? (int)(gridDim.x + atomicAdd(&ctl->next_unit, 1u))
+                                  : units;
+        } else if (wp == 1) {
+            Sweep::begin(T, g, rk, ctl);
+        } else if (wp == 2) {
+            T.tail->pre = time_pre(ctl, tc, true);
+        }
+    }
+    __syncthreads();
+    StepSums<float, AccT> ss;
     int par = 0;
     for (int u = blockIdx.x; u < units; par ^= 1) {
-        if (threadIdx.x == 0)
-            T.tail->unit[par] = units > (int)gridDim.x
-                                    ? (int)(gridDim.x + atomicAdd(&ctl->next_unit, 1u))
-                                    : units;
-        const int r0 = u % nblk * seg;
-        Sweep::run(T, g, rk, u / nblk, r0, min(nr, r0 + seg), wp, lane, ss);
+        const int r0 = u % nblk * seg, r1 = min(nr, r0 + seg);
+        if (u != (int)blockIdx.x && wp == 0 && lane == 0) {
+            Sweep::first_tiles(T, g, h_cur, u / nblk, r0, r1);
+            T.tail->unit[par] = (int)(gridDim.x + atomicAdd(&ctl->next_unit, 1u));
+        }
+        Sweep::run(T, g, rk, h_cur, u / nblk, r0, r1, wp, lane, ss);
         __syncthreads();
         u = T.tail->unit[par];
     }
-    // halo lanes evaluate faces that other strips own
-    if (!(lane * 2 >= G::HL && lane * 2 < G::HL + G::OW))
-        ss.capn = 0u;
+    Sweep::publish(T, ss, ctl, lane, (int)(blockIdx.x & (NSLOT - 1)));
+    // ---- the last CTA to finish prepares the next step
     if (threadIdx.x == 0) {
-        if (T.tail->bad)
-            ctl->err = 3;           // a row tile never arrived; the host reports it
-        ss.a_clamp = T.tail->a_clamp;
-        ss.a_bnd = T.tail->a_bnd;
-        ss.vmax = __uint_as_float(T.tail->vmax);
-        ss.rain_cells = T.tail->rain_cells;
+        int solo = 0;
+        __threadfence();
+        const unsigned prev = atomicAdd(&ctl->ctas_done, 1u);
+        if (prev == gridDim.x - 1) {
+            __threadfence();
+            ctl->h_cur = h_cur ^ 1;
+            ctl->launches += 1;
+            ctl->next_unit = 0u;
+            if (tc.split) {
+                ctl->fin_pending = 1;
+                ctl->ctas_done = 0u;
+            } else {
+                const unsigned vbits = (unsigned)ctl->vmax_bits;
+                finalize<float>(ctl, tc, rk, true, T.tail->pre);
+                // a missed seed defers this step's dt to the full velocity
+                // pass: done here, or launched from here into the tail of the
+                // stream, so it runs before the next step and only when needed
+                if (ctl->need_v) {
+                    if constexpr (TAILV) {
+                        k_init_dt<float, K, MATH>
+                            <<<VPASS_GRID, 256, 0, cudaStreamTailLaunch>>>(g, rk, tc, ctl, 1);
+                        if (cudaGetLastError() != cudaSuccess)
+                            ctl->err = 2;   // the host's poll runs the pass instead
+                    } else {
+                        solo = 1;
+                        T.tail->vmax = vbits;
+                    }
+                }
+            }
+        }
+        T.tail->unit[0] = solo;
     }
-    const StepVals<float> &sv = T.tail->sv;
-    publish_sums<float, AccT, RAINF>(ss, sv, ctl, lane,
-                                     (int)((blockIdx.x * BLK_ROWS + wp) & (NSLOT - 1)));
-    step_tail<float, K, MATH>(g, rk, tc, ctl);
+    if constexpr (!TAILV) {
+        __syncthreads();
+        if (T.tail->unit[0] == 0)
+            return;
+        // the pruned maximum is a velocity some cell has: only deeper cells
+        // than it allows can raise it
+        const float hcut = Sweep::height_cut(*T.tail, __uint_as_float(T.tail->vmax));
+        const float *h = T.tail->sv.hout;
+        float vmax = 0.0f;
+        for (int i = threadIdx.x; i < nr * g.nc; i += BLK_THREADS)
+            vmax = fmaxf(vmax, velocity_at<float, K, MATH>(g, rk, h, i / g.nc, i % g.nc, hcut));
+        vmax = warp_max_nonneg(vmax);
+        if (lane == 0)
+            atomicMax(&T.tail->vmax, __float_as_uint(vmax));
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            ctl->vmax_bits = T.tail->vmax;
+            finalize<float>(ctl, tc, rk, false);
+        }
+    }
 }
 
 template <typename T, typename AccT, int K, int CPL, int MATH, bool RAINF, bool LANDONLY>
@@ -1572,43 +1728,13 @@ __global__ void k_batch_window(const MemberD<T> *members, int n, double window)
 template <typename T, int K, int MATH>
 __device__ void velocity_pass(const GridD<T> &g, const RunK<T> &rk, const TimeCfg &tc, Ctl *ctl)
 {
-    const StepK<T> k = rk.k;
     const T *h = ctl->h_cur ? g.h1 : g.h0;
     T vmax = T(0);
     const long long N = (long long)g.nr * g.nc;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < N;
          idx += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(idx / g.nc), c = (int)(idx % g.nc);
-        const long long a = (long long)(r + PADR) * g.pitch + c + PADC;
-        if (g.m[a] != M_LAND || !(h[a] >= k.tau_h))
-            continue;
-        const T la = g.z[a] + h[a];
-        T mo = T(0), md = T(0);
-        const long long nb[8] = {a + 1, a - 1, a + g.pitch, a - g.pitch,
-                                 a + g.pitch + 1, a + g.pitch - 1, a - g.pitch + 1,
-                                 a - g.pitch - 1};
-#pragma unroll
-        for (int q = 0; q < (K == 8 ? 8 : 4); q++) {
-            const uint32_t mb = g.m[nb[q]];
-            if (mb == M_WALL)
-                continue;
-            const T lb = mb == M_SEA ? k.z_sea : g.z[nb[q]] + h[nb[q]];
-            const T d = fabs(la - lb);
-            if (q < 4)
-                mo = fmax(mo, d);
-            else
-                md = fmax(md, d);
-        }
-        if (rk.open && ((c == 0 && rk.edge_w) || (c == g.nc - 1 && rk.edge_e) ||
-                        (r == 0 && rk.edge_n) || (r == g.nr - 1 && rk.edge_s)))
-            mo = fmax(mo, fabs(la - (g.z[a] - k.S_bnd * k.dx)));
-        T Smax = Mth<T, MATH>::div(mo, k.dx);
-        if (K == 8) {
-            const T Sd = Mth<T, MATH>::div(md, k.d_diag);
-            if (Sd > Smax)
-                Smax = Sd;
-        }
-        const T v = cell_velocity<T, MATH>(h[a], g.n[a], Smax, k);
+        const T v = velocity_at<T, K, MATH>(g, rk, h, (int)(idx / g.nc), (int)(idx % g.nc),
+                                            rk.k.tau_h);
         if (v > vmax)
             vmax = v;
     }

@@ -707,6 +707,7 @@ static int resolve_variant(FcabSim *s)
               (long long)(s->cfg.nrows + s->hn + s->hs + 2 * PADR) * s->pitch < (1ll << 31);
     if (key.blk)
         key.cpl = s->cpl = 2;
+    key.solo = (long long)s->cfg.nrows * s->cfg.ncols <= BLK_SOLO;
     bool ok = key.prec == FCAB_PREC_F32 ? lookup_f32(key, &s->L)
               : key.prec == FCAB_PREC_F32_ALL ? lookup_f32all(key, &s->L)
                                                : lookup_f64(key, &s->L);
