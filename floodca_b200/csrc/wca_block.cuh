@@ -1,4 +1,4 @@
-// The FP32 step on column pairs for all-LAND grids, one CTA per row range.
+// The FP32 step on column pairs, one CTA per row range.
 //
 // The same arithmetic as sweep_segment (FloodCA src/kernels/physics.h and
 // src/common/model.c:321-605), organised as passes of BLK_ROWS rows by a CTA
@@ -27,6 +27,13 @@
 // grids, one warp per row range (before) and this: 4096^2 350 and 220, 2048^2
 // 112 and 70, 1024^2 51.5 and 27.8, 256^2 20.1 and 18.2, 1003 x 1498 with
 // K = 8 104 and 64. Bound by issue slots and the barriers; HBM is at 24 %.
+//
+// Grids with SEA or WALL cells (GEN) carry the mask in the device copies of z
+// and n (k_encode_mask): n is NaN on every cell that is not LAND, z is PAD_Z
+// on WALL (a face to it carries nothing, as to the padding) and -PAD_Z on SEA.
+// A row whose cells are all LAND runs the same code as on an all-LAND grid
+// after a vote on its n; the others take a branch that puts in the sea level
+// and keeps the cells that are not LAND as they are.
 #pragma once
 
 #include <cstddef>
@@ -86,8 +93,10 @@ struct BlkTail {
     BlkK c;
     StepVals<float> sv;
     TimePre pre;
-    AccT a_clamp, a_bnd, a_rain;    // clamped volume, open-edge outflow, rain
+    AccT a_clamp, a_bnd, a_rain, a_sea; // clamped volume, open-edge outflow, rain, outflow to SEA
     long long rain_cells;       // LAND output cells (uniform rain)
+    double bnd[BLK_ROWS][2];    // outflow of the warps' west and east edge cells
+    float qo[2][32];            // open discharge of west and east edge cells, by row
     unsigned cap;               // faces whose volume cap bound
     unsigned vmax;              // bits of the CTA's largest next-step velocity
     int bad;
@@ -168,14 +177,16 @@ struct BlkFace {
     f2 dL, hf, cb, v, rs;
 };
 
-// Faces a -> b in the steps of face2_v / face2_crit / face2_q (see there for
-// the formulas), on the constants at shared address kc (a BlkK).
-// blk_face_v: everything up to the factors of the Manning velocity
+// Faces a -> b between cells of levels La, Lb, elevations za, zb and Manning n
+// of sum ns, centre distance d (nrd = -RN(1/d)) (FloodCA
+// src/kernels/physics.h:51-125), every operation rounded as the reference's,
+// in three steps so that the faces of a row run as one block of independent
+// work. blk_face_v: everything up to the factors of the Manning velocity
 // v * cb * rs = (1/nf) * hf^(2/3) * sqrt(S); `unsure`: a cube root of the lane
 // must be settled by the exact scalar function.
 template <int MATH>
-__device__ __forceinline__ BlkFace blk_face_v(f2 La, f2 Lb, f2 za, f2 zb, f2 na, f2 nb, f2 d,
-                                              f2 nrd, float tau_l, float tau_h, bool &unsure)
+__device__ __forceinline__ BlkFace blk_face_v(f2 La, f2 Lb, f2 za, f2 zb, f2 ns, f2 d, f2 nrd,
+                                              float tau_l, float tau_h, bool &unsure)
 {
     BlkFace f;
     const f2 dL = sub2(La, Lb);
@@ -184,7 +195,7 @@ __device__ __forceinline__ BlkFace blk_face_v(f2 La, f2 Lb, f2 za, f2 zb, f2 na,
     const bool live1 = fabsf(hi2(dL)) >= tau_l && hi2(hf) >= tau_h;
     f.dL = sel2(live0, live1, dL, bc2(0.0f));
     f.hf = sel2(live0, live1, hf, bc2(1.0f));
-    const f2 nf = max2(mul2(bc2(0.5f), add2(na, nb)), bc2(1e-12f));
+    const f2 nf = max2(mul2(bc2(0.5f), ns), bc2(1e-12f));
     if constexpr (MATH == MATH_EXACT) {
         f.v = rcp_2(nf);
         f.v = fma2(fma2(ng2(nf), f.v, bc2(1.0f)), f.v, f.v);
@@ -259,27 +270,24 @@ __device__ __forceinline__ f2 blk_face_q(const BlkFace &f, f2 w, f2 A, f2 rden, 
     return mk2(csign(lo2(Q), lo2(f.dL)), csign(hi2(Q), hi2(f.dL)));
 }
 
-// Discharges of two cells across an open edge, to the virtual neighbour
-// z - S_bnd*dx, h = 0, same n, clipped at zero (FloodCA
-// src/common/model.c:166-177); cap: bit per half whose volume cap binds. The
-// cells' z, h and n lie at shared address `row` (a tile's row), the step's
-// constants at kc and sv. Evaluated on the pair like any other face: the
-// scalar formula, called for each cell from both phases that need it, took
-// half of a 61 x 93 grid's step.
+// Discharges of two cells (z, h, n) across an open edge, to the virtual
+// neighbour z - S_bnd*dx, h = 0, same n, clipped at zero (FloodCA
+// src/common/model.c:166-177); cap: bit per half whose volume cap binds.
+// kc, sv: shared addresses of the step's constants. Evaluated on the pair like
+// any other face: the scalar formula took half of a 61 x 93 grid's step.
 struct OpenPair {
     f2 q;
     unsigned cap;
 };
-static __device__ __noinline__ OpenPair open_pair(uint32_t row, uint32_t kc, uint32_t sv)
+static __device__ __noinline__ OpenPair open_pair(f2 z, f2 h, f2 n, uint32_t kc, uint32_t sv)
 {
-    const f2 z = sld(row + BLK_Z), n = sld(row + BLK_N);
-    const f2 L = add2(z, sld(row + BLK_H));
+    const f2 L = add2(z, h);
     const float S = slf(sv + (uint32_t)offsetof(StepVals<float>, k.S_bnd));
     const float dxs = slf(sv + (uint32_t)offsetof(StepVals<float>, k.dx));
     const float g = slf(sv + (uint32_t)offsetof(StepVals<float>, k.g));
     const f2 lv = sub2(z, bc2(__fmul_rn(S, dxs)));
     bool unsure = false, crit = false;
-    BlkFace f = blk_face_v<MATH_EXACT>(L, lv, z, lv, n, n, bc2(dxs),
+    BlkFace f = blk_face_v<MATH_EXACT>(L, lv, z, lv, add2(n, n), bc2(dxs),
                                        sld(kc + (uint32_t)offsetof(BlkK, nrdx)),
                                        slf(kc + (uint32_t)offsetof(BlkK, tau_l)),
                                        slf(kc + (uint32_t)offsetof(BlkK, tau_h)), unsure);
@@ -314,6 +322,21 @@ __device__ __forceinline__ void open_sides(int r, int c, int nr, int nc, int r_l
              : 0;
 }
 
+// Cells that are not LAND: elevation and level of SEA cells (z = -PAD_Z) are
+// the sea level, the level of WALL cells their elevation PAD_Z.
+__device__ __forceinline__ void sea_levels(f2 &z, f2 &L, f2 n, float zs)
+{
+    z = sel2(lo2(z) < -1e29f, hi2(z) < -1e29f, bc2(zs), z);
+    L = sel2(lo2(n) != lo2(n), hi2(n) != hi2(n), z, L);
+}
+// Sum of two cells' Manning n for their mean; a cell that is not LAND (NaN)
+// takes the other's.
+__device__ __forceinline__ f2 nsum2(f2 a, f2 b)
+{
+    const f2 x = sel2(lo2(a) != lo2(a), hi2(a) != hi2(a), b, a);
+    return add2(x, sel2(lo2(b) != lo2(b), hi2(b) != hi2(b), x, b));
+}
+
 // Q s of the upwind cell (s_down for Q < 0): one of the products is zero.
 __device__ __forceinline__ f2 upwind2(f2 Q, f2 s_up, f2 s_down)
 {
@@ -321,8 +344,10 @@ __device__ __forceinline__ f2 upwind2(f2 Q, f2 s_up, f2 s_down)
     return fma2(min2(Q, z0), s_down, mul2(max2(Q, z0), s_up));
 }
 
-template <typename AccT, int K, int MATH, bool RAINF>
+// GEN: grids with SEA or WALL cells (with the rain as a field).
+template <typename AccT, int K, int MATH, bool RAINF, bool GEN>
 struct BlockSweep {
+    static_assert(RAINF || !GEN, "masked grids carry the rain as a field");
     using SS = StepSums<float, AccT>;
     using Tail = BlkTail<AccT>;
     static constexpr int NF = K == 8 ? 4 : 2;
@@ -366,8 +391,10 @@ struct BlockSweep {
         const StepVals<float> sv = step_vals<float, K>(g, rk, ctl);
         const StepK<float> &k = sv.k;
         t.sv = sv;
-        t.a_clamp = t.a_bnd = t.a_rain = 0;
+        t.a_clamp = t.a_bnd = t.a_rain = t.a_sea = 0;
         t.vmax = t.cap = 0u;
+        for (int q = 0; q < 2 * BLK_ROWS; q++)
+            t.bnd[q >> 1][q & 1] = 0.0;
         t.rain_cells = 0;
         BlkK &c = t.c;
         c.dx = bc2(k.dx);
@@ -427,10 +454,52 @@ struct BlockSweep {
             sst(at + over, v);
     }
 
-    // whether a row of the strip has open edges (all of its cells, or its end)
+    // whether all cells of a row have an open edge
     static __device__ __forceinline__ bool open_row(int edges, int r, int nr)
     {
-        return (edges & 12) || (r == 0 && (edges & 1)) || (r == nr - 1 && (edges & 2));
+        return (r == 0 && (edges & 1)) || (r == nr - 1 && (edges & 2));
+    }
+    // The open west (lanes 0..7) and east (lanes 8..15) edge cells of the
+    // pass's rows, a row per lane: their discharges into Tail::qo by row (modulo 32).
+    // One evaluation a pass instead of two per row of an edge strip: with both
+    // open, a 2048^2 step took 109 us that way and takes 67 this way (66 closed).
+    static __device__ __forceinline__ void open_ends(Tail &tl, uint32_t sb, uint32_t tiles,
+                                                     int first, int r0, int r1, int c_first,
+                                                     int nr, int nc, int edges, int lane)
+    {
+        const int side = lane >> 3 & 1, slot = lane & 7, row = first + slot;
+        const int c = (side ? nc - 1 : 0) - c_first;
+        float z = 0.0f, h = 0.0f, n = 1.0f;
+        const bool on = lane < 16 && (edges & (4 << side));
+        if (on) {
+            const uint32_t a = tiles + (slot + 2) * BLK_ROW_B + 4u * (uint32_t)c;
+            z = slf(a + BLK_Z);
+            h = slf(a + BLK_H);
+            n = slf(a + BLK_N);
+        }
+        const OpenPair o = open_pair(bc2(z), bc2(h), bc2(n), sb + KC, sb + SV);
+        if (on) {
+            const bool land = !GEN || n == n;
+            tl.qo[side][row & 31] = land ? lo2(o.q) : 0.0f;
+            // counted by the strip that writes the column; rows with open
+            // cells all along count theirs in phase C
+            if (land && (o.cap & 1u) && c < Geom<2>::HL + Geom<2>::OW && row >= r0 && row < r1 &&
+                !open_row(edges, row, nr))
+                atomicAdd(&tl.cap, 1u);
+        }
+    }
+
+    // What cells (r, c) and (r, c+1) lose across the open west and east edges,
+    // scaled by s, summed over their open sides.
+    static __device__ __forceinline__ f2 end_flow(const Tail &tl, int r, int c, int nr, int nc,
+                                                  int r_lo, int r_hi, int edges, f2 s)
+    {
+        int k0, k1;
+        open_sides(r, c, nr, nc, r_lo, r_hi, edges & 12, k0, k1);
+        const float e = tl.qo[1][r & 31];
+        const float q = c == 0 && (edges & 4) ? tl.qo[0][r & 31] : e;   // column 0 is a low half
+        return mk2(open_sum<float>(__fmul_rn(q, lo2(s)), k0),
+                   open_sum<float>(__fmul_rn(e, hi2(s)), k1));
     }
 
     // The velocity below which no cell can raise the step's maximum: the CTA's
@@ -479,8 +548,13 @@ struct BlockSweep {
                 atomicAdd(acc, rain);
             if (t.a_clamp != 0)
                 atomicAdd(acc + NSLOT, t.a_clamp);
-            if (t.a_bnd != 0)
-                atomicAdd(acc + 3 * NSLOT, t.a_bnd);
+            if (GEN && t.a_sea != 0)
+                atomicAdd(acc + 2 * NSLOT, t.a_sea);
+            AccT bnd = t.a_bnd;
+            for (int q = 0; q < 2 * BLK_ROWS; q++)
+                bnd += (AccT)t.bnd[q >> 1][q & 1];
+            if (bnd != 0)
+                atomicAdd(acc + 3 * NSLOT, bnd);
             if (t.cap)
                 atomicAdd(&ctl->cap[slot], (unsigned long long)t.cap);
         }
@@ -555,25 +629,46 @@ struct BlockSweep {
             // ---- A: x faces of row i; y (and diagonal) faces of rows i-1, i
             f2 Y1, E1 = z0, W1 = z0;
             {
-                const f2 z = sld(tb + BLK_Z + 2 * BLK_ROW_B), n = sld(tb + BLK_N + 2 * BLK_ROW_B);
-                const f2 L = add2(z, sld(tb + BLK_H + 2 * BLK_ROW_B));
-                const f2 zp = sld(tb + BLK_Z + BLK_ROW_B), npv = sld(tb + BLK_N + BLK_ROW_B);
-                const f2 Lp = add2(zp, sld(tb + BLK_H + BLK_ROW_B));
+                f2 z = sld(tb + BLK_Z + 2 * BLK_ROW_B);
+                const f2 n = sld(tb + BLK_N + 2 * BLK_ROW_B);
+                f2 L = add2(z, sld(tb + BLK_H + 2 * BLK_ROW_B));
+                f2 zp = sld(tb + BLK_Z + BLK_ROW_B);
+                const f2 npv = sld(tb + BLK_N + BLK_ROW_B);
+                f2 Lp = add2(zp, sld(tb + BLK_H + BLK_ROW_B));
+                bool odd = false;           // a cell of the two rows is not LAND
+                if constexpr (GEN) {
+                    odd = lo2(n) != lo2(n) || hi2(n) != hi2(n) || lo2(npv) != lo2(npv) ||
+                          hi2(npv) != hi2(npv);
+                    odd = __any_sync(0xffffffffu, odd);
+                    if (odd) {
+                        const float zs = FCAB_SV(k.z_sea);
+                        sea_levels(z, L, n, zs);
+                        sea_levels(zp, Lp, npv, zs);
+                    }
+                }
                 const f2 zr = right2(z), Lr = right2(L), nrr = right2(n);
                 const f2 dx = FCAB_KC(dx), nrdx = FCAB_KC(nrdx);
                 const float tau_l = slf(sb + KC + (uint32_t)offsetof(BlkK, tau_l));
                 const float tau_h = slf(sb + KC + (uint32_t)offsetof(BlkK, tau_h));
                 BlkFace f[NF];
                 bool unsure = false, crit = false;
-                f[0] = blk_face_v<MATH>(L, Lr, z, zr, n, nrr, dx, nrdx, tau_l, tau_h, unsure);
-                f[1] = blk_face_v<MATH>(Lp, L, zp, z, npv, n, dx, nrdx, tau_l, tau_h, unsure);
+                f2 nx = add2(n, nrr), ny = add2(npv, n);
+                if (GEN && odd) {
+                    nx = nsum2(n, nrr);
+                    ny = nsum2(npv, n);
+                }
+                f[0] = blk_face_v<MATH>(L, Lr, z, zr, nx, dx, nrdx, tau_l, tau_h, unsure);
+                f[1] = blk_face_v<MATH>(Lp, L, zp, z, ny, dx, nrdx, tau_l, tau_h, unsure);
                 if constexpr (K == 8) {
                     const f2 zpr = right2(zp), Lpr = right2(Lp), npr = right2(npv);
                     const f2 dd = FCAB_KC(dd), nrdd = FCAB_KC(nrdd);
-                    f[2] = blk_face_v<MATH>(Lp, Lr, zp, zr, npv, nrr, dd, nrdd, tau_l, tau_h,
-                                            unsure);
-                    f[3] = blk_face_v<MATH>(Lpr, L, zpr, z, npr, n, dd, nrdd, tau_l, tau_h,
-                                            unsure);
+                    f2 ne = add2(npv, nrr), nw = add2(npr, n);
+                    if (GEN && odd) {
+                        ne = nsum2(npv, nrr);
+                        nw = nsum2(npr, n);
+                    }
+                    f[2] = blk_face_v<MATH>(Lp, Lr, zp, zr, ne, dd, nrdd, tau_l, tau_h, unsure);
+                    f[3] = blk_face_v<MATH>(Lpr, L, zpr, z, nw, dd, nrdd, tau_l, tau_h, unsure);
                 }
                 if constexpr (MATH == MATH_EXACT) {
                     if (__any_sync(0xffffffffu, unsure)) {
@@ -609,6 +704,9 @@ struct BlockSweep {
                     keep(rb + BLK_E, E1, last2, over);
                     keep(rb + BLK_W, W1, last2, over);
                 }
+                if ((edges & 12) && wp == BLK_ROWS - 1)
+                    open_ends(tl, sb, tb - lane * 8 - wp * BLK_ROW_B, r + 2 - wp, r0, r1, c_first,
+                              nr, nc, edges, lane);
                 if ((unsigned)(rel + 2) < (unsigned)H)
                     ss.capn += cx;
                 if ((unsigned)(rel + 1) < (unsigned)H)
@@ -636,13 +734,22 @@ struct BlockSweep {
                 }
                 const f2 hp = sld(tb + BLK_H + BLK_ROW_B);
                 if (spec && open_row(edges, r + 1, nr)) {
-                    const OpenPair o = open_pair(tb + BLK_ROW_B, sb + KC, sb + SV);
+                    const OpenPair o = open_pair(sld(tb + BLK_Z + BLK_ROW_B), hp,
+                                                 sld(tb + BLK_N + BLK_ROW_B), sb + KC, sb + SV);
                     int k0, k1;
                     open_sides(r + 1, cbase, nr, nc, g.r_lo, g.r_hi, edges, k0, k1);
+                    if constexpr (GEN) {        // LAND cells only
+                        const f2 n = sld(tb + BLK_ROW_B + BLK_N);
+                        k0 = lo2(n) == lo2(n) ? k0 : 0;
+                        k1 = hi2(n) == hi2(n) ? k1 : 0;
+                    }
                     if ((unsigned)(rel + 1) < (unsigned)H)
                         ss.capn += (o.cap & 1u ? k0 : 0) + (o.cap & 2u ? k1 : 0);
                     out = add2(out, mk2(open_sum<float>(lo2(o.q), k0),
                                         open_sum<float>(hi2(o.q), k1)));
+                } else if (edges & 12) {
+                    out = add2(out, end_flow(tl, r + 1, cbase, nr, nc, g.r_lo, g.r_hi, edges,
+                                             bc2(1.0f)));
                 }
                 const f2 ov = mul2(out, FCAB_KC(dt));
                 const f2 hold = mul2(hp, FCAB_KC(A));
@@ -668,23 +775,72 @@ struct BlockSweep {
             {
                 const f2 S2 = sld(rb + BLK_S + BLK_ROW_B), S3 = sld(rb + BLK_S);
                 const f2 sr = right2(S2);
-                const f2 Qsx = upwind2(sld(rb + BLK_X), S2, sr);
-                f2 net = sub2(left2(Qsx), Qsx);
-                net = sub2(net, upwind2(Y2, S2, S1));
-                net = add2(net, upwind2(sld(rb + BLK_Y), S3, S2));
+                const f2 Qr = upwind2(sld(rb + BLK_X), S2, sr), Ql = left2(Qr);
+                const f2 Qd = upwind2(Y2, S2, S1), Qu = upwind2(sld(rb + BLK_Y), S3, S2);
+                f2 net = sub2(Ql, Qr);
+                net = sub2(net, Qd);
+                net = add2(net, Qu);
+                f2 Qrd = z0, Qlu = z0, Qld = z0, Qru = z0;
                 if constexpr (K == 8) {
-                    net = sub2(net, upwind2(E2, S2, right2(S1)));
-                    net = add2(net, left2(upwind2(sld(rb + BLK_E), S3, sr)));
-                    net = sub2(net, left2(upwind2(W2, sr, S1)));
-                    net = add2(net, upwind2(sld(rb + BLK_W), right2(S3), S2));
+                    Qrd = upwind2(E2, S2, right2(S1));
+                    Qlu = left2(upwind2(sld(rb + BLK_E), S3, sr));
+                    Qld = left2(upwind2(W2, sr, S1));
+                    Qru = upwind2(sld(rb + BLK_W), right2(S3), S2);
+                    net = sub2(net, Qrd);
+                    net = add2(net, Qlu);
+                    net = sub2(net, Qld);
+                    net = add2(net, Qru);
+                }
+                bool l0 = true, l1 = true, odd = false;     // LAND cells; a row with others
+                if constexpr (GEN) {
+                    const f2 n = sld(tb + BLK_N);
+                    l0 = lo2(n) == lo2(n);
+                    l1 = hi2(n) == hi2(n);
+                    odd = __any_sync(0xffffffffu, !l0 || !l1);
+                    if (odd) {
+                        // what SEA cells receive has left the domain (model.c:241-319,
+                        // there counted by the LAND cell of the face)
+                        const f2 z = sld(tb + BLK_Z);
+                        const bool own = own2 && out_lane;
+                        const bool sea0 = own && lo2(z) < -1e29f && cbase >= 0 && cbase < nc;
+                        const bool sea1 = own && hi2(z) < -1e29f && cbase + 1 >= 0 &&
+                                          cbase + 1 < nc;
+                        AccT sea = 0;
+                        const float dt = FCAB_SV(dt);
+#pragma unroll
+                        for (int j = 0; j < 2; j++) {
+                            if (j == 0 ? sea0 : sea1) {
+                                sea += acc_mul<AccT, float>(dt, -get2(Qr, j)) +
+                                       acc_mul<AccT, float>(dt, get2(Ql, j)) +
+                                       acc_mul<AccT, float>(dt, -get2(Qd, j)) +
+                                       acc_mul<AccT, float>(dt, get2(Qu, j));
+                                if constexpr (K == 8)
+                                    sea += acc_mul<AccT, float>(dt, -get2(Qrd, j)) +
+                                           acc_mul<AccT, float>(dt, get2(Qlu, j)) +
+                                           acc_mul<AccT, float>(dt, -get2(Qld, j)) +
+                                           acc_mul<AccT, float>(dt, get2(Qru, j));
+                            }
+                        }
+                        if (__any_sync(0xffffffffu, sea != 0)) {
+                            sea = warp_sum(sea);
+                            if (lane == 0)
+                                atomicAdd(&tl.a_sea, sea);
+                        }
+                    }
                 }
                 const f2 h = sld(tb + BLK_H);
                 if (spec && open_row(edges, r, nr)) {
                     // open-edge outflow scaled by the cell's own limiter
                     // (model.c:553-559), summed over its open slots
-                    const OpenPair o = open_pair(tb, sb + KC, sb + SV);
+                    const OpenPair o = open_pair(sld(tb + BLK_Z), h, sld(tb + BLK_N), sb + KC,
+                                                 sb + SV);
                     int k0, k1;
                     open_sides(r, cbase, nr, nc, g.r_lo, g.r_hi, edges, k0, k1);
+                    if constexpr (GEN) {        // LAND cells only
+                        const f2 n = sld(tb + BLK_N);
+                        k0 = lo2(n) == lo2(n) ? k0 : 0;
+                        k1 = hi2(n) == hi2(n) ? k1 : 0;
+                    }
                     const f2 qs = mul2_sep(o.q, S2);
                     const float q0 = open_sum<float>(lo2(qs), k0);
                     const float q1 = open_sum<float>(hi2(qs), k1);
@@ -696,6 +852,16 @@ struct BlockSweep {
                     bnd = warp_sum(bnd);
                     if (lane == 0 && bnd != 0)
                         atomicAdd(&tl.a_bnd, bnd);
+                } else if (edges & 12) {
+                    const f2 qs = end_flow(tl, r, cbase, nr, nc, g.r_lo, g.r_hi, edges, S2);
+                    net = sub2(net, qs);
+                    // at most one lane each holds column 0 and column nc-1
+                    if (own2 && out_lane && (lo2(qs) != 0.0f || hi2(qs) != 0.0f)) {
+                        const float dt = FCAB_SV(dt);
+                        tl.bnd[wp][cbase == 0 ? 0 : 1] +=
+                            (double)(acc_mul<AccT, float>(dt, lo2(qs)) +
+                                     acc_mul<AccT, float>(dt, hi2(qs)));
+                    }
                 }
                 f2 rain;
                 if constexpr (RAINF) {
@@ -711,17 +877,19 @@ struct BlockSweep {
                 else
                     dq = mul2(net, FCAB_KC(invA));
                 f2 hu = add2(h, add2(mul2_sep(FCAB_KC(dt), dq), rain));
+                if (GEN && odd)
+                    hu = sel2(l0, l1, hu, z0);
                 if (__any_sync(0xffffffffu, lo2(hu) < 0.0f || hi2(hu) < 0.0f)) {
                     float a0 = lo2(hu), a1 = hi2(hu);
                     const bool own = own2 && out_lane;
                     const float A = FCAB_SV(A);
                     if (a0 < 0.0f) {
-                        if (own && cbase >= 0 && cbase < nc)
+                        if (own && l0 && cbase >= 0 && cbase < nc)
                             atomicAdd(&tl.a_clamp, acc_mul<AccT, float>(-a0, A));
                         a0 = 0.0f;
                     }
                     if (a1 < 0.0f) {
-                        if (own && cbase + 1 >= 0 && cbase + 1 < nc)
+                        if (own && l1 && cbase + 1 >= 0 && cbase + 1 < nc)
                             atomicAdd(&tl.a_clamp, acc_mul<AccT, float>(-a1, A));
                         a1 = 0.0f;
                     }
@@ -748,6 +916,12 @@ struct BlockSweep {
                     hu = sel2(in0, in1, hu, h);
                     rain = sel2(in0, in1, rain, z0);
                 }
+                if (GEN && odd) {
+                    const float zs = FCAB_SV(k.z_sea), nan = __int_as_float(0x7fc00000);
+                    Ln = sel2(l0, l1, Ln, mk2(lo2(z) < -1e29f ? zs : nan,
+                                              hi2(z) < -1e29f ? zs : nan));
+                    hu = sel2(l0, l1, hu, h);
+                }
                 keep(rb + BLK_L, Ln, last2, over);
                 if (own2 && out_lane) {
                     if constexpr (sizeof(AccT) == 4) {
@@ -757,16 +931,19 @@ struct BlockSweep {
                         ss.rain_sum += (double)lo2(rain) + (double)hi2(rain);
                     }
                     // a cell that could raise the velocity maximum
-                    cand = lo2(hu) >= hcut || hi2(hu) >= hcut;
+                    cand = (l0 && lo2(hu) >= hcut) || (l1 && hi2(hu) >= hcut);
                     const f2 hm = sld(tb + BLK_M);                  // hmax of row i-2
                     const uint64_t ho = sld(sb + SV + (uint32_t)offsetof(StepVals<float>, hout)).u;
                     st2(reinterpret_cast<float *>(ho) + off2, hu);
-                    st2(g.hmax + off2, max2(hu, hm));
+                    f2 hx = max2(hu, hm);
+                    if (GEN && odd)
+                        hx = sel2(l0, l1, hx, hm);
+                    st2(g.hmax + off2, hx);
                     float *const tmx = g.tmax + off2;
                     const float tv = FCAB_SV(tmax_val);
-                    if (lo2(hu) > lo2(hm))
+                    if (l0 && lo2(hu) > lo2(hm))
                         tmx[0] = tv;
-                    if (hi2(hu) > hi2(hm))
+                    if (l1 && hi2(hu) > hi2(hm))
                         tmx[1] = tv;
                 }
             }
@@ -784,7 +961,7 @@ struct BlockSweep {
                 if (tl.sv.want_v && (unsigned)(rel - 1) < (unsigned)H)
                     velocity_row(tl, g, sld(rb + BLK_L + BLK_ROW_B),
                                  sld(rb + BLK_L + 2 * BLK_ROW_B), sld(rb + BLK_L), r - 1, cbase,
-                                 open_row(edges, r - 1, nr) ? edges : 0,
+                                 edges,
                                  out_lane && cbase >= 0 && cbase < nc,
                                  out_lane && cbase + 1 >= 0 && cbase + 1 < nc, off2 - pitch, thr,
                                  hcut);
@@ -829,10 +1006,15 @@ struct BlockSweep {
         }
         // a candidate's new depth was stored by this CTA before the last barrier
         const f2 hv = in0 || in1 ? ld2_rw(sv.hout + off) : z0;
-        const bool e0 = in0 && lo2(hv) >= hcut, e1 = in1 && hi2(hv) >= hcut;
+        bool e0 = in0 && lo2(hv) >= hcut, e1 = in1 && hi2(hv) >= hcut;
         if (!(e0 || e1))
             return;
-        if (edges) {
+        const f2 nv = ld2(g.n + off);
+        if constexpr (GEN) {
+            e0 = e0 && lo2(nv) == lo2(nv);
+            e1 = e1 && hi2(nv) == hi2(nv);
+        }
+        if ((edges & 12) || open_row(edges, r, g.nr)) {
             // the open virtual neighbour z - S_bnd*dx, h = 0 (physics.h:183-189)
             const bool erow = (r == 0 && (edges & 1)) || (r == g.nr - 1 && (edges & 2));
             const f2 zz = ld2(g.z + off);
@@ -844,7 +1026,6 @@ struct BlockSweep {
                     put2(mo, j, fmaxf(get2(mo, j), get2(dv, j)));
             }
         }
-        const f2 nv = ld2(g.n + off);
         const f2 n2 = mul2(nv, nv);
         f2 S = mul2(mo, bc2(sv.k.rdx));
         if constexpr (K == 8)

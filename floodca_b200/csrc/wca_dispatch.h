@@ -16,7 +16,7 @@ struct VariantKey {
     int math;   // MATH_*
     int rainf;  // per-cell rain field
     int landonly; // every cell LAND (mask not read, padding at PAD_Z)
-    int blk = 0;  // FP32 all-LAND: the block sweep (needs the session's row maps)
+    int blk = 0;  // FP32: the block sweep (needs the session's row maps and coded mask)
     int solo = 0; // block sweep: a missed seed's velocity pass by the last CTA
 };
 
@@ -112,37 +112,36 @@ Launchers make_launchers()
     return L;
 }
 
-template <typename AccT, int K, int MATH, bool RAINF, bool TAILV>
+template <typename AccT, int K, int MATH, bool RAINF, bool GEN, bool TAILV>
 cudaError_t launch_step_blk(const void *g, const void *rk, const TimeCfg &tc, Ctl *ctl, int seg,
                             int grid, cudaStream_t s, int smem)
 {
-    k_step_blk<AccT, K, MATH, RAINF, TAILV><<<grid, BLK_THREADS, smem, s>>>(
+    k_step_blk<AccT, K, MATH, RAINF, GEN, TAILV><<<grid, BLK_THREADS, smem, s>>>(
         *static_cast<const GridD<float> *>(g), *static_cast<const RunK<float> *>(rk), tc, ctl,
         seg);
     return cudaGetLastError();
 }
 
-template <typename AccT, int K, int MATH, bool RAINF, bool TAILV>
+template <typename AccT, int K, int MATH, bool RAINF, bool GEN, bool TAILV>
 Launchers make_launchers_blk()
 {
     Launchers L;
-    L.step = &launch_step_blk<AccT, K, MATH, RAINF, TAILV>;
+    L.step = &launch_step_blk<AccT, K, MATH, RAINF, GEN, TAILV>;
     L.init = &launch_init<float, K, MATH>;
-    L.step_fn = (const void *)&k_step_blk<AccT, K, MATH, RAINF, TAILV>;
+    L.step_fn = (const void *)&k_step_blk<AccT, K, MATH, RAINF, GEN, TAILV>;
     L.threads = BLK_THREADS;
     L.tma_smem = blk_smem_bytes<K>();
     L.blk = 1;
     return L;
 }
 
-template <typename AccT, int K, int MATH>
+template <typename AccT, int K, int MATH, bool TAILV>
 Launchers pick_launchers_blk(const VariantKey &k)
 {
-    if (k.solo)
-        return k.rainf ? make_launchers_blk<AccT, K, MATH, true, false>()
-                       : make_launchers_blk<AccT, K, MATH, false, false>();
-    return k.rainf ? make_launchers_blk<AccT, K, MATH, true, true>()
-                   : make_launchers_blk<AccT, K, MATH, false, true>();
+    if (!k.landonly)
+        return make_launchers_blk<AccT, K, MATH, true, true, TAILV>();
+    return k.rainf ? make_launchers_blk<AccT, K, MATH, true, false, TAILV>()
+                   : make_launchers_blk<AccT, K, MATH, false, false, TAILV>();
 }
 
 // Expands the (K, CPL, RAINF) combinations for one (T, AccT, MATH).
@@ -150,9 +149,13 @@ template <typename T, typename AccT, int MATH>
 bool lookup_kcr(const VariantKey &k, Launchers *out)
 {
     if constexpr (sizeof(T) == 4) {
-        if (k.blk && k.landonly) {
-            *out = k.K == 4 ? pick_launchers_blk<AccT, 4, MATH>(k)
-                            : pick_launchers_blk<AccT, 8, MATH>(k);
+        if (k.blk) {
+            if (k.K == 4)
+                *out = k.solo ? pick_launchers_blk<AccT, 4, MATH, false>(k)
+                              : pick_launchers_blk<AccT, 4, MATH, true>(k);
+            else
+                *out = k.solo ? pick_launchers_blk<AccT, 8, MATH, false>(k)
+                              : pick_launchers_blk<AccT, 8, MATH, true>(k);
             return true;
         }
     }

@@ -1407,11 +1407,11 @@ __device__ __forceinline__ T velocity_at(const GridD<T> &g, const RunK<T> &rk, c
 // (TAILV = false) the last CTA does a missed seed's velocity pass itself
 // instead of launching it. Measured, us a step: 61 x 93 14.5 -> 9.0, 256^2
 // 18.2 -> 11.1, 512^2 19.3 -> 14.3, 1024^2 27.8 -> 25.2.
-template <typename AccT, int K, int MATH, bool RAINF, bool TAILV>
+template <typename AccT, int K, int MATH, bool RAINF, bool GEN, bool TAILV>
 __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
     k_step_blk(GridD<float> g, RunK<float> rk, TimeCfg tc, Ctl *ctl, int seg)
 {
-    using Sweep = BlockSweep<AccT, K, MATH, RAINF>;
+    using Sweep = BlockSweep<AccT, K, MATH, RAINF, GEN>;
     using G = Geom<2>;
     const int active = ctl->active, h_cur = ctl->h_cur;
     if (active == 0)

@@ -129,6 +129,23 @@ __global__ void k_make_cr(const T *C, const T *R, const uint8_t *m, T *cr, long 
         atomicMin(&mm[2], bad);
 }
 
+// The mask in the device copies of z and n: n NaN on cells that are not LAND,
+// z PAD_Z on WALL and -PAD_Z on SEA (no other kernel reads z or n of such
+// cells, nor are they given back).
+__global__ void k_encode_mask(const uint8_t *m, float *z, float *n, long long pitch, int nr, int nc)
+{
+    const long long N = (long long)nr * nc;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
+         i += (long long)gridDim.x * blockDim.x) {
+        const long long a = (i / nc + PADR) * pitch + i % nc + PADC;
+        const uint8_t v = m[a];
+        if (v == M_LAND)
+            continue;
+        z[a] = v == M_SEA ? (float)-PAD_Z : (float)PAD_Z;
+        n[a] = __int_as_float(0x7fc00000);
+    }
+}
+
 size_t esize_of(int prec) { return prec == FCAB_PREC_F64 ? 8 : 4; }
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
@@ -615,11 +632,14 @@ static int upload_common(FcabSim *s, const void *z, const void *h, const void *n
     s->land_cells = 0;
     s->open_faces = 0;
     const bool open = c.boundary == FCA_BND_OPEN;
+    uint8_t mask_max = 0;
     for (long long r = 0; r < c.nrows; r++) {
         const uint8_t *row = mh + r * c.ncols;
         long long cnt = 0;
-        for (long long k = 0; k < c.ncols; k++)
+        for (long long k = 0; k < c.ncols; k++) {
             cnt += row[k] == M_LAND;
+            mask_max = std::max(mask_max, row[k]);
+        }
         s->land_cells += cnt;
         if (open) {
             s->open_faces += (r == 0 && c.edge_n ? cnt : 0) + (r == c.nrows - 1 && c.edge_s ? cnt : 0);
@@ -639,6 +659,17 @@ static int upload_common(FcabSim *s, const void *z, const void *h, const void *n
         k_fill_all<<<1024, 256, 0, s->stream>>>(s->z, (long long)s->nelem, PAD_Z, (int)es);
         CUDA_TRY(cudaGetLastError());
         CUDA_TRY(put_field(s, s->z, z, es, kind));
+    }
+    // FP32 grids with other cells: the mask goes into z and n (block sweep);
+    // a slab's stays on the sweep by warp, which counts its own sea outflow
+    s->mask_coded = !all_land && es == 4 && s->use_tma && !s->slab && mask_max <= M_WALL;
+    if (s->mask_coded) {
+        k_fill_all<<<1024, 256, 0, s->stream>>>(s->z, (long long)s->nelem, PAD_Z, (int)es);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(put_field(s, s->z, z, es, kind));
+        k_encode_mask<<<1024, 256, 0, s->stream>>>(s->m, (float *)s->z, (float *)s->n, s->pitch,
+                                                   (int)c.nrows, (int)c.ncols);
+        CUDA_TRY(cudaGetLastError());
     }
     int inflow_ok = 0;
     if (c.inflow_cell >= 0 && c.inflow_cell < Nup)
@@ -701,9 +732,10 @@ static int resolve_variant(FcabSim *s)
     if (s->esize == 4 && key.landonly && (key.cpl == 2 || key.cpl == 4) &&
         (long long)(s->cfg.nrows + s->hn + s->hs + 2 * PADR) * s->pitch >= (1ll << 31))
         key.cpl = s->cpl = 1;
-    // FP32 all-LAND grids run the block sweep (two columns per lane) unless
-    // one or four columns per lane are asked for
-    key.blk = s->use_tma && key.landonly && (key.cpl == 2 || s->cfg.cols_per_lane == 0) &&
+    // FP32 grids run the block sweep (two columns per lane) unless one or four
+    // columns per lane are asked for
+    key.blk = s->use_tma && (key.landonly || s->mask_coded) && s->cfg.tau_h > 0.0 &&
+              (key.cpl == 2 || s->cfg.cols_per_lane == 0) &&
               (long long)(s->cfg.nrows + s->hn + s->hs + 2 * PADR) * s->pitch < (1ll << 31);
     if (key.blk)
         key.cpl = s->cpl = 2;
@@ -751,7 +783,9 @@ static void grid_view(FcabSim *s, GridD<T> &g)
 {
     g.z = (const T *)s->z;
     g.n = (const T *)s->n;
-    g.cr = s->rain_field ? (const T *)s->cr : nullptr;
+    // the block sweep of masked grids reads the rain as a field, uniform or not
+    g.cr = s->rain_field || (s->have_variant && s->L.blk && !s->landonly) ? (const T *)s->cr
+                                                                          : nullptr;
     g.m = s->m;
     g.h0 = (T *)s->h0;
     g.h1 = (T *)s->h1;

@@ -28,6 +28,7 @@ struct FcabSim {
     fcab::RunK<double> rkd;
     fcab::TimeCfg tc;
     bool rain_field = false;
+    bool mask_coded = false;     // z and n carry the mask (k_encode_mask)
     bool landonly = false;       // mask-free kernel variant (all cells LAND)
     int cpl = 2, grid = 1, warps_total = 4, occupancy = 1;
     int split = 4;               // how the grid shares the rows (Launchers::step)

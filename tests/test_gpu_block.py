@@ -1,4 +1,4 @@
-"""The block sweep (FP32 all-LAND grids) against the oracle, at the sizes
+"""The block sweep (FP32 grids) against the oracle, at the sizes
 where its decomposition can go wrong: grids narrower than a strip, one column
 past a strip, one row, rows one short of and one past a pass of eight, units
 cut to one row, open edges at every side, an inflow cell on a strip's border,
@@ -33,8 +33,8 @@ def _check(dom, p, **kw):
     got = run_session(dom, p, precision="f32", **kw)
     assert got["step"] == want["step"] and got["t"] == want["t"]
     for k in ("h", "hmax", "tmax"):
-        assert np.array_equal(got[k], want[k]), k
-    for k in ("V_rain", "V_bnd", "clamp_err", "V_in"):
+        assert np.array_equal(got[k], want[k], equal_nan=True), k
+    for k in ("V_rain", "V_bnd", "V_sea", "clamp_err", "V_in"):
         assert got[k] == pytest.approx(want[k], rel=1e-9, abs=1e-9), k
     assert got["cap_active"] == want["cap_active"]
     assert got["cap_total"] == want["cap_total"]
@@ -87,3 +87,35 @@ def test_block_sweep_tiny_manning_and_dry_start():
     _check(dom, RunParams(steps=30, T_sim=1e6))
     dom.h[:] = 0.0
     _check(dom, RunParams(steps=30, T_sim=1e6, hyeto="uniform"))
+
+
+@pytest.mark.parametrize("seed", range(60))
+def test_block_sweep_random_masks(seed):
+    """SEA and WALL cells anywhere, also under open edges."""
+    dom, p = _case(7000 + seed)
+    _check(dom, p)
+
+
+@pytest.mark.parametrize("K", [4, 8])
+@pytest.mark.parametrize("size", [(9, 55), (61, 93), (70, 113)])
+@pytest.mark.parametrize("rain_field", [False, True])
+def test_block_sweep_coast(size, K, rain_field):
+    """A shore, wall blocks, and nodata (NaN, infinite, negative) in the
+    rasters of cells that are not LAND, which the model never reads."""
+    nr, nc = size
+    dom = _grid(nr, nc, nr + nc, rain_field, h0=0.5)
+    rng = np.random.default_rng(nc)
+    rr, cc = np.mgrid[0:nr, 0:nc]
+    dom.mask[(rr > 0.8 * nr + 2 * np.sin(0.3 * cc)) | (cc < 2)] = 1
+    dom.mask[rng.random((nr, nc)) < 0.05] = 2
+    off = dom.mask != 0
+    dom.z[off] = rng.choice(np.float32([np.nan, np.inf, -9999.0, 3.0]), off.sum())
+    dom.n[off] = rng.choice(np.float32([np.nan, 0.0, -1.0]), off.sum())
+    dom.h[off] = rng.choice(np.float32([np.nan, np.inf, -9999.0, 0.0, 2.5]), off.sum())
+    for z_sea in (0.0, 6.0):
+        p = RunParams(K=K, steps=30, T_sim=1e6, out_every=600.0, z_sea=z_sea)
+        _check(dom, p)
+        _check(dom, p.with_(edges=(0, 1, 1, 0), hyeto="uniform"), seg_rows=3)
+    _check(dom, RunParams(K=K, steps=12, T_sim=1e6, boundary="closed",
+                          inflow_cell=int(np.flatnonzero(dom.mask.ravel() == 0)[5]),
+                          inflow_peak=50.0, inflow_t_peak=100.0, inflow_t_end=900.0))
