@@ -111,24 +111,22 @@ extern "C" int fcab_batch_create(FcabBatch **out, FcabSim *const *members, int n
     b->key.prec = FCAB_PREC_F32;
     b->key.K = m0->cfg.K;
     b->key.cpl = (cols_per_lane == 1 || cols_per_lane == 2 || cols_per_lane == 4) ? cols_per_lane : 2;
-    if (b->key.K == 8 && b->key.cpl == 4)
-        b->key.cpl = 2;
     b->key.math = m0->cfg.math;
     b->key.rainf = m0->rain_field ? 1 : 0;
     b->key.landonly = m0->landonly ? 1 : 0;
-    // the pair sweep addresses the fields with 32-bit element offsets
-    if (b->key.landonly && b->key.cpl == 2)
-        for (int i = 0; i < n; i++) {
-            const FcabSim *s = members[i];
-            if ((long long)(s->cfg.nrows + s->hn + s->hs + 2 * PADR) * s->pitch >= (1ll << 31))
-                b->key.cpl = 1;
-        }
+    // the block sweep, unless one column per lane is asked for or a member
+    // cannot run it
+    b->key.blk = b->key.cpl != 1;
+    for (int i = 0; i < n && b->key.blk; i++)
+        b->key.blk = runs_block_sweep(members[i]);
+    if (!b->key.blk)
+        b->key.cpl = 1;
     if (!lookup_batch_f32(b->key, &b->L)) {
         delete b;
         return bfail(FCAB_ERR_ARG, "fcab_batch_create: no compiled batch variant");
     }
     b->seg = seg_rows > 0 ? seg_rows : 64;
-    const int ow = 32 * b->key.cpl - 2 * (b->key.cpl == 1 ? 3 : 4);
+    const int ow = b->key.blk ? Geom<2>::OW : Geom<1>::OW;
     std::vector<MemberD<float>> md(n);
     std::vector<int> um;
     for (int i = 0; i < n; i++) {
@@ -136,7 +134,8 @@ extern "C" int fcab_batch_create(FcabBatch **out, FcabSim *const *members, int n
         MemberD<float> &d = md[i];
         d.g.z = (const float *)s->z;
         d.g.n = (const float *)s->n;
-        d.g.cr = s->rain_field ? (const float *)s->cr : nullptr;
+        d.g.cr = s->rain_field || (b->key.blk && !s->landonly) ? (const float *)s->cr : nullptr;
+        d.g.tmap = b->key.blk ? static_cast<const CUtensorMap *>(s->tmaps) : nullptr;
         d.g.m = s->m;
         d.g.h0 = (float *)s->h0;
         d.g.h1 = (float *)s->h1;
@@ -153,6 +152,8 @@ extern "C" int fcab_batch_create(FcabBatch **out, FcabSim *const *members, int n
         d.ctl = s->ctl;
         d.strips = (s->cfg.ncols + ow - 1) / ow;
         d.seg = member_seg_rows && member_seg_rows[i] > 0 ? member_seg_rows[i] : b->seg;
+        if (b->key.blk)     // whole passes: the unit's rows and six halo rows
+            d.seg = (d.seg + 6 + BLK_ROWS - 1) / BLK_ROWS * BLK_ROWS - 6;
         const int blocks = (s->cfg.nrows + d.seg - 1) / d.seg;
         d.units = d.strips * blocks;
         d.unit_off = (int)um.size();
@@ -183,8 +184,12 @@ extern "C" int fcab_batch_create(FcabBatch **out, FcabSim *const *members, int n
     int nsm = 1, per_sm = 1;
     if (e == cudaSuccess)
         e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m0->dev);
+    if (e == cudaSuccess && b->L.smem > 0)
+        e = cudaFuncSetAttribute(b->L.step_fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 b->L.smem);
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->L.step_fn, 128, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->L.step_fn, b->L.threads,
+                                                          b->L.smem);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) {

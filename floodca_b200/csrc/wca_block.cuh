@@ -108,6 +108,20 @@ __host__ __device__ constexpr int blk_smem_bytes()
     return 128 + (int)blk_tail<K>() + (int)sizeof(BlkTail<double>);
 }
 
+__device__ __forceinline__ f2 ld2(const float *p)
+{
+    const float2 v = __ldg(reinterpret_cast<const float2 *>(p));
+    return mk2(v.x, v.y);
+}
+__device__ __forceinline__ f2 ld2_rw(const float *p)
+{
+    const float2 v = *reinterpret_cast<const float2 *>(p);
+    return mk2(v.x, v.y);
+}
+__device__ __forceinline__ void st2(float *p, f2 v)
+{
+    *reinterpret_cast<float2 *>(p) = make_float2(lo2(v), hi2(v));
+}
 // Shared memory by 32-bit shared address.
 __device__ __forceinline__ f2 sld(uint32_t a)
 {
@@ -146,6 +160,59 @@ __device__ __forceinline__ f2 div2_c(f2 a, f2 rc, f2 nc)
 {
     const f2 q = mul2(a, rc);
     return fma2(fma2(q, nc, a), rc, q);
+}
+
+// RN(sqrt(g*hf)) per half of the exact product g*hf (as the reference's
+// (real)sqrt((double)g*(double)hf), physics.h:107-108): from p = RN(g*hf),
+// its error pe = g*hf - p (exact, one fused multiply-add) and s = RN(sqrt(p)),
+// the root of p + pe is s + (p - s^2 + pe)/(2s) to far better than 2^-20 ulp;
+// that sum is rounded to y with its error e (Fast2Sum). `unsure` per half:
+// |e| within 2^-11 of half an ulp of y (tested as fma(e, 1 + 2^-11, y) != y),
+// which also covers the reference's double rounding (its root is rounded to
+// double first, which can only matter within 2^-29 ulp of a midpoint). The
+// exact value is never a float midpoint: a midpoint has 25 significant bits,
+// its square at least 49, and g*hf at most 48.
+__device__ __forceinline__ f2 vcrit2(f2 g, f2 hf, bool &unsure0, bool &unsure1)
+{
+    const f2 p = mul2(g, hf);
+    const f2 pe = fma2(g, hf, neg2(p));
+    const f2 y0 = rsqrt_2(p);
+    const f2 s0 = mul2(p, y0);
+    const f2 h = mul2(bc2(0.5f), y0);
+    const f2 s = fma2(fma2(neg2(s0), s0, p), h, s0);       // RN(sqrt(p))
+    const f2 r = add2(fma2(neg2(s), s, p), pe);              // g*hf - s^2
+    const f2 corr = mul2_sep(r, h);
+    const f2 y = add2(s, corr);
+    const f2 e = add2(sub2(s, y), corr);
+    const f2 chk = fma2(e, bc2(1.00048828125f), y);
+    float y0f, y1f, k0, k1;
+    sp2(y, y0f, y1f);
+    sp2(chk, k0, k1);
+    unsure0 = k0 != y0f;
+    unsure1 = k1 != y1f;
+    return y;
+}
+
+// The exact next-step velocity of the flagged halves (physics.h:193-217),
+// folded into the running maximum vm.
+template <int K, int MATH>
+__device__ __noinline__ float pair_velocity(float vm, bool x0, bool x1, f2 mo, f2 md, f2 hv, f2 nv,
+                                            const StepK<float> *kp)
+{
+    const StepK<float> k = *kp;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        if (j == 0 ? x0 : x1) {
+            float Smax = Mth<float, MATH>::div(get2(mo, j), k.dx);
+            if constexpr (K == 8) {
+                const float Sd = Mth<float, MATH>::div(get2(md, j), k.d_diag);
+                Smax = Sd > Smax ? Sd : Smax;
+            }
+            const float v = cell_velocity<float, MATH>(get2(hv, j), get2(nv, j), Smax, k);
+            vm = v > vm ? v : vm;
+        }
+    }
+    return vm;
 }
 
 // hf^(2/3) per half as cbrt_sq2; `unsure` is raised when either half needs

@@ -32,7 +32,7 @@ struct Launchers {
                         cudaStream_t s, int only_if_needed);
     const void *step_fn;   // __global__ symbol, for occupancy queries
     int threads;           // threads per CTA of the step kernel
-    int tma_smem;          // dynamic shared memory of its TMA row source (0: none)
+    int smem;              // dynamic shared memory of the step kernel
     int blk;               // the block sweep: `grid` CTAs share the rows
 };
 
@@ -45,6 +45,7 @@ struct BatchLaunchers {
                          cudaStream_t s);
     cudaError_t (*window)(const void *members, int n, double window, cudaStream_t s);
     const void *step_fn;
+    int threads, smem;     // per CTA of the step
 };
 bool lookup_batch_f32(const VariantKey &k, BatchLaunchers *out);
 
@@ -54,6 +55,15 @@ cudaError_t launch_batch(const void *members, const int *unit_member, int total_
 {
     k_step_batch<T, AccT, K, CPL, MATH, RAINF, LAND><<<grid, 128, 0, s>>>(
         static_cast<const MemberD<T> *>(members), unit_member, total_units, q, need_list);
+    return cudaGetLastError();
+}
+
+template <typename AccT, int K, int MATH, bool RAINF, bool GEN>
+cudaError_t launch_batch_blk(const void *members, const int *unit_member, int total_units,
+                             BatchQ *q, int *need_list, int grid, cudaStream_t s)
+{
+    k_batch_blk<AccT, K, MATH, RAINF, GEN><<<grid, BLK_THREADS, blk_smem_bytes<K>(), s>>>(
+        static_cast<const MemberD<float> *>(members), unit_member, total_units, q, need_list);
     return cudaGetLastError();
 }
 
@@ -107,7 +117,7 @@ Launchers make_launchers()
     L.init = &launch_init<T, K, MATH>;
     L.step_fn = (const void *)&k_step<T, AccT, K, CPL, MATH, RAINF, LAND>;
     L.threads = step_threads<CPL, MATH>();
-    L.tma_smem = use_pair_sweep<T, K, CPL, LAND>() ? tma_smem_bytes(L.threads / 32) : 0;
+    L.smem = 0;
     L.blk = 0;
     return L;
 }
@@ -130,7 +140,7 @@ Launchers make_launchers_blk()
     L.init = &launch_init<float, K, MATH>;
     L.step_fn = (const void *)&k_step_blk<AccT, K, MATH, RAINF, GEN, TAILV>;
     L.threads = BLK_THREADS;
-    L.tma_smem = blk_smem_bytes<K>();
+    L.smem = blk_smem_bytes<K>();
     L.blk = 1;
     return L;
 }
@@ -144,7 +154,8 @@ Launchers pick_launchers_blk(const VariantKey &k)
                    : make_launchers_blk<AccT, K, MATH, false, false, TAILV>();
 }
 
-// Expands the (K, CPL, RAINF) combinations for one (T, AccT, MATH).
+// Expands the (K, CPL, RAINF) combinations for one (T, AccT, MATH). FP32
+// all-LAND grids run the block sweep, or one column per lane.
 template <typename T, typename AccT, int MATH>
 bool lookup_kcr(const VariantKey &k, Launchers *out)
 {
@@ -161,8 +172,14 @@ bool lookup_kcr(const VariantKey &k, Launchers *out)
     }
 #define FCAB_CASE(KK, CC, RR)                                                    \
     if (k.K == KK && k.cpl == CC && (k.rainf != 0) == RR) {                      \
-        *out = k.landonly ? make_launchers<T, AccT, KK, CC, MATH, RR, true>()   \
-                          : make_launchers<T, AccT, KK, CC, MATH, RR, false>(); \
+        if (k.landonly) {                                                        \
+            if constexpr (sizeof(T) == 4 && CC != 1)                             \
+                return false;                                                    \
+            else                                                                 \
+                *out = make_launchers<T, AccT, KK, CC, MATH, RR, true>();        \
+        } else {                                                                 \
+            *out = make_launchers<T, AccT, KK, CC, MATH, RR, false>();           \
+        }                                                                        \
         return true;                                                             \
     }
     FCAB_CASE(4, 1, false) FCAB_CASE(4, 1, true)

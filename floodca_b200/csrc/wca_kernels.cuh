@@ -1201,37 +1201,9 @@ __device__ __forceinline__ void publish_sums(StepSums<T, AccT> &ss, const StepVa
 
 }  // namespace fcab
 
-#include "wca_sweep_f2.cuh"
-#include "wca_sweep_f4.cuh"
 #include "wca_block.cuh"
 
 namespace fcab {
-
-// The pair sweep runs the FP32 all-LAND K = 4 grids at two columns per
-// lane; every other variant runs sweep_segment (all of them with
-// FCAB_PAIR_SWEEP=0, a build option for comparing the two).
-#ifndef FCAB_PAIR_SWEEP
-#define FCAB_PAIR_SWEEP 1
-#endif
-// For K = 8 the scalar sweep is the faster of the two (measured at 4096^2
-// on a B200: 24.8 against 23.4 Gcell/s exact, 36.4 against 32.5 fast; the
-// pair sweep's K = 8 face state leaves it 8 warps per SM); FCAB_PAIR_K8=1
-// runs K = 8 on the pair sweep too.
-#ifndef FCAB_PAIR_K8
-#define FCAB_PAIR_K8 0
-#endif
-template <typename T, int K, int CPL, bool LANDONLY>
-__host__ __device__ constexpr bool use_pair_sweep()
-{
-    return FCAB_PAIR_SWEEP && sizeof(T) == 4 && CPL == 2 && LANDONLY && (K == 4 || FCAB_PAIR_K8);
-}
-// The four-column sweep (two pairs per lane) runs the FP32 all-LAND K = 4
-// grids at four columns per lane.
-template <typename T, int K, int CPL, bool LANDONLY>
-__host__ __device__ constexpr bool use_quad_sweep()
-{
-    return FCAB_PAIR_SWEEP && sizeof(T) == 4 && CPL == 4 && K == 4 && LANDONLY;
-}
 
 // Launch shape of the step kernel: threads per CTA and the resident warps
 // per SM the register allocation aims for (65536 / (32 x warps) registers
@@ -1259,51 +1231,6 @@ __host__ __device__ constexpr int step_min_blocks()
                             : CPL == 2 ? (MATH == MATH_EXACT && K == 4 ? 16 : 12) : 8)) /
            (step_threads<CPL, MATH>() / 32);
 }
-// Resident warps per SM the pair sweep's register allocation aims for.
-// Measured at 4096^2 on a B200 (one-row loop, same box): 16 warps (128
-// registers, about 160 B of spill stores) 44.4-45.1 Gcell/s, 12 warps (160
-// registers, no spills) 41.2-41.4, 20 warps (96 registers, 532 B of
-// spills) 37.4, 8 warps 30.5-31.3: occupancy outweighs the spills up to 16.
-#ifndef FCAB_PAIR_WARPS
-#define FCAB_PAIR_WARPS 16
-#endif
-// K = 8 holds twice the face state: 8 warps (up to 255 registers, no spills)
-#ifndef FCAB_PAIR_WARPS_K8
-#define FCAB_PAIR_WARPS_K8 8
-#endif
-template <int K>
-__host__ __device__ constexpr int pair_warps()
-{
-    return K == 8 ? FCAB_PAIR_WARPS_K8 : FCAB_PAIR_WARPS;
-}
-// The batched step keeps a member descriptor and step constants per warp
-// besides the sweep state. With stage E's depth and n and the hmax row out
-// of the register ring it spills 108 B at 16 warps (128 registers), and the
-// config-4 ensemble (256 members) ran 50.9 G cell-steps/s against 48.8 at
-// 12 warps (168 registers, no spills) on one box.
-#ifndef FCAB_PAIR_WARPS_BATCH
-#define FCAB_PAIR_WARPS_BATCH 16
-#endif
-template <int K>
-__host__ __device__ constexpr int pair_warps_batch()
-{
-    return K == 8 ? FCAB_PAIR_WARPS_K8 : FCAB_PAIR_WARPS_BATCH;
-}
-// Resident warps per SM of the four-column sweep (twice the pair sweep's
-// state per lane: up to 255 registers at 8 warps)
-#ifndef FCAB_QUAD_WARPS
-#define FCAB_QUAD_WARPS 8
-#endif
-template <typename T, int K, int CPL, int MATH, bool LANDONLY>
-__host__ __device__ constexpr int step_blocks_per_sm()
-{
-    return use_pair_sweep<T, K, CPL, LANDONLY>()
-               ? pair_warps<K>() / (step_threads<CPL, MATH>() / 32)
-               : use_quad_sweep<T, K, CPL, LANDONLY>()
-                     ? FCAB_QUAD_WARPS / (step_threads<CPL, MATH>() / 32)
-                     : step_min_blocks<K, CPL, MATH>();
-}
-
 // Resident CTAs of the block sweep the register allocation aims for.
 #ifndef FCAB_BLK_CTAS
 #define FCAB_BLK_CTAS 4
@@ -1514,7 +1441,7 @@ __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
 
 template <typename T, typename AccT, int K, int CPL, int MATH, bool RAINF, bool LANDONLY>
 __global__ void __launch_bounds__(step_threads<CPL, MATH>(),
-                                  step_blocks_per_sm<T, K, CPL, MATH, LANDONLY>()) k_step(GridD<T> g, RunK<T> rk, TimeCfg tc, Ctl *ctl,
+                                  step_min_blocks<K, CPL, MATH>()) k_step(GridD<T> g, RunK<T> rk, TimeCfg tc, Ctl *ctl,
                                               int warps_total)
 {
     using G = Geom<CPL>;
@@ -1532,63 +1459,12 @@ __global__ void __launch_bounds__(step_threads<CPL, MATH>(),
     if (wid >= warps_total)
         w0 = w1 = 0;
 
-    // step constants in shared memory for the pair sweep's exact
-    // re-evaluations; the warps' TMA rings and barriers (dynamic shared memory)
-    __shared__ StepK<T> sk;
-    __shared__ uint32_t tphase[step_threads<CPL, MATH>() / 32];
-    __shared__ int tma_bad;
-    extern __shared__ __align__(1024) unsigned char fcab_dsm[];
-    uint32_t ring = 0u, bars = 0u;
-    const int wib = threadIdx.x >> 5;
-    if constexpr (use_quad_sweep<T, K, CPL, LANDONLY>()) {
-        if (threadIdx.x == 0)
-            sk = sv.k;
-        __syncthreads();
-    }
-    if constexpr (use_pair_sweep<T, K, CPL, LANDONLY>()) {
-        if (threadIdx.x == 0) {
-            sk = sv.k;
-            tma_bad = 0;
-        }
-        // TMA destinations must start on 128-byte boundaries: the rings
-        // start at the dynamic area rounded up to 1024 bytes (the area has
-        // 1 KB of slack for it)
-        const uint32_t dbase = (smem_addr(fcab_dsm) + 1023u) & ~1023u;
-        if (g.tmap) {
-            constexpr int W = step_threads<CPL, MATH>() / 32;
-            ring = dbase + wib * TMA_WARP_B;
-            bars = dbase + W * TMA_WARP_B + wib * TMA_NS * 8;
-            if (lane == 0) {
-                for (int q = 0; q < TMA_NS; q++)
-                    mbar_init1(bars + 8u * q);
-                tphase[wib] = 0u;
-                fence_proxy_async_smem();
-            }
-        }
-        __syncthreads();
-    }
     while (w0 < w1) {
         const int strip = (int)(w0 / nr);
         const int r0 = (int)(w0 % nr);
         const int r1 = (int)min((long long)nr, (long long)r0 + (w1 - w0));
         w0 += r1 - r0;
-        if constexpr (use_pair_sweep<T, K, CPL, LANDONLY>()) {
-            bool bad = false;
-            PairSweep<AccT, K, MATH, RAINF>::run(g, rk, sv, &sk, strip, r0, r1, lane, ss, ring,
-                                                 bars, &tphase[wib], &bad);
-            if (bad && lane == 0)
-                tma_bad = 1;
-        } else if constexpr (use_quad_sweep<T, K, CPL, LANDONLY>()) {
-            QuadSweep<AccT, MATH, RAINF>::run(g, rk, sv, &sk, strip, r0, r1, lane, ss);
-        } else {
-            sweep_segment<T, AccT, K, CPL, MATH, RAINF, LANDONLY>(g, rk, sv, strip, r0, r1, lane,
-                                                                  ss);
-        }
-    }
-    if constexpr (use_pair_sweep<T, K, CPL, LANDONLY>()) {
-        __syncthreads();
-        if (threadIdx.x == 0 && tma_bad)
-            ctl->err = 3;           // a row tile never arrived; the host reports it
+        sweep_segment<T, AccT, K, CPL, MATH, RAINF, LANDONLY>(g, rk, sv, strip, r0, r1, lane, ss);
     }
 
     publish_sums<T, AccT, RAINF>(ss, sv, ctl, lane, wid & (NSLOT - 1));
@@ -1615,14 +1491,13 @@ struct MemberD {
 
 struct BatchQ {
     unsigned int next_unit;
-    unsigned int warps_out;
+    unsigned int warps_out;     // warps (block sweep: CTAs) that found no more units
     unsigned int nneed;         // members whose step deferred its dt (seed missed)
     unsigned int vfull_out;     // CTAs done with the full velocity passes
 };
 
 template <typename T, typename AccT, int K, int CPL, int MATH, bool RAINF, bool LANDONLY>
-__global__ void __launch_bounds__(128, use_pair_sweep<T, K, CPL, LANDONLY>() ? pair_warps_batch<K>() / 4
-                                                                      : (CPL == 2 ? 4 : 1))
+__global__ void __launch_bounds__(128, CPL == 2 ? 4 : 1)
 k_step_batch(const MemberD<T> *members,
                                                     const int *unit_member, int total_units,
                                                     BatchQ *q, int *need_list)
@@ -1670,10 +1545,7 @@ k_step_batch(const MemberD<T> *members,
         __syncwarp();
         const StepVals<T> &sv = ssv[wib];
         StepSums<T, AccT> ss;
-        if constexpr (use_pair_sweep<T, K, CPL, LANDONLY>())
-            PairSweep<AccT, K, MATH, RAINF>::run(g, rk, sv, &ssv[wib].k, strip, r0, r1, lane, ss);
-        else
-            sweep_segment<T, AccT, K, CPL, MATH, RAINF, LANDONLY>(g, rk, sv, strip, r0, r1, lane,
+        sweep_segment<T, AccT, K, CPL, MATH, RAINF, LANDONLY>(g, rk, sv, strip, r0, r1, lane,
                                                                   ss);
         publish_sums<T, AccT, RAINF>(ss, sv, ctl, lane, (int)(u & (NSLOT - 1)));
         if (lane == 0) {
@@ -1695,6 +1567,90 @@ k_step_batch(const MemberD<T> *members,
         __threadfence();
         const unsigned nw = gridDim.x * (blockDim.x >> 5);
         if (atomicAdd(&q->warps_out, 1u) == nw - 1u) {
+            q->next_unit = 0u;
+            q->warps_out = 0u;
+        }
+    }
+}
+
+// The batched step on the block sweep: units (rows of a strip of a member)
+// are taken by CTAs. What a unit starts with (the member's descriptor, its
+// step constants and clock, the first tiles) is 5000 cycles of dependent loads
+// and overlaps with the three other CTAs of the SM. Measured on a B200, us a
+// step, units of 64 rows, against warps taking units: 24 members of side
+// 256..1024 327 -> 193, 24 of side 128..256 193 -> 49, 8 of side 512..1024
+// 216 -> 112.
+template <typename AccT, int K, int MATH, bool RAINF, bool GEN>
+__global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
+    k_batch_blk(const MemberD<float> *members, const int *unit_member, int total_units, BatchQ *q,
+                int *need_list)
+{
+    using Sweep = BlockSweep<AccT, K, MATH, RAINF, GEN>;
+    extern __shared__ __align__(1024) unsigned char fcab_dsm[];
+    __shared__ MemberD<float> md;
+    __shared__ int s_unit[2];
+    static_assert(sizeof(MemberD<float>) % 4 == 0, "word copy");
+    char *const sm = reinterpret_cast<char *>(fcab_dsm) +
+                     ((128u - (smem_addr(fcab_dsm) & 127u)) & 127u);
+    int lane;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+    const int wp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    typename Sweep::Cta T;
+    Sweep::attach(T, sm);
+    if (threadIdx.x == 0) {
+        Sweep::init_barriers(T);
+        s_unit[0] = (int)atomicAdd(&q->next_unit, 1u);
+    }
+    __syncthreads();
+    int par = 0;
+    for (int u = s_unit[0]; u < total_units; u = s_unit[par]) {
+        const int m = unit_member[u];
+        {
+            const unsigned *src = reinterpret_cast<const unsigned *>(members + m);
+            unsigned *dst = reinterpret_cast<unsigned *>(&md);
+            for (int w = threadIdx.x; w < (int)(sizeof(MemberD<float>) / 4); w += BLK_THREADS)
+                dst[w] = src[w];
+        }
+        par ^= 1;
+        if (threadIdx.x == 0)
+            s_unit[par] = (int)atomicAdd(&q->next_unit, 1u);
+        __syncthreads();
+        Ctl *const ctl = md.ctl;
+        if (ctl->active) {
+            const int h_cur = ctl->h_cur;
+            const int local = u - md.unit_off, strip = local % md.strips;
+            const int r0 = local / md.strips * md.seg, r1 = min(md.g.nr, r0 + md.seg);
+            if (lane == 0) {
+                if (wp == 0)
+                    Sweep::first_tiles(T, md.g, h_cur, strip, r0, r1);
+                else if (wp == 1)
+                    Sweep::begin(T, md.g, md.rk, ctl);
+                else if (wp == 2)
+                    T.tail->pre = time_pre(ctl, md.tc, true);
+            }
+            __syncthreads();
+            StepSums<float, AccT> ss;
+            Sweep::run(T, md.g, md.rk, h_cur, strip, r0, r1, wp, lane, ss);
+            __syncthreads();
+            Sweep::publish(T, ss, ctl, lane, u & (NSLOT - 1));
+            if (threadIdx.x == 0) {
+                __threadfence();
+                const unsigned prev = atomicAdd(&ctl->ctas_done, 1u);
+                if (prev == (unsigned)md.units - 1u) {
+                    __threadfence();
+                    ctl->h_cur = h_cur ^ 1;
+                    ctl->launches += 1;
+                    finalize<float>(ctl, md.tc, md.rk, true, T.tail->pre);
+                    if (ctl->need_v)    // seed missed: the full pass after this launch
+                        need_list[atomicAdd(&q->nneed, 1u)] = m;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&q->warps_out, 1u) == gridDim.x - 1u) {
             q->next_unit = 0u;
             q->warps_out = 0u;
         }

@@ -582,7 +582,9 @@ static int upload_common(FcabSim *s, const void *z, const void *h, const void *n
     const size_t es = s->esize;
     if (!z || !h || !mask)
         return fail(FCAB_ERR_ARG, "z, h and mask are required");
-    CUDA_TRY(cudaMemsetAsync(s->z, 0, s->nelem * es, s->stream));
+    // padding elevation PAD_Z: every face to it carries nothing, mask or not
+    k_fill_all<<<1024, 256, 0, s->stream>>>(s->z, (long long)s->nelem, PAD_Z, (int)es);
+    CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemsetAsync(s->h0, 0, s->nelem * es, s->stream));
     CUDA_TRY(cudaMemsetAsync(s->h1, 0, s->nelem * es, s->stream));
     CUDA_TRY(cudaMemsetAsync(s->hmax, 0, s->nelem * es, s->stream));
@@ -655,18 +657,10 @@ static int upload_common(FcabSim *s, const void *z, const void *h, const void *n
         land_up += mup[k] == M_LAND;
     const bool all_land = c.tau_h > 0.0 && s->land_cells == N && land_up == Nup;
     s->landonly = all_land;
-    if (all_land) {
-        k_fill_all<<<1024, 256, 0, s->stream>>>(s->z, (long long)s->nelem, PAD_Z, (int)es);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(put_field(s, s->z, z, es, kind));
-    }
     // FP32 grids with other cells: the mask goes into z and n (block sweep);
     // a slab's stays on the sweep by warp, which counts its own sea outflow
     s->mask_coded = !all_land && es == 4 && s->use_tma && !s->slab && mask_max <= M_WALL;
     if (s->mask_coded) {
-        k_fill_all<<<1024, 256, 0, s->stream>>>(s->z, (long long)s->nelem, PAD_Z, (int)es);
-        CUDA_TRY(cudaGetLastError());
-        CUDA_TRY(put_field(s, s->z, z, es, kind));
         k_encode_mask<<<1024, 256, 0, s->stream>>>(s->m, (float *)s->z, (float *)s->n, s->pitch,
                                                    (int)c.nrows, (int)c.ncols);
         CUDA_TRY(cudaGetLastError());
@@ -715,6 +709,12 @@ extern "C" int fcab_sim_set_rain(FcabSim *s, const void *C, const void *Rday)
     return rebuild_rain(s, false);
 }
 
+bool fcab::runs_block_sweep(const FcabSim *s)
+{
+    return s->esize == 4 && s->use_tma && (s->landonly || s->mask_coded) && s->cfg.tau_h > 0.0 &&
+           (long long)(s->cfg.nrows + s->hn + s->hs + 2 * PADR) * s->pitch < (1ll << 31);
+}
+
 static int resolve_variant(FcabSim *s)
 {
     if (!s->variant_dirty && s->have_variant)
@@ -726,19 +726,14 @@ static int resolve_variant(FcabSim *s)
     key.math = s->cfg.precision == FCAB_PREC_F32 ? s->cfg.math : FCAB_MATH_EXACT;
     key.rainf = s->rain_field ? 1 : 0;
     key.landonly = s->landonly ? 1 : 0;
-    // the pair and four-column sweeps (FP32, all-LAND, two or four columns
-    // per lane) address the fields with 32-bit element offsets: larger grids
-    // take one column per lane
-    if (s->esize == 4 && key.landonly && (key.cpl == 2 || key.cpl == 4) &&
-        (long long)(s->cfg.nrows + s->hn + s->hs + 2 * PADR) * s->pitch >= (1ll << 31))
-        key.cpl = s->cpl = 1;
-    // FP32 grids run the block sweep (two columns per lane) unless one or four
-    // columns per lane are asked for
-    key.blk = s->use_tma && (key.landonly || s->mask_coded) && s->cfg.tau_h > 0.0 &&
-              (key.cpl == 2 || s->cfg.cols_per_lane == 0) &&
-              (long long)(s->cfg.nrows + s->hn + s->hs + 2 * PADR) * s->pitch < (1ll << 31);
-    if (key.blk)
-        key.cpl = s->cpl = 2;
+    // FP32 grids run the block sweep unless one column per lane is asked for;
+    // all-LAND grids that cannot run one column per lane
+    key.blk = s->cfg.cols_per_lane != 1 && runs_block_sweep(s);
+    if (key.blk && s->cfg.cols_per_lane == 0)
+        s->cpl = 2;
+    else if (!key.blk && s->esize == 4 && key.landonly)
+        s->cpl = 1;
+    key.cpl = s->cpl;
     key.solo = (long long)s->cfg.nrows * s->cfg.ncols <= BLK_SOLO;
     bool ok = key.prec == FCAB_PREC_F32 ? lookup_f32(key, &s->L)
               : key.prec == FCAB_PREC_F32_ALL ? lookup_f32all(key, &s->L)
@@ -749,7 +744,7 @@ static int resolve_variant(FcabSim *s)
     // Grid: resident CTAs, or fewer so every warp streams >= seg_rows rows.
     int nsm = 0, per_sm = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->dev));
-    const int smem = s->use_tma ? s->L.tma_smem : 0;
+    const int smem = s->L.smem;
     if (smem > 0)
         CUDA_TRY(cudaFuncSetAttribute(s->L.step_fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       smem));
@@ -796,11 +791,8 @@ static void grid_view(FcabSim *s, GridD<T> &g)
     g.nc = s->cfg.ncols;
     g.r_lo = -s->hn;
     g.r_hi = s->cfg.nrows + s->hs;
-    g.tmap = s->use_tma && s->L.tma_smem > 0 ? static_cast<const CUtensorMap *>(s->tmaps)
-                                             : nullptr;
+    g.tmap = s->L.blk ? static_cast<const CUtensorMap *>(s->tmaps) : nullptr;
 }
-
-static int step_smem(const FcabSim *s) { return s->use_tma ? s->L.tma_smem : 0; }
 
 // Host launches per step: the step; with seeded dt pruning and no tail
 // launch, also the guarded full velocity pass (it returns at once unless the
@@ -819,7 +811,7 @@ static cudaError_t launch_one(FcabSim *s)
         GridD<double> g;
         grid_view(s, g);
         e = s->L.step(&g, &s->rkd, s->tc, s->ctl, s->split, s->grid, s->stream,
-                      step_smem(s));
+                      s->L.smem);
         if (e == cudaSuccess && s->tc.vseed_on && !s->tc.tail_vpass)
             e = s->L.init(&g, &s->rkd, s->tc, s->ctl, full_grid, s->stream, 1);
         return e;
@@ -827,7 +819,7 @@ static cudaError_t launch_one(FcabSim *s)
     GridD<float> g;
     grid_view(s, g);
     e = s->L.step(&g, &s->rkf, s->tc, s->ctl, s->split, s->grid, s->stream,
-                  step_smem(s));
+                  s->L.smem);
     if (e == cudaSuccess && s->tc.vseed_on && !s->tc.tail_vpass)
         e = s->L.init(&g, &s->rkf, s->tc, s->ctl, full_grid, s->stream, 1);
     return e;
@@ -1104,7 +1096,7 @@ extern "C" int fcab_sim_info(FcabSim *s, FcabInfo *info)
     info->land_cells = s->land_cells;
     info->faces_per_step = s->faces_per_step;
     info->pitch = s->pitch;
-    info->tma_rows = s->use_tma && s->L.tma_smem > 0 ? 1 : 0;
+    info->tma_rows = s->L.blk;
     return 0;
 }
 
@@ -1297,12 +1289,12 @@ extern "C" int fcab_sim_slab_step(FcabSim *s)
         GridD<double> g;
         grid_view(s, g);
         CUDA_TRY(s->L.step(&g, &s->rkd, s->tc, s->ctl, s->split, s->grid, s->stream,
-                           step_smem(s)));
+                           s->L.smem));
     } else {
         GridD<float> g;
         grid_view(s, g);
         CUDA_TRY(s->L.step(&g, &s->rkf, s->tc, s->ctl, s->split, s->grid, s->stream,
-                           step_smem(s)));
+                           s->L.smem));
     }
     s->launches += 1;
     return 0;

@@ -57,6 +57,9 @@ int pick_cpl(const FcabConfig &c);
 // per_sm CTAs of wpb warps) with segments of cfg.seg_rows rows when set,
 // else an even split, at least 4 rows per warp (wca_sim.cu).
 long long step_warps(const FcabConfig &c, int cpl, int nsm, int per_sm, int wpb);
+// Whether a session's fields suit the block sweep: FP32 with row maps, all LAND
+// or with its mask coded in z and n, tau_h > 0, 32-bit element offsets.
+bool runs_block_sweep(const FcabSim *s);
 // Rows of a work unit of the block sweep (cfg.seg_rows when set).
 int blk_seg(const FcabConfig &c, int nsm, int per_sm);
 // Run constants of an FP32 configuration (defined in wca_sim.cu).
