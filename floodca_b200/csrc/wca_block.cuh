@@ -22,11 +22,14 @@
 // barrier between the phases each phase's registers die with it (64
 // registers, 32 warps per SM), the row ring is a fixed address distance
 // instead of register moves, and rows are shared by the CTA, so a range costs
-// six rows of halo per CTA instead of per warp. 446 warp instructions per row
-// at 64 % of the issue slots. Measured on a B200, microseconds a step, warm
-// grids, one warp per row range (before) and this: 4096^2 350 and 220, 2048^2
-// 112 and 70, 1024^2 51.5 and 27.8, 256^2 20.1 and 18.2, 1003 x 1498 with
-// K = 8 104 and 64. Bound by issue slots and the barriers; HBM is at 24 %.
+// six rows of halo per CTA instead of per warp. About 420 warp instructions
+// per row at 63 % of the issue slots. Measured on a B200, microseconds a
+// step, warm grids, one warp per row range (before) and this: 4096^2 350 and
+// 215, 2048^2 112 and 65, 1024^2 51.5 and 22.9, 256^2 20.1 and 10.5, 1003 x
+// 1498 with K = 8 104 and 49, 733 x 1101 with SEA and WALL cells 54 and 26.
+// Bound by issue slots and the barriers (HBM is at 24 %). Tried and slower: 3
+// CTAs of 80 registers without spills 2 %, CTAs of four warps 4 % (20 to 35 % on
+// small grids), the next pass's A before the barrier after D 10 %.
 //
 // Grids with SEA or WALL cells (GEN) carry the mask in the device copies of z
 // and n (k_encode_mask): n is NaN on every cell that is not LAND, z is PAD_Z
@@ -37,6 +40,7 @@
 #pragma once
 
 #include <cstddef>
+#include <type_traits>
 
 #include "wca_f2.cuh"
 #include "wca_tma.cuh"
@@ -48,10 +52,12 @@ constexpr int BLK_THREADS = 32 * BLK_ROWS;
 constexpr int BLK_STAGES = 3;               // tile stages: the pass at work and those ahead
 constexpr uint32_t BLK_ROW_B = 256;         // bytes of a strip row
 // Cells up to which the step's last CTA does a missed seed's velocity pass
-// alone: it reads the depths (4 B a cell) and evaluates the few cells deep
-// enough to matter. One step in a hundred needs it; a launch that could
-// launch the pass costs 1.3 us on every step.
-constexpr long long BLK_SOLO = 1ll << 18;
+// alone: it reads the depths (4 B a cell, about 100 us for 2^20 cells) and
+// evaluates the few cells deep enough to matter. One step in a hundred needs
+// it; a kernel that could launch the pass costs 1.3 us more to launch every
+// step, cannot overlap its start with the step before, and its graph takes 4
+// ms more to build and free.
+constexpr long long BLK_SOLO = 1ll << 20;
 
 // Shared memory, in bytes from a 128-byte boundary. Tile stage: rows
 // first-2 .. first+7 of z, h, n and rows first-2 .. first+5 of hmax, so that a
@@ -85,6 +91,17 @@ struct BlkK {
     float tau_l, tau_h;
 };
 
+// The CTA's current unit, written by its first thread. Here rather than in
+// registers: thirty values that every pass carried cost 48 to 104 B of spills.
+struct BlkUnit {
+    int H, passes;              // rows; passes
+    int lo, hi;                 // rows r0 + rel with rel < lo or rel >= hi are special
+    int r0, c_first, edges;     // open edges: bit 0 north, 1 south, 2 west, 3 east
+    int tx, ty, h_cur;          // column of the tiles; row of the next tiles to load
+    unsigned pass;              // passes of the CTA so far: stages and barrier parities
+    float hcut;                 // depth below which no cell raises the velocity maximum
+};
+
 // After the rings: what every thread of the CTA reads (so that no phase holds
 // it in registers) and the CTA's rare sums.
 template <typename AccT>
@@ -92,6 +109,7 @@ struct BlkTail {
     unsigned long long bar[BLK_STAGES];
     BlkK c;
     StepVals<float> sv;
+    BlkUnit un;
     TimePre pre;
     AccT a_clamp, a_bnd, a_rain, a_sea; // clamped volume, open-edge outflow, rain, outflow to SEA
     long long rain_cells;       // LAND output cells (uniform rain)
@@ -101,6 +119,7 @@ struct BlkTail {
     unsigned vmax;              // bits of the CTA's largest next-step velocity
     int bad;
     int unit[2];                // next unit of the CTA, by unit parity
+    int nblk, units;            // units per strip and in all
 };
 template <int K>
 __host__ __device__ constexpr int blk_smem_bytes()
@@ -133,6 +152,12 @@ __device__ __forceinline__ float slf(uint32_t a)
 {
     float v;
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ int sli(uint32_t a)
+{
+    int v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
     return v;
 }
 __device__ __forceinline__ void sst(uint32_t a, f2 v)
@@ -421,32 +446,37 @@ struct BlockSweep {
     static constexpr uint32_t TAIL = blk_tail<K>();
     static constexpr uint32_t KC = TAIL + (uint32_t)offsetof(Tail, c);
     static constexpr uint32_t SV = TAIL + (uint32_t)offsetof(Tail, sv);
+    static constexpr uint32_t UN = TAIL + (uint32_t)offsetof(Tail, un);
 #define FCAB_KC(m) sld(sb + KC + (uint32_t)offsetof(BlkK, m))
 #define FCAB_SV(m) slf(sb + SV + (uint32_t)offsetof(StepVals<float>, m))
+#define FCAB_UN(m) sli(sb + UN + (uint32_t)offsetof(BlkUnit, m))
 
-    // Per-CTA state that persists over units: the count of tile passes so far
-    // decides stages, barrier parities and ring buffers.
+    // The CTA's memory: shared address (128-byte aligned), and its tail, whose
+    // generic address is made where it is used (rare paths).
     struct Cta {
-        uint32_t sb;                // shared address of the CTA's memory (128-byte aligned)
-        Tail *tail;
-        unsigned pass;
+        uint32_t sb;
+        __device__ __forceinline__ Tail *tail() const
+        {
+            uint64_t p;
+            asm volatile("{\n\t.reg .u64 t;\n\tcvt.u64.u32 t, %1;\n\t"
+                         "cvta.shared.u64 %0, t;\n\t}"
+                         : "=l"(p)
+                         : "r"(sb + TAIL));
+            return reinterpret_cast<Tail *>(p);
+        }
     };
 
     // What a unit reads of a row above its first one, from rings that no
     // phase has written yet, only reaches rows that are dropped: the rings
     // need no clearing.
-    static __device__ __forceinline__ void attach(Cta &T, char *sm)
-    {
-        T.sb = smem_addr(sm);
-        T.tail = reinterpret_cast<Tail *>(sm + TAIL);
-        T.pass = 0;
-    }
+    static __device__ __forceinline__ void attach(Cta &T, char *sm) { T.sb = smem_addr(sm); }
     // one thread, once per CTA
     static __device__ __forceinline__ void init_barriers(Cta &T)
     {
         for (int q = 0; q < BLK_STAGES; q++)
-            mbar_init1(T.sb + TAIL + 8u * q);
-        T.tail->bad = 0;
+            mbar_init2(T.sb + TAIL + 8u * q);
+        T.tail()->bad = 0;
+        T.tail()->un.pass = 0u;
         fence_proxy_async_smem();
     }
 
@@ -454,7 +484,7 @@ struct BlockSweep {
     static __device__ __forceinline__ void begin(Cta &T, const GridD<float> &g,
                                                  const RunK<float> &rk, const Ctl *ctl)
     {
-        Tail &t = *T.tail;
+        Tail &t = *T.tail();
         const StepVals<float> sv = step_vals<float, K>(g, rk, ctl);
         const StepK<float> &k = sv.k;
         t.sv = sv;
@@ -482,35 +512,94 @@ struct BlockSweep {
     }
 
     // one thread: the tiles of a pass (from row y0, two above the pass's
-    // first) into its stage
+    // first) into its stage. The barrier of a stage takes two arrivals, one
+    // with the fields that never change (z, n) and one with those that the
+    // step before wrote (h, hmax).
+    static __device__ __forceinline__ void issue_fixed(uint32_t sb, const CUtensorMap *tm, int tx,
+                                                       int y0, unsigned pass)
+    {
+        const unsigned st = pass % BLK_STAGES;
+        const uint32_t bar = sb + TAIL + 8u * st, dst = sb + st * BLK_STAGE_B;
+        mbar_arrive_tx(bar, 2 * BLK_TILE_B);
+        tma_load_tile(dst + BLK_Z, tm, bar, tx, y0);
+        tma_load_tile(dst + BLK_N, tm + 1, bar, tx, y0);
+    }
+    static __device__ __forceinline__ void issue_state(uint32_t sb, const CUtensorMap *tm,
+                                                       const CUtensorMap *th, int tx, int y0,
+                                                       unsigned pass)
+    {
+        const unsigned st = pass % BLK_STAGES;
+        const uint32_t bar = sb + TAIL + 8u * st, dst = sb + st * BLK_STAGE_B;
+        mbar_arrive_tx(bar, BLK_STAGE_B - 2 * BLK_TILE_B);
+        tma_load_tile(dst + BLK_H, th, bar, tx, y0);
+        tma_load_tile(dst + BLK_M, tm + 4, bar, tx, y0);
+    }
     static __device__ __forceinline__ void issue(uint32_t sb, const CUtensorMap *tm,
                                                  const CUtensorMap *th, int tx, int y0,
                                                  unsigned pass)
     {
-        const unsigned st = pass % BLK_STAGES;
-        const uint32_t bar = sb + TAIL + 8u * st, dst = sb + st * BLK_STAGE_B;
         fence_proxy_async_smem();
-        mbar_arrive_tx(bar, BLK_STAGE_B);
-        tma_load_tile(dst + BLK_Z, tm, bar, tx, y0);
-        tma_load_tile(dst + BLK_H, th, bar, tx, y0);
-        tma_load_tile(dst + BLK_N, tm + 1, bar, tx, y0);
-        tma_load_tile(dst + BLK_M, tm + 4, bar, tx, y0);
+        issue_fixed(sb, tm, tx, y0, pass);
+        issue_state(sb, tm, th, tx, y0, pass);
     }
-    // one thread: the tiles of a unit's first passes
-    static __device__ __forceinline__ void first_tiles(const Cta &T, const GridD<float> &g,
-                                                       int h_cur, int strip, int r0, int r1)
+    // one thread: a unit's descriptor
+    static __device__ __forceinline__ void open_unit(const Cta &T, const GridD<float> &g,
+                                                     const RunK<float> &rk, int strip, int r0,
+                                                     int r1)
     {
         using Gm = Geom<2>;
-        const int np = (r1 - r0 + 6 + BLK_ROWS - 1) / BLK_ROWS;
-        for (int b = 0; b < min(np, BLK_STAGES - 1); b++)
-            issue(T.sb, g.tmap, g.tmap + (h_cur ? 3 : 2), strip * Gm::OW - Gm::HL + PADC,
-                  r0 - 5 + PADR + b * BLK_ROWS, T.pass + b);
+        BlkUnit &u = T.tail()->un;
+        const int c = strip * Gm::OW - Gm::HL;
+        u.H = r1 - r0;
+        u.passes = (r1 - r0 + 6 + BLK_ROWS - 1) / BLK_ROWS;
+        // special rows: r < 1 or r >= nr - 2; in strips with a column outside
+        // the grid, column 0 or nc-1, or the inflow cell, all of them
+        const bool all = c <= 0 || c + Gm::SW > g.nc - 1 ||
+                         (rk.inflow_c >= c && rk.inflow_c < c + Gm::SW);
+        u.lo = all ? 0x7fffffff : 1 - r0;
+        u.hi = g.nr - 2 - r0;
+        u.r0 = r0;
+        u.c_first = c;
+        u.edges = !rk.open ? 0
+                           : (rk.edge_n ? 1 : 0) | (rk.edge_s ? 2 : 0) |
+                                 (rk.edge_w && c <= 0 ? 4 : 0) |
+                                 (rk.edge_e && c + Gm::SW > g.nc - 1 ? 8 : 0);
+        u.tx = c + PADC;            // a multiple of 4 floats
+        u.ty = r0 - 5 + PADR;
+    }
+    // one thread, after open_unit: the tiles of its first passes, the fixed
+    // fields, then (h_cur known) the state
+    static __device__ __forceinline__ void first_fixed(const Cta &T, const GridD<float> &g)
+    {
+        const BlkUnit &u = T.tail()->un;
+        fence_proxy_async_smem();
+        for (int b = 0; b < min(u.passes, BLK_STAGES - 1); b++)
+            issue_fixed(T.sb, g.tmap, u.tx, u.ty + b * BLK_ROWS, u.pass + b);
+    }
+    static __device__ __forceinline__ void first_state(const Cta &T, const GridD<float> &g,
+                                                       int h_cur)
+    {
+        BlkUnit &u = T.tail()->un;
+        for (int b = 0; b < min(u.passes, BLK_STAGES - 1); b++)
+            issue_state(T.sb, g.tmap, g.tmap + (h_cur ? 3 : 2), u.tx, u.ty + b * BLK_ROWS,
+                        u.pass + b);
+        u.h_cur = h_cur;
+        u.ty += (BLK_STAGES - 1) * BLK_ROWS;
+    }
+    // one thread, instead of first_state: the fixed tiles land and are dropped
+    static __device__ __forceinline__ void first_drop(const Cta &T)
+    {
+        const BlkUnit &u = T.tail()->un;
+        for (int b = 0; b < min(u.passes, BLK_STAGES - 1); b++) {
+            mbar_arrive(T.sb + TAIL + 8u * ((u.pass + b) % BLK_STAGES));
+            arrived(T, u.pass + b);
+        }
     }
     // one thread: waits for the tiles of a pass
     static __device__ __forceinline__ void arrived(const Cta &T, unsigned pass)
     {
         if (!mbar_wait_bounded(T.sb + TAIL + 8u * (pass % BLK_STAGES), (pass / BLK_STAGES) & 1u))
-            T.tail->bad = 1;
+            T.tail()->bad = 1;
     }
     // a row of a phase value: into slot w + 2, and for the last two warps
     // into the other buffer's slot w - 6 (`over`: the distance to it)
@@ -526,18 +615,18 @@ struct BlockSweep {
     {
         return (r == 0 && (edges & 1)) || (r == nr - 1 && (edges & 2));
     }
-    // The open west (lanes 0..7) and east (lanes 8..15) edge cells of the
+    // The open west (first BLK_ROWS lanes) and east (next) edge cells of the
     // pass's rows, a row per lane: their discharges into Tail::qo by row (modulo 32).
     // One evaluation a pass instead of two per row of an edge strip: with both
     // open, a 2048^2 step took 109 us that way and takes 67 this way (66 closed).
     static __device__ __forceinline__ void open_ends(Tail &tl, uint32_t sb, uint32_t tiles,
-                                                     int first, int r0, int r1, int c_first,
-                                                     int nr, int nc, int edges, int lane)
+                                                     int first, int nr, int nc, int lane)
     {
-        const int side = lane >> 3 & 1, slot = lane & 7, row = first + slot;
-        const int c = (side ? nc - 1 : 0) - c_first;
+        const int edges = tl.un.edges, r0 = tl.un.r0, r1 = r0 + tl.un.H;
+        const int side = lane / BLK_ROWS & 1, slot = lane % BLK_ROWS, row = r0 + first + slot;
+        const int c = (side ? nc - 1 : 0) - tl.un.c_first;
         float z = 0.0f, h = 0.0f, n = 1.0f;
-        const bool on = lane < 16 && (edges & (4 << side));
+        const bool on = lane < 2 * BLK_ROWS && (edges & (4 << side));
         if (on) {
             const uint32_t a = tiles + (slot + 2) * BLK_ROW_B + 4u * (uint32_t)c;
             z = slf(a + BLK_Z);
@@ -587,7 +676,7 @@ struct BlockSweep {
                                                    int slot)
     {
         using Gm = Geom<2>;
-        Tail &t = *T.tail;
+        Tail &t = *T.tail();
         // halo lanes evaluate faces that other strips own
         const bool out = lane * 2 >= Gm::HL && lane * 2 < Gm::HL + Gm::OW;
         const unsigned cap = __reduce_add_sync(0xffffffffu, out ? ss.capn : 0u);
@@ -633,65 +722,47 @@ struct BlockSweep {
         }
     }
 
-    // Rows [r0, r1) of one strip, by the whole CTA; its first tiles are on
-    // their way (first_tiles). wp: the warp's index, as a warp-uniform value.
-    static __device__ __forceinline__ void run(Cta &T, const GridD<float> &g,
-                                               const RunK<float> &rk, int h_cur, int strip,
-                                               int r0, int r1, int wp, int lane, SS &ss)
+    // The unit at T.tail()->un, by the whole CTA; its first tiles are on their
+    // way. wp: the warp's index, as a warp-uniform value.
+    static __device__ __forceinline__ void run(const Cta &T, const GridD<float> &g,
+                                               const RunK<float> &rk, int wp, int lane, SS &ss)
     {
         using Gm = Geom<2>;
-        Tail &tl = *T.tail;
         const uint32_t sb = T.sb;
         const f2 z0 = bc2(0.0f);
-        const int nr = g.nr, nc = g.nc, pitch = (int)g.pitch;
-        const int c_first = strip * Gm::OW - Gm::HL;
-        const int cbase = c_first + lane * 2;
         const bool out_lane = lane * 2 >= Gm::HL && lane * 2 < Gm::HL + Gm::OW;
-        // open edges (bit 0 north, 1 south, 2 west, 3 east) this strip has
-        const int edges = !rk.open ? 0
-                                   : (rk.edge_n ? 1 : 0) | (rk.edge_s ? 2 : 0) |
-                                         (rk.edge_w && c_first <= 0 ? 4 : 0) |
-                                         (rk.edge_e && c_first + Gm::SW > nc - 1 ? 8 : 0);
-        // strips with a column outside the grid, column 0 or nc-1, or the
-        // inflow cell: their rows take the special branches
-        const bool spec_strip = c_first <= 0 || c_first + Gm::SW > nc - 1 ||
-                                (rk.inflow_c >= c_first && rk.inflow_c < c_first + Gm::SW);
-        const int H = r1 - r0;
-        const int np = (H + 6 + BLK_ROWS - 1) / BLK_ROWS;           // passes
-        const CUtensorMap *tm = g.tmap;
-        const CUtensorMap *th = tm + (h_cur ? 3 : 2);
-        const int tx = c_first + PADC;                              // a multiple of 4 floats
-        const int ty = r0 - 5 + PADR;
-        const unsigned pass0 = T.pass;
-        if (wp == 0 && lane == 0)
-            arrived(T, pass0);
-        float hcut = height_cut(tl, threshold(tl));
+        const int pitch = (int)g.pitch;
+        if (wp == 0 && lane == 0) {
+            Tail &tl = *T.tail();
+            tl.un.hcut = height_cut(tl, threshold(tl));
+            arrived(T, tl.un.pass);
+        }
         __syncthreads();
 
         const bool last2 = wp >= BLK_ROWS - 2;
         const uint32_t sl = sb + lane * 8 + wp * BLK_ROW_B;
         uint32_t rb = sl + BLK_RINGS;                               // this pass's rings
-        uint32_t turn = blk_buf<K>();                               // to the other buffer
-        if (pass0 & 1u) {
-            rb += turn;
-            turn = 0u - turn;
-        }
-        uint32_t tb = sl + pass0 % BLK_STAGES * BLK_STAGE_B;        // this pass's tiles
-        const uint32_t tb_end = sl + BLK_STAGES * BLK_STAGE_B;
+        uint32_t tb = sl + (unsigned)FCAB_UN(pass) % BLK_STAGES * BLK_STAGE_B; // and tiles
         int rel = wp - 5;                   // row i-2 relative to r0
-        int off2 = (r0 + rel + PADR) * pitch + cbase + PADC;        // its element
+        int off2 = (FCAB_UN(r0) + rel + PADR) * pitch + FCAB_UN(c_first) + lane * 2 + PADC;
         bool prev_cand = false;
 
-        for (int b = 0; b < np; b++) {
-            if (wp == 0 && lane == 0 && b + BLK_STAGES - 1 < np)
-                // the stage's rows were last read in pass b-1, before its last barrier
-                issue(sb, tm, th, tx, ty + (b + BLK_STAGES - 1) * BLK_ROWS,
-                      pass0 + b + BLK_STAGES - 1);
-            const uint32_t over = turn - (BLK_ROWS - 2) * BLK_ROW_B;
-            const int r = r0 + rel;                                 // row i-2
-            const bool own2 = (unsigned)rel < (unsigned)H;          // written
-            // rows i-1, i-2 on or outside the grid's first and last rows
-            const bool spec = spec_strip || r < 1 || r + 2 >= nr;
+        for (int left = FCAB_UN(passes); left > 0; left--) {
+            if (wp == 0 && lane == 0 && left > BLK_STAGES - 1) {
+                // the stage's rows were last read in the pass before, before its last barrier
+                BlkUnit &u = T.tail()->un;
+                issue(sb, g.tmap, g.tmap + (u.h_cur ? 3 : 2), u.tx, u.ty,
+                      u.pass + BLK_STAGES - 1);
+                u.ty += BLK_ROWS;
+            }
+            // to the other buffer, less the slots of the last two warps
+            const uint32_t over = (rb == sl + BLK_RINGS ? blk_buf<K>() : 0u - blk_buf<K>()) -
+                                  (BLK_ROWS - 2) * BLK_ROW_B;
+            const int H = FCAB_UN(H);
+            const bool own2 = (unsigned)rel < (unsigned)H;          // row i-2 is written
+            // rows i-1, i-2 on or outside the grid's first and last rows, or a
+            // special strip: they run the copy of C and D with the branches
+            const bool spec = rel < FCAB_UN(lo) || rel >= FCAB_UN(hi);
 
             // ---- A: x faces of row i; y (and diagonal) faces of rows i-1, i
             f2 Y1, E1 = z0, W1 = z0;
@@ -771,9 +842,9 @@ struct BlockSweep {
                     keep(rb + BLK_E, E1, last2, over);
                     keep(rb + BLK_W, W1, last2, over);
                 }
-                if ((edges & 12) && wp == BLK_ROWS - 1)
-                    open_ends(tl, sb, tb - lane * 8 - wp * BLK_ROW_B, r + 2 - wp, r0, r1, c_first,
-                              nr, nc, edges, lane);
+                if (wp == BLK_ROWS - 1 && (FCAB_UN(edges) & 12))
+                    open_ends(*T.tail(), sb, tb - lane * 8 - wp * BLK_ROW_B, rel + 2 - wp, g.nr,
+                              g.nc, lane);
                 if ((unsigned)(rel + 2) < (unsigned)H)
                     ss.capn += cx;
                 if ((unsigned)(rel + 1) < (unsigned)H)
@@ -785,7 +856,12 @@ struct BlockSweep {
             //      489-502), in the reference order +x, -x, +y, -y, d1+, d1-,
             //      d2+, d2-, open slots
             f2 Y2, S1 = bc2(1.0f), E2 = z0, W2 = z0;
-            {
+            auto phase_c = [&](auto special_tag) {
+                constexpr bool special = decltype(special_tag)::value;
+                const int r = special ? FCAB_UN(r0) + rel : 0;
+                const int edges = special ? FCAB_UN(edges) : 0;
+                const int cbase = special ? FCAB_UN(c_first) + lane * 2 : 0;
+                const int nr = g.nr, nc = g.nc;
                 const f2 X1 = sld(rb + BLK_X + BLK_ROW_B);
                 Y2 = sld(rb + BLK_Y + BLK_ROW_B);
                 f2 out = sub2(max2(X1, z0), min2(left2(X1), z0));
@@ -800,7 +876,7 @@ struct BlockSweep {
                     out = sub2(out, min2(W2, z0));
                 }
                 const f2 hp = sld(tb + BLK_H + BLK_ROW_B);
-                if (spec && open_row(edges, r + 1, nr)) {
+                if (special && open_row(edges, r + 1, nr)) {
                     const OpenPair o = open_pair(sld(tb + BLK_Z + BLK_ROW_B), hp,
                                                  sld(tb + BLK_N + BLK_ROW_B), sb + KC, sb + SV);
                     int k0, k1;
@@ -814,8 +890,8 @@ struct BlockSweep {
                         ss.capn += (o.cap & 1u ? k0 : 0) + (o.cap & 2u ? k1 : 0);
                     out = add2(out, mk2(open_sum<float>(lo2(o.q), k0),
                                         open_sum<float>(hi2(o.q), k1)));
-                } else if (edges & 12) {
-                    out = add2(out, end_flow(tl, r + 1, cbase, nr, nc, g.r_lo, g.r_hi, edges,
+                } else if (special && (edges & 12)) {
+                    out = add2(out, end_flow(*T.tail(), r + 1, cbase, nr, nc, g.r_lo, g.r_hi, edges,
                                              bc2(1.0f)));
                 }
                 const f2 ov = mul2(out, FCAB_KC(dt));
@@ -832,18 +908,36 @@ struct BlockSweep {
                     S1 = sel2(l0, l1, q, S1);
                 }
                 keep(rb + BLK_S, S1, last2, over);
-            }
+            };
+            if (spec)
+                phase_c(std::true_type{});
+            else
+                phase_c(std::false_type{});
             __syncthreads();
 
             // ---- D: net inflow of row i-2 from the upwind-scaled
             //      discharges, depth update, clamp, inflow, hmax and tmax
             //      (model.c:511-597)
             bool cand = false;
-            {
+            auto phase_d = [&](auto special_tag) {
+                constexpr bool special = decltype(special_tag)::value;
+                const int r = special ? FCAB_UN(r0) + rel : 0;
+                const int edges = special ? FCAB_UN(edges) : 0;
+                const int nr = g.nr, nc = g.nc;
+                auto column = [&]() { return FCAB_UN(c_first) + lane * 2; };
                 const f2 S2 = sld(rb + BLK_S + BLK_ROW_B), S3 = sld(rb + BLK_S);
-                const f2 sr = right2(S2);
-                const f2 Qr = upwind2(sld(rb + BLK_X), S2, sr), Ql = left2(Qr);
-                const f2 Qd = upwind2(Y2, S2, S1), Qu = upwind2(sld(rb + BLK_Y), S3, S2);
+                // the limiter binds in few rows (it is 1 in the others, and the
+                // discharges their own products with it): measured 1 to 3 % of a step
+                f2 sr = S2, Qr = sld(rb + BLK_X), Ql, Qd = Y2, Qu = sld(rb + BLK_Y);
+                const bool lim = fminf(fminf(lo2(S1), lo2(S2)), lo2(S3)) < 1.0f ||
+                                 fminf(fminf(hi2(S1), hi2(S2)), hi2(S3)) < 1.0f;
+                if (K == 8 || __any_sync(0xffffffffu, lim)) {
+                    sr = right2(S2);
+                    Qr = upwind2(Qr, S2, sr);
+                    Qd = upwind2(Y2, S2, S1);
+                    Qu = upwind2(Qu, S3, S2);
+                }
+                Ql = left2(Qr);
                 f2 net = sub2(Ql, Qr);
                 net = sub2(net, Qd);
                 net = add2(net, Qu);
@@ -868,6 +962,7 @@ struct BlockSweep {
                         // what SEA cells receive has left the domain (model.c:241-319,
                         // there counted by the LAND cell of the face)
                         const f2 z = sld(tb + BLK_Z);
+                        const int cbase = column();
                         const bool own = own2 && out_lane;
                         const bool sea0 = own && lo2(z) < -1e29f && cbase >= 0 && cbase < nc;
                         const bool sea1 = own && hi2(z) < -1e29f && cbase + 1 >= 0 &&
@@ -891,17 +986,18 @@ struct BlockSweep {
                         if (__any_sync(0xffffffffu, sea != 0)) {
                             sea = warp_sum(sea);
                             if (lane == 0)
-                                atomicAdd(&tl.a_sea, sea);
+                                atomicAdd(&T.tail()->a_sea, sea);
                         }
                     }
                 }
                 const f2 h = sld(tb + BLK_H);
-                if (spec && open_row(edges, r, nr)) {
+                if (special && open_row(edges, r, nr)) {
                     // open-edge outflow scaled by the cell's own limiter
                     // (model.c:553-559), summed over its open slots
                     const OpenPair o = open_pair(sld(tb + BLK_Z), h, sld(tb + BLK_N), sb + KC,
                                                  sb + SV);
                     int k0, k1;
+                    const int cbase = column();
                     open_sides(r, cbase, nr, nc, g.r_lo, g.r_hi, edges, k0, k1);
                     if constexpr (GEN) {        // LAND cells only
                         const f2 n = sld(tb + BLK_N);
@@ -918,14 +1014,15 @@ struct BlockSweep {
                         bnd = acc_mul<AccT, float>(dt, q0) + acc_mul<AccT, float>(dt, q1);
                     bnd = warp_sum(bnd);
                     if (lane == 0 && bnd != 0)
-                        atomicAdd(&tl.a_bnd, bnd);
-                } else if (edges & 12) {
-                    const f2 qs = end_flow(tl, r, cbase, nr, nc, g.r_lo, g.r_hi, edges, S2);
+                        atomicAdd(&T.tail()->a_bnd, bnd);
+                } else if (special && (edges & 12)) {
+                    const int cbase = column();
+                    const f2 qs = end_flow(*T.tail(), r, cbase, nr, nc, g.r_lo, g.r_hi, edges, S2);
                     net = sub2(net, qs);
                     // at most one lane each holds column 0 and column nc-1
                     if (own2 && out_lane && (lo2(qs) != 0.0f || hi2(qs) != 0.0f)) {
                         const float dt = FCAB_SV(dt);
-                        tl.bnd[wp][cbase == 0 ? 0 : 1] +=
+                        T.tail()->bnd[wp][cbase == 0 ? 0 : 1] +=
                             (double)(acc_mul<AccT, float>(dt, lo2(qs)) +
                                      acc_mul<AccT, float>(dt, hi2(qs)));
                     }
@@ -949,23 +1046,25 @@ struct BlockSweep {
                 if (__any_sync(0xffffffffu, lo2(hu) < 0.0f || hi2(hu) < 0.0f)) {
                     float a0 = lo2(hu), a1 = hi2(hu);
                     const bool own = own2 && out_lane;
+                    const int cbase = column();
                     const float A = FCAB_SV(A);
                     if (a0 < 0.0f) {
                         if (own && l0 && cbase >= 0 && cbase < nc)
-                            atomicAdd(&tl.a_clamp, acc_mul<AccT, float>(-a0, A));
+                            atomicAdd(&T.tail()->a_clamp, acc_mul<AccT, float>(-a0, A));
                         a0 = 0.0f;
                     }
                     if (a1 < 0.0f) {
                         if (own && l1 && cbase + 1 >= 0 && cbase + 1 < nc)
-                            atomicAdd(&tl.a_clamp, acc_mul<AccT, float>(-a1, A));
+                            atomicAdd(&T.tail()->a_clamp, acc_mul<AccT, float>(-a1, A));
                         a1 = 0.0f;
                     }
                     hu = mk2(a0, a1);
                 }
                 const f2 z = sld(tb + BLK_Z);
                 f2 Ln = add2(z, hu);
-                if (spec) {
+                if (special) {
                     const bool rin = r >= g.r_lo && r < g.r_hi;
+                    const int cbase = column();
                     const bool in0 = rin && cbase >= 0 && cbase < nc;
                     const bool in1 = rin && cbase + 1 >= 0 && cbase + 1 < nc;
                     if (r == rk.inflow_r) {
@@ -998,6 +1097,7 @@ struct BlockSweep {
                         ss.rain_sum += (double)lo2(rain) + (double)hi2(rain);
                     }
                     // a cell that could raise the velocity maximum
+                    const float hcut = __int_as_float(FCAB_UN(hcut));
                     cand = (l0 && lo2(hu) >= hcut) || (l1 && hi2(hu) >= hcut);
                     const f2 hm = sld(tb + BLK_M);                  // hmax of row i-2
                     const uint64_t ho = sld(sb + SV + (uint32_t)offsetof(StepVals<float>, hout)).u;
@@ -1013,9 +1113,17 @@ struct BlockSweep {
                     if (l1 && hi2(hu) > hi2(hm))
                         tmx[1] = tv;
                 }
+            };
+            if (spec)
+                phase_d(std::true_type{});
+            else
+                phase_d(std::false_type{});
+            if (wp == 0 && lane == 0) {
+                BlkUnit &u = T.tail()->un;
+                u.pass += 1;
+                if (left > 1)
+                    arrived(T, u.pass);
             }
-            if (wp == 0 && lane == 0 && b + 1 < np)
-                arrived(T, pass0 + b + 1);
             const bool any_cand = __syncthreads_or(cand) != 0;
 
             // ---- E: next step's stable velocity of row i-3 from the new
@@ -1023,32 +1131,32 @@ struct BlockSweep {
             //      of this pass sits in rows i-3 of this pass or, for the
             //      last warp's row, of the next one.
             if (any_cand || prev_cand) {
-                const float thr = threshold(tl);
-                hcut = height_cut(tl, thr);
+                Tail &tl = *T.tail();
+                const float thr = threshold(tl), hcut = height_cut(tl, thr);
+                const int r = tl.un.r0 + rel, cbase = tl.un.c_first + lane * 2;
                 if (tl.sv.want_v && (unsigned)(rel - 1) < (unsigned)H)
                     velocity_row(tl, g, sld(rb + BLK_L + BLK_ROW_B),
                                  sld(rb + BLK_L + 2 * BLK_ROW_B), sld(rb + BLK_L), r - 1, cbase,
-                                 edges,
-                                 out_lane && cbase >= 0 && cbase < nc,
-                                 out_lane && cbase + 1 >= 0 && cbase + 1 < nc, off2 - pitch, thr,
-                                 hcut);
+                                 tl.un.edges, out_lane && cbase >= 0 && cbase < g.nc,
+                                 out_lane && cbase + 1 >= 0 && cbase + 1 < g.nc, off2 - pitch,
+                                 thr, hcut);
+                if (wp == 0 && lane == 0)
+                    tl.un.hcut = hcut;      // read in D, after two barriers
             }
             prev_cand = any_cand;
 
-            rb += turn;
-            turn = 0u - turn;
-            tb += BLK_STAGE_B;
-            if (tb == tb_end)
-                tb = sl;
+            rb = 2 * (sl + BLK_RINGS) + blk_buf<K>() - rb;
+            tb = tb == sl + (BLK_STAGES - 1) * BLK_STAGE_B ? sl : tb + BLK_STAGE_B;
             rel += BLK_ROWS;
             off2 += BLK_ROWS * pitch;
         }
-        T.pass += np;
         // uniform rain on LAND output cells
         if constexpr (sizeof(AccT) == 8 && !RAINF) {
-            if (wp == 0 && lane == 0)
-                tl.rain_cells += (long long)H * (min(nc, c_first + Gm::HL + Gm::OW) -
-                                                 (c_first + Gm::HL));
+            if (wp == 0 && lane == 0) {
+                Tail &tl = *T.tail();
+                const int c0 = tl.un.c_first + Gm::HL;
+                tl.rain_cells += (long long)tl.un.H * (min(g.nc, c0 + Gm::OW) - c0);
+            }
         }
     }
 
@@ -1112,6 +1220,7 @@ struct BlockSweep {
     }
 #undef FCAB_KC
 #undef FCAB_SV
+#undef FCAB_UN
 };
 
 }  // namespace fcab

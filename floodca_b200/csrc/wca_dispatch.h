@@ -126,10 +126,21 @@ template <typename AccT, int K, int MATH, bool RAINF, bool GEN, bool TAILV>
 cudaError_t launch_step_blk(const void *g, const void *rk, const TimeCfg &tc, Ctl *ctl, int seg,
                             int grid, cudaStream_t s, int smem)
 {
-    k_step_blk<AccT, K, MATH, RAINF, GEN, TAILV><<<grid, BLK_THREADS, smem, s>>>(
-        *static_cast<const GridD<float> *>(g), *static_cast<const RunK<float> *>(rk), tc, ctl,
-        seg);
-    return cudaGetLastError();
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3(BLK_THREADS);
+    c.dynamicSmemBytes = (size_t)smem;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    // only where both launches fit on the GPU (two CTAs of each per SM):
+    // measured 3 to 9 % faster up to 512^2, 3 % slower at 733 x 1101
+    c.numAttrs = !TAILV && grid <= 2 * 148 ? 1 : 0;
+    return cudaLaunchKernelEx(&c, &k_step_blk<AccT, K, MATH, RAINF, GEN, TAILV>,
+                              *static_cast<const GridD<float> *>(g),
+                              *static_cast<const RunK<float> *>(rk), tc, ctl, seg);
 }
 
 template <typename AccT, int K, int MATH, bool RAINF, bool GEN, bool TAILV>

@@ -1332,7 +1332,9 @@ __device__ __forceinline__ T velocity_at(const GridD<T> &g, const RunK<T> &rk, c
 // before anything else is computed, the constants and the clock are worked
 // out by two other warps meanwhile, and on grids of up to BLK_SOLO cells
 // (TAILV = false) the last CTA does a missed seed's velocity pass itself
-// instead of launching it. Measured, us a step: 61 x 93 14.5 -> 9.0, 256^2
+// instead of launching it, and a step starts while the one before it ends:
+// its barriers are set up and its first tiles of z and n on their way before
+// it waits for that one. Measured, us a step: 61 x 93 14.5 -> 9.0, 256^2
 // 18.2 -> 11.1, 512^2 19.3 -> 14.3, 1024^2 27.8 -> 25.2.
 template <typename AccT, int K, int MATH, bool RAINF, bool GEN, bool TAILV>
 __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
@@ -1340,47 +1342,64 @@ __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
 {
     using Sweep = BlockSweep<AccT, K, MATH, RAINF, GEN>;
     using G = Geom<2>;
-    const int active = ctl->active, h_cur = ctl->h_cur;
-    if (active == 0)
-        return;
     extern __shared__ __align__(1024) unsigned char fcab_dsm[];
     char *const sm = reinterpret_cast<char *>(fcab_dsm) +
                      ((128u - (smem_addr(fcab_dsm) & 127u)) & 127u);
     int lane;       // volatile: held in a register, not read again from the special register
     asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
-    const int wp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
-    // units of `seg` rows of a strip, taken from the step's counter (the first
-    // one by the CTA's index)
-    const int nr = g.nr, nstrips = (g.nc + G::OW - 1) / G::OW;
-    const int nblk = (nr + seg - 1) / seg, units = nstrips * nblk;
+    int wp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    asm volatile("" : "+r"(wp));
     typename Sweep::Cta T;
     Sweep::attach(T, sm);
+    if (wp == 0 && lane == 0) {
+        // units of `seg` rows of a strip, taken from the step's counter (the
+        // first one by the CTA's index)
+        Sweep::init_barriers(T);
+        const int nblk = (g.nr + seg - 1) / seg, u = blockIdx.x;
+        T.tail()->nblk = nblk;
+        T.tail()->units = (g.nc + G::OW - 1) / G::OW * nblk;
+        const int r0 = u % nblk * seg;
+        Sweep::open_unit(T, g, rk, u / nblk, r0, min(g.nr, r0 + seg));
+        Sweep::first_fixed(T, g);
+    }
+    if constexpr (!TAILV) {
+        wait_previous();
+        let_next();
+    }
+    const int active = ctl->active;
+    if (active == 0) {
+        if (wp == 0 && lane == 0)
+            Sweep::first_drop(T);
+        return;
+    }
     if (lane == 0) {
         if (wp == 0) {
-            Sweep::init_barriers(T);
-            const int r0 = blockIdx.x % nblk * seg;
-            Sweep::first_tiles(T, g, h_cur, blockIdx.x / nblk, r0, min(nr, r0 + seg));
-            T.tail->unit[0] = units > (int)gridDim.x
-                                  ? (int)(gridDim.x + atomicAdd(&ctl->next_unit, 1u))
-                                  : units;
+            Sweep::first_state(T, g, ctl->h_cur);
+            const int units = T.tail()->units;
+            T.tail()->unit[0] = units > (int)gridDim.x
+                                    ? (int)(gridDim.x + atomicAdd(&ctl->next_unit, 1u))
+                                    : units;
         } else if (wp == 1) {
             Sweep::begin(T, g, rk, ctl);
         } else if (wp == 2) {
-            T.tail->pre = time_pre(ctl, tc, true);
+            T.tail()->pre = time_pre(ctl, tc, true);
         }
     }
     __syncthreads();
     StepSums<float, AccT> ss;
-    int par = 0;
-    for (int u = blockIdx.x; u < units; par ^= 1) {
-        const int r0 = u % nblk * seg, r1 = min(nr, r0 + seg);
-        if (u != (int)blockIdx.x && wp == 0 && lane == 0) {
-            Sweep::first_tiles(T, g, h_cur, u / nblk, r0, r1);
-            T.tail->unit[par] = (int)(gridDim.x + atomicAdd(&ctl->next_unit, 1u));
-        }
-        Sweep::run(T, g, rk, h_cur, u / nblk, r0, r1, wp, lane, ss);
+    for (int par = 0;; par ^= 1) {
+        Sweep::run(T, g, rk, wp, lane, ss);
         __syncthreads();
-        u = T.tail->unit[par];
+        const int u = T.tail()->unit[par];
+        if (u >= T.tail()->units)
+            break;
+        if (wp == 0 && lane == 0) {
+            const int nblk = T.tail()->nblk, r0 = u % nblk * seg;
+            Sweep::open_unit(T, g, rk, u / nblk, r0, min(g.nr, r0 + seg));
+            Sweep::first_fixed(T, g);
+            Sweep::first_state(T, g, T.tail()->un.h_cur);
+            T.tail()->unit[par ^ 1] = (int)(gridDim.x + atomicAdd(&ctl->next_unit, 1u));
+        }
     }
     Sweep::publish(T, ss, ctl, lane, (int)(blockIdx.x & (NSLOT - 1)));
     // ---- the last CTA to finish prepares the next step
@@ -1390,7 +1409,7 @@ __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
         const unsigned prev = atomicAdd(&ctl->ctas_done, 1u);
         if (prev == gridDim.x - 1) {
             __threadfence();
-            ctl->h_cur = h_cur ^ 1;
+            ctl->h_cur = T.tail()->un.h_cur ^ 1;
             ctl->launches += 1;
             ctl->next_unit = 0u;
             if (tc.split) {
@@ -1398,7 +1417,7 @@ __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
                 ctl->ctas_done = 0u;
             } else {
                 const unsigned vbits = (unsigned)ctl->vmax_bits;
-                finalize<float>(ctl, tc, rk, true, T.tail->pre);
+                finalize<float>(ctl, tc, rk, true, T.tail()->pre);
                 // a missed seed defers this step's dt to the full velocity
                 // pass: done here, or launched from here into the tail of the
                 // stream, so it runs before the next step and only when needed
@@ -1410,30 +1429,50 @@ __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
                             ctl->err = 2;   // the host's poll runs the pass instead
                     } else {
                         solo = 1;
-                        T.tail->vmax = vbits;
+                        T.tail()->vmax = vbits;
                     }
                 }
             }
         }
-        T.tail->unit[0] = solo;
+        T.tail()->unit[0] = solo;
     }
     if constexpr (!TAILV) {
         __syncthreads();
-        if (T.tail->unit[0] == 0)
+        if (T.tail()->unit[0] == 0)
             return;
         // the pruned maximum is a velocity some cell has: only deeper cells
         // than it allows can raise it
-        const float hcut = Sweep::height_cut(*T.tail, __uint_as_float(T.tail->vmax));
-        const float *h = T.tail->sv.hout;
+        const float hcut = Sweep::height_cut(*T.tail(), __uint_as_float(T.tail()->vmax));
+        const float *h = T.tail()->sv.hout;
         float vmax = 0.0f;
-        for (int i = threadIdx.x; i < nr * g.nc; i += BLK_THREADS)
-            vmax = fmaxf(vmax, velocity_at<float, K, MATH>(g, rk, h, i / g.nc, i % g.nc, hcut));
+        for (int r = wp; r < g.nr; r += BLK_ROWS) {
+            const float *row = h + (long long)(r + PADR) * g.pitch + PADC;
+            for (int c0 = lane * 4; c0 < g.nc; c0 += 512) {
+                float4 v[4];        // the padding right of a row is zeros
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    v[q] = c0 + 128 * q < g.nc
+                               ? *reinterpret_cast<const float4 *>(row + c0 + 128 * q)
+                               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+                for (int q = 0; q < 4; q++) {
+                    const float4 x = q == 0 ? v[0] : q == 1 ? v[1] : q == 2 ? v[2] : v[3];
+                    const float top = fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w));
+                    if (!(top >= hcut))
+                        continue;
+                    for (int j = 0; j < 4; j++)
+                        if (c0 + 128 * q + j < g.nc)
+                            vmax = fmaxf(vmax, velocity_at<float, K, MATH>(
+                                                   g, rk, h, r, c0 + 128 * q + j, hcut));
+                }
+            }
+        }
         vmax = warp_max_nonneg(vmax);
         if (lane == 0)
-            atomicMax(&T.tail->vmax, __float_as_uint(vmax));
+            atomicMax(&T.tail()->vmax, __float_as_uint(vmax));
         __syncthreads();
         if (threadIdx.x == 0) {
-            ctl->vmax_bits = T.tail->vmax;
+            ctl->vmax_bits = T.tail()->vmax;
             finalize<float>(ctl, tc, rk, false);
         }
     }
@@ -1594,7 +1633,8 @@ __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
                      ((128u - (smem_addr(fcab_dsm) & 127u)) & 127u);
     int lane;
     asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
-    const int wp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    int wp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    asm volatile("" : "+r"(wp));
     typename Sweep::Cta T;
     Sweep::attach(T, sm);
     if (threadIdx.x == 0) {
@@ -1621,16 +1661,18 @@ __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
             const int local = u - md.unit_off, strip = local % md.strips;
             const int r0 = local / md.strips * md.seg, r1 = min(md.g.nr, r0 + md.seg);
             if (lane == 0) {
-                if (wp == 0)
-                    Sweep::first_tiles(T, md.g, h_cur, strip, r0, r1);
-                else if (wp == 1)
+                if (wp == 0) {
+                    Sweep::open_unit(T, md.g, md.rk, strip, r0, r1);
+                    Sweep::first_fixed(T, md.g);
+                    Sweep::first_state(T, md.g, h_cur);
+                } else if (wp == 1)
                     Sweep::begin(T, md.g, md.rk, ctl);
                 else if (wp == 2)
-                    T.tail->pre = time_pre(ctl, md.tc, true);
+                    T.tail()->pre = time_pre(ctl, md.tc, true);
             }
             __syncthreads();
             StepSums<float, AccT> ss;
-            Sweep::run(T, md.g, md.rk, h_cur, strip, r0, r1, wp, lane, ss);
+            Sweep::run(T, md.g, md.rk, wp, lane, ss);
             __syncthreads();
             Sweep::publish(T, ss, ctl, lane, u & (NSLOT - 1));
             if (threadIdx.x == 0) {
@@ -1640,7 +1682,7 @@ __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
                     __threadfence();
                     ctl->h_cur = h_cur ^ 1;
                     ctl->launches += 1;
-                    finalize<float>(ctl, md.tc, md.rk, true, T.tail->pre);
+                    finalize<float>(ctl, md.tc, md.rk, true, T.tail()->pre);
                     if (ctl->need_v)    // seed missed: the full pass after this launch
                         need_list[atomicAdd(&q->nneed, 1u)] = m;
                 }

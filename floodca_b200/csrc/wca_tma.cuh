@@ -1,6 +1,6 @@
-// TMA row tiles for the pair sweep: PTX wrappers for mbarriers and 2-D
-// tensor loads (cp.async.bulk.tensor, no multicast), and the host-side
-// tensor maps of a session's padded fields.
+// TMA row tiles of the block sweep: PTX wrappers for mbarriers and 2-D
+// tensor loads (cp.async.bulk.tensor, no multicast), and for a launch that
+// overlaps the one before it.
 #pragma once
 
 #include <cuda.h>
@@ -16,9 +16,14 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p)
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-__device__ __forceinline__ void mbar_init1(uint32_t bar)
+__device__ __forceinline__ void mbar_init2(uint32_t bar)
 {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(bar) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ void mbar_arrive_tx(uint32_t bar, uint32_t bytes)
@@ -52,6 +57,18 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
             return false;
     }
     return true;
+}
+
+// A kernel launched with programmatic stream serialization starts while the
+// one before it is running: wait_previous() holds until that one has finished
+// and its writes are visible; let_next() allows the next one to start.
+__device__ __forceinline__ void wait_previous()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void let_next()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // Orders this thread's earlier generic-proxy accesses to shared memory
