@@ -106,15 +106,20 @@ int load_rday(FcaGrid *g, const char *path, real lambda)
 int drive(FcabSim *s, FcaGrid *g, const FcaRunCfg *cfg, FcaAcc *acc, FcaTimers *tm,
           void (*poll)(void *), void *pctx, int poll_every, double t_wall0)
 {
-    int chunk = 32;
+    int chunk = 32, taken = acc->step;
     for (;;) {
-        if (fcab_sim_advance(s, chunk) != 0)
+        // a run of a fixed number of steps goes out whole (a pause only makes
+        // what was sent past it do nothing)
+        const int left = cfg->steps > 0 ? cfg->steps - taken : 0;
+        const int most = cfg->n_force_days > 0 || poll || cfg->progress_every > 0 ? 256 : 1 << 16;
+        if (fcab_sim_advance(s, left > 0 && left < most ? left : left > 0 ? most : chunk) != 0)
             return -2;
         FcabPoll p;
         if (fcab_sim_poll(s, &p) != 0)
             return -2;
         if (p.done)
             return 0;
+        taken = p.step;
         if (!p.pause) {
             if (chunk < 256)
                 chunk *= 2;

@@ -146,6 +146,52 @@ __global__ void k_encode_mask(const uint8_t *m, float *z, float *n, long long pi
     }
 }
 
+// Counts over a mask: LAND cells of the session's own rows, of their first and
+// last row and column, and with a slab's halo rows; SEA cells; values other
+// than LAND, SEA, WALL; whether cell `cell` of the uploaded rows is LAND.
+struct MaskStats {
+    unsigned int land, land_up, sea, other, north, south, west, east, inflow_land;
+};
+
+__global__ void k_mask_stats(const uint8_t *m, long long pitch, int nr, int nc, int hn, int hs,
+                             long long cell, MaskStats *out)
+{
+    unsigned int land = 0, up = 0, sea = 0, other = 0;
+    const long long N = (long long)(hn + nr + hs) * nc;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N;
+         i += (long long)gridDim.x * blockDim.x) {
+        const int r = (int)(i / nc) - hn, c = (int)(i % nc);
+        const uint8_t v = m[(r + PADR) * pitch + c + PADC];
+        const bool own = r >= 0 && r < nr, is_land = v == M_LAND;
+        land += own && is_land;
+        up += is_land;
+        sea += v == M_SEA;
+        other += v > M_WALL;
+        if (is_land && own) {
+            if (r == 0)
+                atomicAdd(&out->north, 1u);
+            if (r == nr - 1)
+                atomicAdd(&out->south, 1u);
+            if (c == 0)
+                atomicAdd(&out->west, 1u);
+            if (c == nc - 1)
+                atomicAdd(&out->east, 1u);
+        }
+        if (i == cell && is_land)
+            out->inflow_land = 1u;
+    }
+    land = __reduce_add_sync(0xffffffffu, land);
+    up = __reduce_add_sync(0xffffffffu, up);
+    sea = __reduce_add_sync(0xffffffffu, sea);
+    other = __reduce_add_sync(0xffffffffu, other);
+    if ((threadIdx.x & 31) == 0) {
+        if (land) atomicAdd(&out->land, land);
+        if (up) atomicAdd(&out->land_up, up);
+        if (sea) atomicAdd(&out->sea, sea);
+        if (other) atomicAdd(&out->other, other);
+    }
+}
+
 size_t esize_of(int prec) { return prec == FCAB_PREC_F64 ? 8 : 4; }
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
@@ -481,25 +527,26 @@ extern "C" void fcab_sim_destroy(FcabSim *s)
     delete s;
 }
 
-// Copies a row-major nrows x ncols array (host or device) into the interior of
-// a padded field; a slab's arrays carry its halo rows too.
-static cudaError_t put_field(FcabSim *s, void *dst, const void *src, size_t esz,
-                             cudaMemcpyKind kind)
+// A field's interior (a slab's with its halo rows) and the dense array it is
+// copied to or from.
+static fcab::RowCopy whole_field(FcabSim *s, void *dst, const void *src, size_t esz)
 {
-    char *d = (char *)dst + ((size_t)(PADR - s->hn) * s->pitch + PADC) * esz;
-    const size_t rows = (size_t)(s->cfg.nrows + s->hn + s->hs);
-    if (kind == cudaMemcpyHostToDevice)
-        return fcab::h2d_rows(d, (size_t)s->pitch * esz, src, (size_t)s->cfg.ncols * esz, rows,
-                              s->stream);
-    return cudaMemcpy2DAsync(d, (size_t)s->pitch * esz, src, (size_t)s->cfg.ncols * esz,
-                             (size_t)s->cfg.ncols * esz, rows, kind, s->stream);
+    return {(char *)dst + ((size_t)(PADR - s->hn) * s->pitch + PADC) * esz,
+            (size_t)s->pitch * esz, const_cast<void *>(src), (size_t)s->cfg.ncols * esz,
+            (size_t)(s->cfg.nrows + s->hn + s->hs)};
 }
 
-static cudaError_t get_field(FcabSim *s, void *dst, const void *src, size_t esz)
+// Copies row-major arrays (all on the host, or all on the device) into the
+// interiors of padded fields.
+static cudaError_t put_fields(FcabSim *s, const fcab::RowCopy *f, int n, cudaMemcpyKind kind)
 {
-    const char *sp = (const char *)src + ((size_t)PADR * s->pitch + PADC) * esz;
-    return fcab::d2h_rows(dst, sp, (size_t)s->pitch * esz, (size_t)s->cfg.ncols * esz,
-                          (size_t)s->cfg.nrows, s->stream);
+    if (kind == cudaMemcpyHostToDevice)
+        return fcab::h2d_rows(f, n, s->stream);
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < n && e == cudaSuccess; i++)
+        e = cudaMemcpy2DAsync(f[i].dev, f[i].dpitch, f[i].host, f[i].row_bytes, f[i].row_bytes,
+                              f[i].rows, kind, s->stream);
+    return e;
 }
 
 static int fill_interior(FcabSim *s, void *dst, double v)
@@ -590,20 +637,13 @@ static int upload_common(FcabSim *s, const void *z, const void *h, const void *n
     CUDA_TRY(cudaMemsetAsync(s->hmax, 0, s->nelem * es, s->stream));
     CUDA_TRY(cudaMemsetAsync(s->tmax, 0, s->nelem * es, s->stream));
     CUDA_TRY(cudaMemsetAsync(s->m, M_WALL, s->nelem, s->stream));
-    CUDA_TRY(put_field(s, s->z, z, es, kind));
-    CUDA_TRY(put_field(s, s->h0, h, es, kind));
-    CUDA_TRY(put_field(s, s->m, mask, 1, kind));
     if (n) {
         CUDA_TRY(cudaMemsetAsync(s->n, 0, s->nelem * es, s->stream));
-        CUDA_TRY(put_field(s, s->n, n, es, kind));
     } else {
         int rc = fill_interior(s, s->n, as_real(0.03, c.precision));
         if (rc)
             return rc;
     }
-    CUDA_TRY(put_field(s, s->hmax, hmax ? hmax : h, es, kind));
-    if (tmax)
-        CUDA_TRY(put_field(s, s->tmax, tmax, es, kind));
     // staging copies of C and Rday for the rain field
     if (!s->tmpC)
         CUDA_TRY(fcab::cached_malloc(&s->tmpC, s->nelem * es));
@@ -611,63 +651,63 @@ static int upload_common(FcabSim *s, const void *z, const void *h, const void *n
         CUDA_TRY(fcab::cached_malloc(&s->tmpR, s->nelem * es));
     CUDA_TRY(cudaMemsetAsync(s->tmpC, 0, s->nelem * es, s->stream));
     CUDA_TRY(cudaMemsetAsync(s->tmpR, 0, s->nelem * es, s->stream));
+    fcab::RowCopy f[8];
+    int nf = 0;
+    f[nf++] = whole_field(s, s->z, z, es);
+    f[nf++] = whole_field(s, s->h0, h, es);
+    f[nf++] = whole_field(s, s->m, mask, 1);
+    if (n)
+        f[nf++] = whole_field(s, s->n, n, es);
+    if (hmax && hmax != h)
+        f[nf++] = whole_field(s, s->hmax, hmax, es);
+    if (tmax)
+        f[nf++] = whole_field(s, s->tmax, tmax, es);
     if (C)
-        CUDA_TRY(put_field(s, s->tmpC, C, es, kind));
+        f[nf++] = whole_field(s, s->tmpC, C, es);
     if (Rday)
-        CUDA_TRY(put_field(s, s->tmpR, Rday, es, kind));
+        f[nf++] = whole_field(s, s->tmpR, Rday, es);
+    CUDA_TRY(put_fields(s, f, nf, kind));
+    if (!hmax || hmax == h)
+        CUDA_TRY(cudaMemcpyAsync(s->hmax, s->h0, s->nelem * es, cudaMemcpyDeviceToDevice,
+                                 s->stream));
     int rc = rebuild_rain(s, true);
     if (rc)
         return rc;
-    // has SEA / inflow cell LAND
-    std::vector<uint8_t> probe;
+    // what the mask holds, and whether the inflow cell is LAND
     const long long N = (long long)c.nrows * c.ncols;
     const long long Nup = (long long)(c.nrows + s->hn + s->hs) * c.ncols;   // with halo rows
-    const uint8_t *mup = mask;
-    if (kind != cudaMemcpyHostToDevice) {
-        probe.resize((size_t)Nup);
-        CUDA_TRY(cudaMemcpy(probe.data(), mask, (size_t)Nup, cudaMemcpyDeviceToHost));
-        mup = probe.data();
-    }
-    const uint8_t *mh = mup + (long long)s->hn * c.ncols;              // own rows
-    const int has_sea = memchr(mup, M_SEA, (size_t)Nup) != nullptr;
-    // LAND cells per row; open faces only on the open edges' rows/columns
-    s->land_cells = 0;
+    MaskStats ms;
+    memset(&ms, 0, sizeof(ms));
+    static_assert(sizeof(MaskStats) <= 64, "session scratch");
+    CUDA_TRY(cudaMemsetAsync(s->scratch, 0, sizeof(MaskStats), s->stream));
+    k_mask_stats<<<512, 256, 0, s->stream>>>(s->m, s->pitch, c.nrows, c.ncols, s->hn, s->hs,
+                                             c.inflow_cell >= 0 && c.inflow_cell < Nup
+                                                 ? c.inflow_cell
+                                                 : -1,
+                                             (MaskStats *)s->scratch);
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaMemcpyAsync(&ms, s->scratch, sizeof(ms), cudaMemcpyDeviceToHost, s->stream));
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    const int has_sea = ms.sea != 0;
+    // open faces only on the open edges' rows and columns
+    s->land_cells = (long long)ms.land;
     s->open_faces = 0;
-    const bool open = c.boundary == FCA_BND_OPEN;
-    uint8_t mask_max = 0;
-    for (long long r = 0; r < c.nrows; r++) {
-        const uint8_t *row = mh + r * c.ncols;
-        long long cnt = 0;
-        for (long long k = 0; k < c.ncols; k++) {
-            cnt += row[k] == M_LAND;
-            mask_max = std::max(mask_max, row[k]);
-        }
-        s->land_cells += cnt;
-        if (open) {
-            s->open_faces += (r == 0 && c.edge_n ? cnt : 0) + (r == c.nrows - 1 && c.edge_s ? cnt : 0);
-            s->open_faces += (c.edge_w && row[0] == M_LAND) + (c.edge_e && row[c.ncols - 1] == M_LAND);
-        }
-    }
+    if (c.boundary == FCA_BND_OPEN)
+        s->open_faces = (c.edge_n ? (long long)ms.north : 0) + (c.edge_s ? (long long)ms.south : 0) +
+                        (c.edge_w ? (long long)ms.west : 0) + (c.edge_e ? (long long)ms.east : 0);
     // all-LAND grids use the mask-free kernel: padding elevation PAD_Z makes
     // every face to the padding carry zero discharge (needs tau_h > 0)
-    long long land_up = s->land_cells;       // with a slab's halo rows
-    for (long long k = 0; k < (long long)s->hn * c.ncols; k++)
-        land_up += mup[k] == M_LAND;
-    for (long long k = N + (long long)s->hn * c.ncols; k < Nup; k++)
-        land_up += mup[k] == M_LAND;
-    const bool all_land = c.tau_h > 0.0 && s->land_cells == N && land_up == Nup;
+    const bool all_land = c.tau_h > 0.0 && s->land_cells == N && (long long)ms.land_up == Nup;
     s->landonly = all_land;
     // FP32 grids with other cells: the mask goes into z and n (block sweep);
     // a slab's stays on the sweep by warp, which counts its own sea outflow
-    s->mask_coded = !all_land && es == 4 && s->use_tma && !s->slab && mask_max <= M_WALL;
+    s->mask_coded = !all_land && es == 4 && s->use_tma && !s->slab && ms.other == 0;
     if (s->mask_coded) {
         k_encode_mask<<<1024, 256, 0, s->stream>>>(s->m, (float *)s->z, (float *)s->n, s->pitch,
                                                    (int)c.nrows, (int)c.ncols);
         CUDA_TRY(cudaGetLastError());
     }
-    int inflow_ok = 0;
-    if (c.inflow_cell >= 0 && c.inflow_cell < Nup)
-        inflow_ok = mup[c.inflow_cell] == M_LAND;
+    const int inflow_ok = ms.inflow_land != 0;
     const long long nr = c.nrows, nc = c.ncols;
     // a slab also owns the faces between its last row and the south halo
     const long long ny = nr - 1 + (s->hs > 0 ? 1 : 0);
@@ -702,10 +742,13 @@ extern "C" int fcab_sim_set_rain(FcabSim *s, const void *C, const void *Rday)
 {
     if (!s->uploaded)
         return fail(FCAB_ERR_STATE, "set_rain before upload");
+    fcab::RowCopy f[2];
+    int nf = 0;
     if (C)
-        CUDA_TRY(put_field(s, s->tmpC, C, s->esize, cudaMemcpyHostToDevice));
+        f[nf++] = whole_field(s, s->tmpC, C, s->esize);
     if (Rday)
-        CUDA_TRY(put_field(s, s->tmpR, Rday, s->esize, cudaMemcpyHostToDevice));
+        f[nf++] = whole_field(s, s->tmpR, Rday, s->esize);
+    CUDA_TRY(put_fields(s, f, nf, cudaMemcpyHostToDevice));
     return rebuild_rain(s, false);
 }
 
@@ -972,9 +1015,12 @@ extern "C" int fcab_sim_resume(FcabSim *s, int force_day)
 extern "C" int fcab_sim_run(FcabSim *s)
 {
     FcabPoll p;
-    int chunk = GRAPH_STEPS;
+    int chunk = GRAPH_STEPS, done_steps = s->step0;
     for (;;) {
-        int rc = fcab_sim_advance(s, chunk);
+        // a run of a fixed number of steps goes out whole, whatever it is
+        // (steps past the end do nothing, but cost a launch each)
+        const int left = s->cfg.max_steps > 0 ? s->cfg.max_steps - done_steps : 0;
+        int rc = fcab_sim_advance(s, left > 0 ? std::min(left, 1 << 16) : chunk);
         if (rc)
             return rc;
         rc = fcab_sim_poll(s, &p);
@@ -984,6 +1030,7 @@ extern "C" int fcab_sim_run(FcabSim *s)
             return 0;
         if (p.pause)
             return fail(FCAB_ERR_STATE, "run paused (forcing or progress); use the drop-in loop");
+        done_steps = p.step;
         if (chunk < 8 * GRAPH_STEPS)
             chunk *= 2;
     }
@@ -1048,12 +1095,21 @@ extern "C" int fcab_sim_download(FcabSim *s, void *h, void *hmax, void *tmax)
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     const Ctl *c = (const Ctl *)s->ctl_host;
     s->h_cur_host = c->h_cur;
+    fcab::RowCopy f[3];
+    int nf = 0;
+    auto own_rows = [&](void *dst, void *src) {
+        fcab::RowCopy x = whole_field(s, src, dst, s->esize);
+        x.dev = (char *)x.dev + (size_t)s->hn * x.dpitch;
+        x.rows = (size_t)s->cfg.nrows;
+        f[nf++] = x;
+    };
     if (h)
-        CUDA_TRY(get_field(s, h, c->h_cur ? s->h1 : s->h0, s->esize));
+        own_rows(h, c->h_cur ? s->h1 : s->h0);
     if (hmax)
-        CUDA_TRY(get_field(s, hmax, s->hmax, s->esize));
+        own_rows(hmax, s->hmax);
     if (tmax)
-        CUDA_TRY(get_field(s, tmax, s->tmax, s->esize));
+        own_rows(tmax, s->tmax);
+    CUDA_TRY(fcab::d2h_rows(f, nf, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     return 0;
 }
@@ -1161,11 +1217,18 @@ extern "C" int fcab_sim_upload_state(FcabSim *s, const void *h, const void *hmax
     if (!h)
         return fail(FCAB_ERR_ARG, "h is required");
     s->h_cur_host = 0;
-    CUDA_TRY(put_field(s, s->h0, h, s->esize, cudaMemcpyHostToDevice));
-    CUDA_TRY(put_field(s, s->hmax, hmax ? hmax : h, s->esize, cudaMemcpyHostToDevice));
+    fcab::RowCopy f[3];
+    int nf = 0;
+    f[nf++] = whole_field(s, s->h0, h, s->esize);
+    if (hmax && hmax != h)
+        f[nf++] = whole_field(s, s->hmax, hmax, s->esize);
     if (tmax)
-        CUDA_TRY(put_field(s, s->tmax, tmax, s->esize, cudaMemcpyHostToDevice));
-    else
+        f[nf++] = whole_field(s, s->tmax, tmax, s->esize);
+    CUDA_TRY(put_fields(s, f, nf, cudaMemcpyHostToDevice));
+    if (!hmax || hmax == h)     // the padding of both is zeros
+        CUDA_TRY(cudaMemcpyAsync(s->hmax, s->h0, s->nelem * s->esize, cudaMemcpyDeviceToDevice,
+                                 s->stream));
+    if (!tmax)
         CUDA_TRY(cudaMemsetAsync(s->tmax, 0, s->nelem * s->esize, s->stream));
     return 0;
 }

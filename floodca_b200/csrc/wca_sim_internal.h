@@ -69,10 +69,15 @@ void make_run_params_f32(const FcabConfig &cfg, RunK<float> *rk, TimeCfg *tc);
 // h2d_rows returns once the host rows have been read (the transfer may still
 // run; later work on `stream` follows it); d2h_rows returns with the host
 // rows written.
-cudaError_t h2d_rows(void *dst, size_t dpitch, const void *src, size_t row_bytes, size_t rows,
-                     cudaStream_t stream);
-cudaError_t d2h_rows(void *dst, const void *src, size_t spitch, size_t row_bytes, size_t rows,
-                     cudaStream_t stream);
+// Several fields go through the threads together.
+struct RowCopy {
+    void *dev;              // first device row
+    size_t dpitch;          // bytes from row to row
+    void *host;             // dense host rows
+    size_t row_bytes, rows;
+};
+cudaError_t h2d_rows(const RowCopy *f, int n, cudaStream_t stream);
+cudaError_t d2h_rows(const RowCopy *f, int n, cudaStream_t stream);
 // Caching allocator of session buffers (mem_cache.cu): freed blocks are kept
 // per device for the next request of about the same size. A block must be
 // idle (its stream synchronised) when it is freed.
