@@ -94,6 +94,7 @@ def core() -> C.CDLL:
         "fcab_unet_add": (C.c_int, [_P, _P, _LL, _P]),
         "fcab_unet_relu_bwd": (C.c_int, [_P, _P, _LL, _P]),
         "fcab_unet_dropout": (C.c_int, [_P, _LL, C.c_float, C.c_uint32, _P]),
+        "fcab_unet_act_bwd": (C.c_int, [_P, _P, _LL, _I, C.c_float, C.c_uint32, _P, _P]),
         "fcab_unet_bias_grad": (C.c_int, [_P, _LL, _I, _P, _P]),
         "fcab_unet_head_fwd": (C.c_int, [_P, _P, _P, _P, _I, _I, _I, _I, _P]),
         "fcab_unet_head_bwd": (C.c_int, [_P] * 8 + [_I, _I, _I, _I, _P]),

@@ -96,6 +96,12 @@ class UNet:
         self.dhb = torch.zeros_like(self.hb)
         self.hstate = [torch.zeros_like(self.hw), torch.zeros_like(self.hw),
                        torch.zeros_like(self.hb), torch.zeros_like(self.hb)]
+        # one buffer behind every gradient, cleared by one launch
+        owners = [(c, k) for c in self.convs() for k in ("dw", "db")] + [(self, "dhw"), (self, "dhb")]
+        sizes = [getattr(o, k).numel() for o, k in owners]
+        self._grads = torch.zeros(sum(sizes), device=device)
+        for (o, k), part in zip(owners, self._grads.split(sizes)):
+            setattr(o, k, part.view_as(getattr(o, k)))
         self.step_t = 0
         self._bufs = {}
 
@@ -192,10 +198,9 @@ class UNet:
     def _conv_bwd(self, conv, g, x, y, N, H, W, key, need_dx, st, drop_seed=None):
         """g: gradient at the conv's (post-ReLU, post-dropout) output y."""
         L = self.L
-        if drop_seed is not None:
-            self._drop(g, drop_seed, st)
-        check(L.fcab_unet_relu_bwd(_p(g), _p(y), g.numel(), st), "relu_bwd")
-        check(L.fcab_unet_bias_grad(_p(g), g.shape[0], conv.cout, _p(conv.db), st), "bias_grad")
+        p, seed = (0.0, 0) if drop_seed is None else (self.p_drop, drop_seed & 0xFFFFFFFF)
+        check(L.fcab_unet_act_bwd(_p(g), _p(y), g.numel(), conv.cout, p, seed, _p(conv.db), st),
+              "act_bwd")
         check(L.fcab_unet_conv_wgrad(_p(g), _p(x), N, H, W, conv.cin, conv.cout, _p(conv.dw), st),
               "wgrad")
         if not need_dx:
@@ -214,11 +219,7 @@ class UNet:
         N, H, W = self.N, self.H, self.W
         A = self.acts
         seed = self.seed
-        for t in (self.dhw, self.dhb):
-            t.zero_()
-        for c in self.convs():
-            c.dw.zero_()
-            c.db.zero_()
+        self._grads.zero_()
         self.loss_sum = torch.zeros(1, device=self.device)
         c0 = self.dec[2][1].cout
         g = self._buf("g_head", N, H, W, c0)

@@ -493,6 +493,12 @@ FCAB_API int fcab_unet_add(void *y, const void *x, long long n, void *stream);
 FCAB_API int fcab_unet_relu_bwd(void *g, const void *y, long long n, void *stream);
 /* In-place inverted dropout with a hashed mask of (seed, element). */
 FCAB_API int fcab_unet_dropout(void *x, long long n, float p, uint32_t seed, void *stream);
+/* The dropout (p > 0: the mask of fcab_unet_dropout with this seed), ReLU
+ * and bias gradients at a convolution's output in one pass: g is masked and
+ * scaled, then zeroed where y <= 0, and its channel sums go into db[C]; n
+ * elements, C = 8 times a power of two up to 512. */
+FCAB_API int fcab_unet_act_bwd(void *g, const void *y, long long n, int C, float p, uint32_t seed,
+                               float *db, void *stream);
 /* db[c] += sum over the P rows of g[.][C]. */
 FCAB_API int fcab_unet_bias_grad(const void *g, long long P, int C, float *db, void *stream);
 /* 1x1 output head C -> 1 (C = 32 or 64): out[N][H][W] fp32. */

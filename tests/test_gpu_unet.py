@@ -232,6 +232,29 @@ def test_dropout_bias_head_adam():
     assert np.allclose(w.cpu().numpy(), ww, rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("C,P,p", [(32, 1, 0.0), (32, 70001, 0.1), (64, 4099, 0.5), (128, 515, 0.1),
+                                   (256, 33, 0.0), (256, 2050, 0.25)])
+def test_act_bwd_equals_its_three_passes(C, P, p):
+    """The fused gradient at a convolution's output against the dropout, ReLU
+    and bias passes of their own: g bit for bit; the bias sums, of the same
+    bf16 values in another order, within P FP32 roundings of their magnitude
+    (at most 2^-24 sqrt(P) relative in the mean; 1e-5 of the sum of magnitudes)."""
+    L = core()
+    gen = torch.Generator(device="cuda").manual_seed(C + P)
+    g = torch.randn((P, C), generator=gen, device="cuda").to(torch.bfloat16)
+    y = torch.randn((P, C), generator=gen, device="cuda").clamp_min(0).to(torch.bfloat16)
+    want, got = g.clone(), g.clone()
+    if p > 0:
+        assert L.fcab_unet_dropout(_p(want), want.numel(), p, 77, None) == 0
+    assert L.fcab_unet_relu_bwd(_p(want), _p(y), want.numel(), None) == 0
+    db = torch.ones(C, device="cuda")
+    assert L.fcab_unet_act_bwd(_p(got), _p(y), got.numel(), C, p, 77, _p(db), None) == 0
+    assert torch.equal(got.view(torch.int16), want.view(torch.int16))
+    w = want.double()
+    assert bool(((db.double() - 1 - w.sum(0)).abs() <= 1e-5 * w.abs().sum(0) + 1e-6).all())
+    assert L.fcab_unet_act_bwd(_p(got), _p(y), got.numel(), 24, p, 77, _p(db), None) != 0
+
+
 def _bf16_round(t):
     """Rounds to bf16 in the forward pass with an identity gradient, where the
     kernels store bf16 activations (so ReLU masks and pooling arg maxes see
