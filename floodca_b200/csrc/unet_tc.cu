@@ -681,61 +681,90 @@ k_conv_halo(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUte
 }
 
 // ---------------------------------------------------------------------------
-// Weight gradient: dW[co][tap][ci] += sum_p dY[p][co] * X[p + shift(tap)][ci]
-// as M = 128 output channels x N = 64*NB input channels x K = pixels, both
-// operands MN-major (channels contiguous): each is loaded as boxes of 64
-// channels x 64 pixels (128-byte swizzle; K groups of 8 pixels 1024 B apart,
-// 64-channel blocks 8 KB apart). Each CTA takes one tap, one channel tile and
-// one pixel range and adds its partial sums with FP32 atomics.
+// Weight gradient: dW[co][tap][ci] += sum_q dY[q - (v-1)*Wp][co] * X[q + h-1][ci]
+// for tap = 3*v + h, as a GEMM over pixels q with both operands MN-major
+// (channels contiguous). A tap is a shift of one operand by whole pixels, and
+// a pixel is one row of a tile, so one pair of tiles serves several taps:
+//   h  the three are the N blocks of one B operand: X rows q-1 .. q+64 in one
+//      tile of 66 rows, block h starting h rows in (leading byte offset = one
+//      row; the swizzle follows the shared-memory address, so a block may
+//      start anywhere in its pattern). N = 3 * XB.
+//   v  is a shift of dY. With Cout = 32 three tiles, one per v, are the M
+//      blocks (M = 128, the fourth unread), with Cout = 64 two, and v 2 is
+//      another CTA's; more output channels fill M, one v to a CTA.
+// A CTA takes a range of pixels and at most 192 columns of sums, so that two
+// fit an SM's TMEM and one's epilogue (16-byte FP32 atomics to dW where its
+// alignment allows) runs beside the other's loop.
+// The bound is the tensor cores' reading of MN-major operands, about 32 bytes
+// a cycle: 128 cycles for M = 128 x K = 16 and 2 N/2 for N (261 a MMA for N =
+// 96, 320 for 192, where the products take 24 and 48). One tap per CTA read A
+// nine times, this reads it once or three times. Measured, 32 images of 256 x
+// 256, all 14 layers: 3.44 ms before, 1.71 now (32 to 32 channels 331 to
+// 220 us, 192 to 64 381 to 146, 384 to 128 224 to 105).
+//
+// Tensor-core sums are cut off, not rounded, once per MMA, so the error of a
+// partial sum grows with its pixels (1e-4 of dW at the full resolution's
+// 33,000): a range is never longer than it was, and shorter by at most 32
+// steps, which keeps dW within 1e-5 of what it was. At the full resolution
+// that leaves half of the SMs idle; 148 ranges took 146 us there.
 
 struct WgArgs {
-    int P, Wp, Cin, Cout;
-    int kpc;      // 64-pixel steps per CTA
-    float *dw;    // [Cout][9][Cin]
+    int Wp, Cin, Cout;
+    int kpc, ksteps;  // 64-pixel steps per CTA and in all
+    int nx;           // x blocks (of XB channels) per CTA
+    int ci_groups;    // CTAs side by side on the input channels
+    int stages, stage_bytes;
+    int vec;          // dw is 16-byte aligned
+    float *dw;        // [Cout][9][Cin]
 };
 
-template <int NB>
-struct WgCfg {
-    static constexpr int A_BYTES = 2 * 8192;
-    static constexpr int B_BYTES = NB * 8192;
-    static constexpr int STAGE = A_BYTES + B_BYTES;
-    static constexpr int STAGES = 4;
-    static constexpr uint32_t TCOLS = NB == 1 ? 64 : NB == 2 ? 128 : 256;
-    static constexpr int SMEM = 1024 + STAGES * STAGE + (2 * STAGES + 1) * 8 + 16;
+// Row of 2*B bytes, tile strides in shared memory (B = 32: 64-byte swizzle,
+// 512-byte pattern; 64: 128-byte swizzle, 1024-byte pattern).
+template <int B>
+struct WgTile {
+    static constexpr uint32_t ROW = 2u * B;
+    static constexpr uint32_t DY = 64u * ROW;
+    static constexpr uint32_t XBYTES = 66u * ROW;
+    static constexpr uint32_t X = (XBYTES + 8u * ROW - 1) / (8u * ROW) * (8u * ROW);
+    static constexpr uint32_t layout = B == 64 ? 2u : 4u;
 };
 
-template <int NB>
-__global__ void __launch_bounds__(128, 1)
+template <int DB, int XB>
+__global__ void __launch_bounds__(256, 2)
 k_conv_wgrad(const __grid_constant__ CUtensorMap tdy, const __grid_constant__ CUtensorMap tx, WgArgs a)
 {
-    using Cfg = WgCfg<NB>;
-    constexpr int S = Cfg::STAGES;
+    using D = WgTile<DB>;
+    using X = WgTile<XB>;
+    constexpr int NCOL = 3 * XB;    // TMEM columns of one MMA
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t *sm = smem_raw + (base - raw);
-    const uint32_t bar0 = base + S * Cfg::STAGE;
-    uint32_t *tslot = (uint32_t *)(sm + S * Cfg::STAGE + (2 * S + 1) * 8);
+    const int S = a.stages;
+    const uint32_t bar0 = base + (uint32_t)(S * a.stage_bytes);
+    uint32_t *tslot = (uint32_t *)(sm + S * a.stage_bytes + (2 * S + 1) * 8);
     auto full = [&](int s) { return bar0 + 8u * s; };
     auto empty = [&](int s) { return bar0 + 8u * (S + s); };
     const uint32_t done = bar0 + 8u * (2 * S);
-    auto sA = [&](int s) { return base + (uint32_t)(s * Cfg::STAGE); };
-    auto sB = [&](int s) { return base + (uint32_t)(s * Cfg::STAGE + Cfg::A_BYTES); };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tap = blockIdx.y % 9;
-    const int co0 = (blockIdx.y / 9) * 128;
-    const int ci0 = blockIdx.z * 64 * NB;
-    const int kb0 = blockIdx.x * a.kpc;
-    const int ksteps_total = (a.P + 63) / 64;
-    int nk = ksteps_total - kb0;
-    nk = nk < a.kpc ? nk : a.kpc;
+    // which taps and channels (x), which pixels (y)
+    const int cg = blockIdx.x % a.ci_groups, vg = blockIdx.x / a.ci_groups;
+    const bool wide = DB == 64 && a.Cout > 64;
+    const int v0 = DB == 32 ? 0 : wide ? vg % 3 : 2 * vg;
+    const int co0 = wide ? vg / 3 * 128 : 0;
+    const int ci0 = cg * a.nx * XB;
+    const int kb0 = blockIdx.y * a.kpc;
+    const int nk = min(a.kpc, a.ksteps - kb0);
     if (nk <= 0)
         return;     // uniform across the CTA, before any allocation
-    const int na = (a.Cout - co0) >= 128 ? 2 : ((a.Cout - co0) + 63) / 64;
-    int nb = (a.Cin - ci0 + 63) / 64;
-    nb = nb < NB ? nb : NB;
-    const int shift = (tap / 3 - 1) * a.Wp + (tap % 3 - 1);
+    // dY tiles: by v, or by channel
+    const int nd = wide ? (a.Cout - co0 > 64 ? 2 : 1) : DB == 32 ? 3 : 2 - vg;
+    const int nx = min(a.nx, (a.Cin - ci0 + XB - 1) / XB);
+    const uint32_t xoff = (DB == 32 ? 3u : 2u) * D::DY;       // first x tile of a stage
+    uint32_t tcols = 32;
+    while (tcols < (uint32_t)(nx * NCOL))
+        tcols *= 2;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; s++) {
@@ -747,70 +776,98 @@ k_conv_wgrad(const __grid_constant__ CUtensorMap tdy, const __grid_constant__ CU
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 0)
-        tmem_alloc(smem_u32(tslot), Cfg::TCOLS);
+        tmem_alloc(smem_u32(tslot), tcols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
     if (warp == 0 && lane == 0) {
+        int s = 0, round = 0;
         for (int k = 0; k < nk; k++) {
-            const int s = k % S;
-            if (k >= S && !mbar_wait(empty(s), (uint32_t)((k / S) - 1) & 1u)) {
+            if (round > 0 && !mbar_wait(empty(s), (uint32_t)(round - 1) & 1u)) {
                 set_err(4);
                 break;
             }
-            const int px = (kb0 + k) * 64;
-            mbar_expect_tx(full(s), (uint32_t)(na + nb) * 8192u);
-            for (int j = 0; j < na; j++)
-                tma_load_2d(sA(s) + 8192u * j, &tdy, full(s), co0 + 64 * j, px);
-            for (int j = 0; j < nb; j++)
-                tma_load_2d(sB(s) + 8192u * j, &tx, full(s), ci0 + 64 * j, px + shift);
+            const uint32_t st = base + (uint32_t)(s * a.stage_bytes);
+            const int q = (kb0 + k) * 64 - 1;
+            mbar_expect_tx(full(s), (uint32_t)nd * D::DY + (uint32_t)nx * X::XBYTES);
+            for (int j = 0; j < nd; j++)
+                tma_load_2d(st + j * D::DY, &tdy, full(s), wide ? co0 + DB * j : 0,
+                            q - (v0 + (wide ? 0 : j) - 1) * a.Wp);
+            for (int b = 0; b < nx; b++)
+                tma_load_2d(st + xoff + b * X::X, &tx, full(s), ci0 + XB * b, q - 1);
+            if (++s == S) {
+                s = 0;
+                round++;
+            }
         }
     } else if (warp == 1 && lane == 0) {
-        // N = 64 * nb columns (the blocks that were loaded)
-        const uint32_t idesc = idesc_bf16(128, 64 * nb, true, true);
+        const uint32_t idesc = idesc_bf16(128, NCOL, true, true);
+        int s = 0;
+        uint32_t par = 0;
         for (int k = 0; k < nk; k++) {
-            const int s = k % S;
-            if (!mbar_wait(full(s), (uint32_t)(k / S) & 1u)) {
+            if (!mbar_wait(full(s), par)) {
                 set_err(5);
                 break;
             }
             tc_fence_after();
+            const uint32_t st = base + (uint32_t)(s * a.stage_bytes);
 #pragma unroll
             for (int kk = 0; kk < 4; kk++) {
-                const uint64_t ad = smem_desc(sA(s) + 2048u * kk, 8192u, 1024u, 2u);
-                const uint64_t bd = smem_desc(sB(s) + 2048u * kk, 8192u, 1024u, 2u);
-                umma_bf16(tmem, ad, bd, idesc, (k | kk) != 0 ? 1u : 0u);
+                // a single 64-channel tile stands for both M blocks
+                const uint64_t ad = smem_desc(st + 16 * kk * D::ROW, nd == 1 ? 0u : D::DY, 8 * D::ROW,
+                                              D::layout);
+                for (int b = 0; b < nx; b++) {
+                    const uint64_t bd = smem_desc(st + xoff + b * X::X + 16 * kk * X::ROW, X::ROW,
+                                                  8 * X::ROW, X::layout);
+                    umma_bf16(tmem + (uint32_t)(b * NCOL), ad, bd, idesc, (k | kk) != 0 ? 1u : 0u);
+                }
             }
             umma_commit(empty(s));
+            if (++s == S) {
+                s = 0;
+                par ^= 1u;
+            }
         }
         umma_commit(done);
+        if (!mbar_wait(done, 0))
+            set_err(6);
     }
-    __syncwarp();
-    if (!mbar_wait(done, 0))
-        set_err(6);
-    __syncwarp();
+    __syncthreads();
     tc_fence_after();
 
-    const int co = co0 + warp * 32 + lane;
-    const bool live = co < a.Cout;
+    // warps w and w + 4 read TMEM lanes 32*(w%4).. of alternate 32-column chunks
+    const int row = (warp & 3) * 32 + lane;
+    const int v = wide ? v0 : v0 + row / DB, co = wide ? co0 + row : row % DB;
+    const bool live = v < 3 && co < a.Cout;
+    const int chunks = nx * NCOL / 32;
 #pragma unroll 1
-    for (int c = 0; c < 64 * nb; c += 32) {
-        float v[32];
-        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
+    for (int ch = warp >> 2; ch < chunks; ch += 2) {
+        float t[32];
+        tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(ch * 32), t);
+        const int b = ch * 32 / NCOL, rem = ch * 32 % NCOL;
+        const int ci = ci0 + b * XB + rem % XB;
         if (live) {
-            float *dst = a.dw + ((size_t)co * 9 + tap) * a.Cin + ci0 + c;
+            float *dst = a.dw + ((size_t)co * 9 + v * 3 + rem / XB) * a.Cin + ci;
 #pragma unroll
-            for (int j = 0; j < 32; j++)
-                if (ci0 + c + j < a.Cin)
-                    atomicAdd(dst + j, v[j]);
+            for (int j = 0; j < 32; j += 4) {
+                if (ci + j >= a.Cin)
+                    continue;
+                if (a.vec) {
+                    atomicAdd((float4 *)(dst + j), make_float4(t[j], t[j + 1], t[j + 2], t[j + 3]));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        atomicAdd(dst + j + i, t[j + i]);
+                }
+            }
         }
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 0)
-        tmem_dealloc(tmem, Cfg::TCOLS);
+        tmem_dealloc(tmem, tcols);
 }
 
 // ---------------------------------------------------------------------------
@@ -1483,22 +1540,30 @@ int conv_gemm(const void *x, int N, int H, int W, int Cin, const void *w, int Co
     return 0;
 }
 
-template <int NB>
-cudaError_t launch_wgrad(const CUtensorMap &tdy, const CUtensorMap &tx, const WgArgs &a, dim3 grid,
-                         cudaStream_t st)
+template <int DB, int XB>
+cudaError_t launch_wgrad(const void *dy, const void *x, long long P, WgArgs a, dim3 grid, cudaStream_t st)
 {
-    using Cfg = WgCfg<NB>;
+    using D = WgTile<DB>;
+    using X = WgTile<XB>;
+    CUtensorMap tdy, tx;
+    if (!make_map(&tdy, dy, P, a.Cout, DB, 64, DB == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B) ||
+        !make_map(&tx, x, P, a.Cin, XB, 66, XB == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B))
+        return cudaErrorInvalidValue;
+    a.stage_bytes = (int)(((DB == 32 ? 3 : 2) * D::DY + a.nx * X::X + 1023) / 1024 * 1024);
+    // two CTAs per SM
+    a.stages = (SMEM_MAX / 2 - 2048 - 256) / a.stage_bytes;
+    const int smem = 1024 + a.stages * a.stage_bytes + 256;
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (!attr_set[dev & 63]) {
-        cudaError_t e = cudaFuncSetAttribute(k_conv_wgrad<NB>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(k_conv_wgrad<DB, XB>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX / 2);
         if (e != cudaSuccess)
             return e;
         attr_set[dev & 63] = true;
     }
-    k_conv_wgrad<NB><<<grid, 128, Cfg::SMEM, st>>>(tdy, tx, a);
+    k_conv_wgrad<DB, XB><<<grid, 256, smem, st>>>(tdy, tx, a);
     return cudaGetLastError();
 }
 
@@ -1534,36 +1599,40 @@ int fcab_unet_conv_wgrad(const void *dy, const void *x, int N, int H, int W, int
     const long long P = (long long)N * (H + 2) * (W + 2);
     if (P >= (1ll << 31) - 256)
         return fail(FCAB_ERR_ARG, "wgrad: too many pixels");
-    CUtensorMap tdy, tx;
-    if (!make_map(&tdy, dy, P, Cout, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B) ||
-        !make_map(&tx, x, P, Cin, 64, 64, CU_TENSOR_MAP_SWIZZLE_128B))
-        return fail(FCAB_ERR_CUDA, "wgrad: tensor map encoding failed");
-    const int nb_needed = (Cin + 63) / 64;
-    const int NB = nb_needed >= 4 ? 4 : nb_needed;
-    const int ci_tiles = (Cin + 64 * NB - 1) / (64 * NB);
-    const int co_tiles = (Cout + 127) / 128;
-    const long long ksteps = (P + 63) / 64;
-    // about four CTAs per SM in total
-    long long want = (148LL * 4) / (9LL * co_tiles * ci_tiles);
-    if (want < 1)
-        want = 1;
-    long long kpc = (ksteps + want - 1) / want;
-    if (kpc < 8)
-        kpc = 8;
-    const long long splits = (ksteps + kpc - 1) / kpc;
+    // x blocks of 64 channels where they divide Cin, else of 32 (N = 96 beside
+    // 192 in one MMA, but no work on channels that are not there)
+    const bool x64 = Cin % 64 == 0;
+    const int XB = x64 ? 64 : 32;
     WgArgs a;
-    a.P = (int)P;
     a.Wp = W + 2;
     a.Cin = Cin;
     a.Cout = Cout;
-    a.kpc = (int)kpc;
+    a.vec = ((uintptr_t)dw & 15) == 0;
     a.dw = dw;
-    dim3 grid((unsigned)splits, (unsigned)(9 * co_tiles), (unsigned)ci_tiles);
+    // q runs over -1 .. P, beyond which no tap of X is inside
+    a.ksteps = (int)((P + 2 + 63) / 64);
+    a.nx = Cin > 32 && !x64 ? 2 : 1;                        // by the 192 columns
+    const int nblk = (Cin + XB - 1) / XB;
+    a.ci_groups = (nblk + a.nx - 1) / a.nx;
+    const int co_tiles = (Cout + 127) / 128;
+    const int groups = a.ci_groups * (Cout == 32 ? 1 : Cout == 64 ? 2 : 3 * co_tiles);
+    // At least 592 / 9 ranges over the channel tiles of 128 x 256 (and 8 steps
+    // in each), more where that evens out the waves and shortens a range by at
+    // most 32 steps.
+    int want = 592 / (9 * co_tiles * ((Cin + 255) / 256));
+    want = want < 1 ? 1 : want;
+    const int most = (a.ksteps + want - 1) / want;
+    const int even = (want * groups + 147) / 148 * 148 / groups;
+    a.kpc = (a.ksteps + even - 1) / even;
+    a.kpc = a.kpc < most - 32 ? most - 32 : a.kpc;
+    a.kpc = a.kpc < most - most / 6 ? most : a.kpc;
+    a.kpc = a.kpc < 8 ? 8 : a.kpc;
+    const dim3 grid((unsigned)groups, (unsigned)((a.ksteps + a.kpc - 1) / a.kpc));
     cudaStream_t st = (cudaStream_t)stream;
-    cudaError_t e = NB == 1   ? launch_wgrad<1>(tdy, tx, a, grid, st)
-                    : NB == 2 ? launch_wgrad<2>(tdy, tx, a, grid, st)
-                    : NB == 3 ? launch_wgrad<3>(tdy, tx, a, grid, st)
-                              : launch_wgrad<4>(tdy, tx, a, grid, st);
+    cudaError_t e = Cout == 32 ? (x64 ? launch_wgrad<32, 64>(dy, x, P, a, grid, st)
+                                      : launch_wgrad<32, 32>(dy, x, P, a, grid, st))
+                               : (x64 ? launch_wgrad<64, 64>(dy, x, P, a, grid, st)
+                                      : launch_wgrad<64, 32>(dy, x, P, a, grid, st));
     if (e != cudaSuccess)
         return fail(FCAB_ERR_CUDA, cudaGetErrorString(e));
     return 0;

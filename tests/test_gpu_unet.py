@@ -232,6 +232,34 @@ def test_dropout_bias_head_adam():
     assert np.allclose(w.cpu().numpy(), ww, rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("N,H,W,Cin,Cout,off", [
+    (1, 1, 1, 16, 32, 0), (3, 5, 62, 32, 32, 0), (2, 9, 7, 96, 32, 1), (1, 13, 11, 64, 32, 0), (2, 6, 30, 48, 64, 0),
+    (2, 17, 9, 64, 64, 3), (1, 8, 129, 80, 96, 0), (4, 33, 31, 64, 128, 0), (2, 12, 10, 128, 160, 0),
+    (1, 31, 33, 16, 192, 0), (2, 7, 5, 192, 256, 0), (40, 64, 66, 32, 64, 0)])
+def test_wgrad_layouts_are_exact(N, H, W, Cin, Cout, off):
+    """Every way the weight gradient lays its taps out (output channels of 32,
+    64 and more, with ragged channel tiles; input channels in blocks of 32 and
+    64; row lengths of any parity; a dw off the 16-byte boundary) on small
+    integers, whose sums FP32 holds exactly: equal to the sums in 64 bits.
+    Added to what dw held."""
+    L = core()
+    gen = torch.Generator(device="cuda").manual_seed(Cin + Cout)
+    x = torch.randint(-2, 3, (N, H, W, Cin), generator=gen, device="cuda").double()
+    dy = torch.randint(-2, 3, (N, H, W, Cout), generator=gen, device="cuda").double()
+    border = lambda t: torch.nn.functional.pad(t, (0, 0, 1, 1, 1, 1))  # noqa: E731
+    xp = border(x)
+    want = torch.stack([torch.einsum("nhwo,nhwi->oi", dy, xp[:, k // 3:k // 3 + H, k % 3:k % 3 + W])
+                        for k in range(9)], 1)
+    xb, dyb = xp.to(torch.bfloat16).contiguous(), border(dy).to(torch.bfloat16).contiguous()
+    buf = torch.ones(Cout * 9 * Cin + 4, device="cuda")
+    dw = buf[off:off + Cout * 9 * Cin].view(Cout, 9, Cin)
+    assert L.fcab_unet_conv_wgrad(_p(dyb), _p(xb), N, H, W, Cin, Cout, _p(dw), None) == 0
+    torch.cuda.synchronize()
+    assert L.fcab_unet_device_error() == 0
+    assert torch.equal(dw.double(), want + 1)
+    assert bool((buf[:off] == 1).all() and (buf[off + dw.numel():] == 1).all())
+
+
 @pytest.mark.parametrize("C,P,p", [(32, 1, 0.0), (32, 70001, 0.1), (64, 4099, 0.5), (128, 515, 0.1),
                                    (256, 33, 0.0), (256, 2050, 0.25)])
 def test_act_bwd_equals_its_three_passes(C, P, p):
