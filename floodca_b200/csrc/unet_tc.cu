@@ -458,25 +458,32 @@ k_conv_gemm(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUte
 }
 
 // ---------------------------------------------------------------------------
-// Small-channel convolutions (16- or 32-channel K blocks): one halo'd A tile
-// per super-tile of MT x 128 pixels serves all nine taps. The tile holds the
-// rows p0 - Wp - 1 .. p0 + MT*128 + Wp of the activation matrix in the
-// unswizzled K-major layout: 8-channel planes of 16-byte rows, 8-row groups
-// 128 B apart (SBO) and planes `plane` bytes apart (LBO), i.e. plain linear
-// rows, so tap (ky, kx) of tile t is the same tile read from row
-// t*128 + ky*Wp + kx. Per 128 output pixels this loads (MT*128 + 2*Wp +
-// 2) / MT rows instead of 9 x 128. Weights stay resident (swizzled, as in
-// k_conv_gemm). Same warp roles as k_conv_gemm; TMEM holds two buffers of MT
-// accumulators, TCS columns each.
+// Convolutions whose halo'd A tile fits beside the resident weights: the one
+// tile of a super-tile of MT x 128 pixels serves all nine taps. It holds the
+// rows p0 - Wp - 1 .. p0 + MT*128 + Wp of the activation matrix, CK channels
+// each, K-major and swizzled as in k_conv_gemm; the swizzle follows the
+// shared-memory address, so tap (ky, kx) of tile t is the same tile read from
+// row t*128 + ky*Wp + kx on. Per 128 output pixels this loads (MT*128 + 2*Wp +
+// 2) / MT rows instead of 9 x 128. Weights stay resident. Same warp roles as
+// k_conv_gemm; TMEM holds two buffers of MT accumulators, TCS columns each.
+// The bound was the TMA unit, which takes a row of a box in about the same
+// time whether it has 16 bytes or 128: as planes of 8 channels (16-byte rows,
+// unswizzled) a 32-channel tile took four times the rows. Now it is the tensor
+// cores' reading of A, 64 cycles for 128 pixels x K = 16 whatever N is: 70 % of
+// the time at 32 to 32 channels. Measured, 32 images: 32 to 32 channels at 256
+// x 256 122 us with planes, 93 now; 64 to 64 at 128 x 128 98 us in k_conv_gemm,
+// 54 here; 64 to 128 at 64 x 64 33 and 23.
+
+constexpr int HALO_BOX = 32;
 
 struct HaloArgs {
     int P, Hp, Wp;          // padded pixel count, padded height and width
     int Cin, Cout;
     int nsup;               // super-tiles of MT x 128 pixels
     int nkb;                // channel blocks (Cin / CK)
-    int rows_alloc;         // rows per 8-channel plane (multiple of 128)
+    int boxes;              // boxes of HALO_BOX pixels in a halo tile
     int stages;             // ring stages (one halo tile per channel block)
-    int stage_bytes;        // (CK / 8) x rows_alloc x 16
+    int stage_bytes;        // at least boxes x HALO_BOX x CK x 2
     unsigned long long m_hw, m_w;   // ceil(2^48 / (Hp*Wp)), ceil(2^48 / Wp)
     const float *bias;      // [Cout] or null
     bf16 *y;                // [P][Cout]
@@ -485,7 +492,7 @@ struct HaloArgs {
 
 template <int CK, int BN, int MT>
 struct HaloCfg {
-    static constexpr int NPL = CK / 8;                      // planes per stage
+    static constexpr uint32_t ROW = 2u * CK;                // bytes of a pixel
     static constexpr int B_BYTES = BN * CK * 2;
     static constexpr int B_AL = (B_BYTES + 1023) / 1024 * 1024;
     static constexpr uint32_t TCS = BN <= 32 ? 32 : BN <= 64 ? 64 : 128;   // columns per tile
@@ -503,7 +510,6 @@ k_conv_halo(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUte
     const uint32_t base = (raw + 1023u) & ~1023u;
     uint8_t *sm = smem_raw + (base - raw);
     const int S = a.stages;
-    const uint32_t plane = (uint32_t)a.rows_alloc * 16u;
     const uint32_t bres_off = (uint32_t)(S * a.stage_bytes);
     const uint32_t bar_off = bres_off + (uint32_t)(9 * a.nkb * Cfg::B_AL);
     const uint32_t bar0 = base + bar_off;
@@ -540,7 +546,6 @@ k_conv_halo(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUte
     tc_fence_after();
     const uint32_t tmem = *tslot;
     const int nkb = a.nkb;
-    const int nbox = a.rows_alloc / 128;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -549,7 +554,7 @@ k_conv_halo(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUte
             for (int tap = 0; tap < 9; tap++)
                 for (int kb = 0; kb < nkb; kb++)
                     tma_load_2d(sB(tap * nkb + kb), &tw, bfull, tap * a.Cin + kb * CK, 0);
-            const uint32_t tx_bytes = (uint32_t)(Cfg::NPL * nbox * 128 * 16);
+            const uint32_t tx_bytes = (uint32_t)(a.boxes * HALO_BOX) * Cfg::ROW;
             int s = 0;
             uint32_t ph = 0;
             bool wrapped = false, bad = false;
@@ -562,10 +567,9 @@ k_conv_halo(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUte
                         break;
                     }
                     mbar_expect_tx(full(s), tx_bytes);
-                    for (int j = 0; j < Cfg::NPL; j++)
-                        for (int b = 0; b < nbox; b++)
-                            tma_load_2d(sA(s) + (uint32_t)j * plane + (uint32_t)b * 2048u, &tx,
-                                        full(s), kb * CK + 8 * j, r0 + 128 * b);
+                    for (int b = 0; b < a.boxes; b++)
+                        tma_load_2d(sA(s) + (uint32_t)(b * HALO_BOX) * Cfg::ROW, &tx, full(s), kb * CK,
+                                    r0 + HALO_BOX * b);
                     if (++s == S) {
                         s = 0;
                         ph ^= 1u;
@@ -599,18 +603,16 @@ k_conv_halo(const __grid_constant__ CUtensorMap tx, const __grid_constant__ CUte
                     const uint32_t st = sA(s);
                     for (int tap = 0; tap < 9; tap++) {
                         const int ky = tap >= 6 ? 2 : tap >= 3 ? 1 : 0;
-                        const uint32_t off = (uint32_t)(ky * a.Wp + (tap - 3 * ky)) * 16u;
+                        const uint32_t off = (uint32_t)(ky * a.Wp + (tap - 3 * ky)) * Cfg::ROW;
                         const uint32_t bb = sB(tap * nkb + kb);
+                        // consecutive MMAs go to different accumulators
 #pragma unroll
-                        for (int t = 0; t < MT; t++) {
-                            const uint32_t d = tmem + (uint32_t)((buf * MT + t) * Cfg::TCS);
+                        for (int kk = 0; kk < CK / 16; kk++) {
 #pragma unroll
-                            for (int kk = 0; kk < CK / 16; kk++) {
-                                // K = 16: planes 2kk (k 0-7) and 2kk+1 (k 8-15, LBO apart)
-                                const uint32_t aa = st + (uint32_t)(2 * kk) * plane +
-                                                    (uint32_t)(t * 128) * 16u + off;
-                                umma_bf16(d, smem_desc(aa, plane, 128u, 0u),
-                                          kdesc<CK>(bb + 32u * kk), idesc,
+                            for (int t = 0; t < MT; t++) {
+                                const uint32_t d = tmem + (uint32_t)((buf * MT + t) * Cfg::TCS);
+                                const uint32_t aa = st + (uint32_t)(t * 128) * Cfg::ROW + off + 32u * kk;
+                                umma_bf16(d, kdesc<CK>(aa), kdesc<CK>(bb + 32u * kk), idesc,
                                           (kb | tap | kk) != 0 ? 1u : 0u);
                             }
                         }
@@ -1431,8 +1433,8 @@ cudaError_t launch_halo(const CUtensorMap &txh, const CUtensorMap &tw, const Hal
     return cudaGetLastError();
 }
 
-// The halo path for 16/32-channel K blocks and one output tile of at most
-// 128 channels, when its tiles fit in shared memory. Returns
+// The halo path for 16/32-channel K blocks, or 64 input channels, and one
+// output tile of at most 128 channels, when its tiles fit in shared memory. Returns
 // cudaErrorNotSupported when the shape does not qualify (the caller then
 // uses k_conv_gemm).
 template <int CK>
@@ -1441,24 +1443,31 @@ cudaError_t try_halo(const void *x, const CUtensorMap &tw, int N, int H, int W, 
 {
     if (Cout > 128)
         return cudaErrorNotSupported;
-    const int MT = Cout <= 64 ? 4 : 2;
+    // 64 channels leave room for smaller super-tiles
+    const int MT = (Cout <= 64 ? 4 : 2) / (CK == 64 ? 2 : 1);
     const long long P = (long long)N * (H + 2) * (W + 2);
+    // up to one GEMM tile per SM, super-tiles of two are the longer chain
+    // (64 to 64, 32 x 32: 9.6 us there, 10.9 here; two images of 128 x 128:
+    // 12.9 and 10.8)
+    if (CK == 64 && MT > 1 && P <= 148 * 128)
+        return cudaErrorNotSupported;
     const int Wp = W + 2;
     const int rows = MT * 128 + 2 * Wp + 2;
-    const int rows_alloc = (rows + 127) / 128 * 128;
-    if (rows_alloc * 16 >= (1 << 18))          // LBO field limit
-        return cudaErrorNotSupported;
+    const int pad = CK == 64 ? HALO_BOX : 128;
     const int nkb = Cin / CK;
     const int bn_al = (Cout * CK * 2 + 1023) / 1024 * 1024;
     const int bres = 9 * nkb * bn_al;
-    const int stage = (CK / 8) * rows_alloc * 16;
+    const int stage = (rows + pad - 1) / pad * pad * 2 * CK;
     const int fixed = 1024 + bres + 64 + 4 * Cout;
     int stages = (SMEM_MAX - fixed) / (stage + 16);
     stages = stages > 4 ? 4 : stages;
     if (stages < 2)
         return cudaErrorNotSupported;
     CUtensorMap txh;
-    if (!make_map(&txh, x, P, Cin, 8, 128, CU_TENSOR_MAP_SWIZZLE_NONE))
+    if (!make_map(&txh, x, P, Cin, CK, HALO_BOX,
+                  CK == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+                  : CK == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                             : CU_TENSOR_MAP_SWIZZLE_32B))
         return cudaErrorInvalidValue;
     HaloArgs a;
     a.P = (int)P;
@@ -1468,7 +1477,7 @@ cudaError_t try_halo(const void *x, const CUtensorMap &tw, int N, int H, int W, 
     a.Cout = Cout;
     a.nsup = (int)((P + MT * 128 - 1) / (MT * 128));
     a.nkb = nkb;
-    a.rows_alloc = rows_alloc;
+    a.boxes = (rows + HALO_BOX - 1) / HALO_BOX;
     a.stages = stages;
     a.stage_bytes = stage;
     a.m_hw = ((1ull << 48) + (unsigned long long)(a.Hp * a.Wp) - 1) / (unsigned long long)(a.Hp * a.Wp);
@@ -1477,11 +1486,12 @@ cudaError_t try_halo(const void *x, const CUtensorMap &tw, int N, int H, int W, 
     a.y = (bf16 *)y;
     a.relu = relu;
     const int smem = fixed + stages * (stage + 16);
+    constexpr int M4 = CK == 64 ? 2 : 4, M2 = M4 / 2;
     switch (Cout) {
-    case 32: return launch_halo<CK, 32, 4>(txh, tw, a, smem, st);
-    case 64: return launch_halo<CK, 64, 4>(txh, tw, a, smem, st);
-    case 96: return launch_halo<CK, 96, 2>(txh, tw, a, smem, st);
-    case 128: return launch_halo<CK, 128, 2>(txh, tw, a, smem, st);
+    case 32: return launch_halo<CK, 32, M4>(txh, tw, a, smem, st);
+    case 64: return launch_halo<CK, 64, M4>(txh, tw, a, smem, st);
+    case 96: return launch_halo<CK, 96, M2>(txh, tw, a, smem, st);
+    case 128: return launch_halo<CK, 128, M2>(txh, tw, a, smem, st);
     default: return cudaErrorNotSupported;
     }
 }
@@ -1507,9 +1517,10 @@ int conv_gemm(const void *x, int N, int H, int W, int Cin, const void *w, int Co
     CUtensorMap tx, tw;
     if (!make_map(&tx, x, P, Cin, CK, 128, sw) || !make_map(&tw, w, Cout, 9 * Cin, CK, bn, sw))
         return fail(FCAB_ERR_CUDA, "conv: tensor map encoding failed");
-    if (CK <= 32 && bn == Cout) {
-        const cudaError_t he = CK == 32 ? try_halo<32>(x, tw, N, H, W, Cin, Cout, bias, relu, y, st)
-                                        : try_halo<16>(x, tw, N, H, W, Cin, Cout, bias, relu, y, st);
+    if ((CK <= 32 || Cin == 64) && bn == Cout) {
+        const cudaError_t he = CK == 64   ? try_halo<64>(x, tw, N, H, W, Cin, Cout, bias, relu, y, st)
+                               : CK == 32 ? try_halo<32>(x, tw, N, H, W, Cin, Cout, bias, relu, y, st)
+                                          : try_halo<16>(x, tw, N, H, W, Cin, Cout, bias, relu, y, st);
         if (he == cudaSuccess)
             return 0;
         if (he != cudaErrorNotSupported)

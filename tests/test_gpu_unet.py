@@ -232,6 +232,34 @@ def test_dropout_bias_head_adam():
     assert np.allclose(w.cpu().numpy(), ww, rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("N,H,W,Cin,Cout", [
+    (1, 146, 128, 64, 32), (1, 146, 126, 64, 64), (3, 79, 81, 64, 64), (7, 50, 53, 64, 32), (2, 90, 260, 64, 64),
+    (1, 1, 1, 64, 96), (2, 9, 77, 64, 128), (1, 5, 78, 64, 128), (3, 30, 31, 64, 96), (2, 40, 300, 32, 32),
+    (1, 3, 430, 32, 32), (2, 33, 35, 96, 32), (1, 11, 200, 16, 128)])
+def test_conv_halo_tiles_are_exact(N, H, W, Cin, Cout):
+    """Convolutions over one halo tile for all taps: sizes on both sides of the
+    rules that choose it, of every parity and off the tile's multiples, on small
+    integers whose sums bf16 holds exactly (|sum| <= 256): equal to the sums in
+    64 bits, the border zero."""
+    L = core()
+    gen = torch.Generator(device="cuda").manual_seed(Cin + Cout + W)
+    pick = lambda *s: (torch.randint(-1, 2, s, generator=gen, device="cuda")  # noqa: E731
+                       * (torch.rand(s, generator=gen, device="cuda") < 0.2)).double()
+    x, w = pick(N, H, W, Cin), pick(Cout, 9, Cin)
+    b = torch.randint(-3, 4, (Cout,), generator=gen, device="cuda").float()
+    pad = lambda t: torch.nn.functional.pad(t, (0, 0, 1, 1, 1, 1))  # noqa: E731
+    xp = pad(x)
+    want = b.double() + sum(xp[:, k // 3:k // 3 + H, k % 3:k % 3 + W] @ w[:, k].T for k in range(9))
+    assert float(want.abs().max()) <= 256
+    xb, wb = xp.to(torch.bfloat16).contiguous(), w.to(torch.bfloat16).contiguous()
+    for relu in (0, 1):
+        y = torch.zeros((N, H + 2, W + 2, Cout), dtype=torch.bfloat16, device="cuda")
+        assert L.fcab_unet_conv_fwd(_p(xb), N, H, W, Cin, _p(wb), Cout, _p(b), relu, _p(y), None) == 0
+        torch.cuda.synchronize()
+        assert L.fcab_unet_device_error() == 0
+        assert torch.equal(y.double(), pad(want.clamp_min(0) if relu else want))
+
+
 @pytest.mark.parametrize("N,H,W,Cin,Cout,off", [
     (1, 1, 1, 16, 32, 0), (3, 5, 62, 32, 32, 0), (2, 9, 7, 96, 32, 1), (1, 13, 11, 64, 32, 0), (2, 6, 30, 48, 64, 0),
     (2, 17, 9, 64, 64, 3), (1, 8, 129, 80, 96, 0), (4, 33, 31, 64, 128, 0), (2, 12, 10, 128, 160, 0),
