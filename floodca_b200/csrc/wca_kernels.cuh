@@ -1253,7 +1253,7 @@ constexpr int VPASS_GRID = 148 * 8;
 // ---- the last CTA to finish prepares the next step
 template <typename T, int K, int MATH>
 __device__ __forceinline__ void step_tail(const GridD<T> &g, const RunK<T> &rk, const TimeCfg &tc,
-                                          Ctl *ctl)
+                                          Ctl *ctl, const TimePre &pre)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1268,7 +1268,7 @@ __device__ __forceinline__ void step_tail(const GridD<T> &g, const RunK<T> &rk, 
                 ctl->fin_pending = 1;
                 ctl->ctas_done = 0u;
             } else {
-                finalize<T>(ctl, tc, rk, true);
+                finalize<T>(ctl, tc, rk, true, pre);
                 // a missed seed defers this step's dt to the full velocity
                 // pass: launched from here into the tail of the stream, so
                 // it runs before the next step and only when needed
@@ -1487,27 +1487,59 @@ __global__ void __launch_bounds__(step_threads<CPL, MATH>(),
     if (ctl->active == 0)
         return;
     const int lane = threadIdx.x & 31;
-    const int wid = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    // A block's warps, and the blocks of an SM, take ranges far apart: where the
+    // water is, ranges cost several times a dry one's, and neighbours are alike.
+    const int wid = (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
     const StepVals<T> sv = step_vals<T, K>(g, rk, ctl);
+    __shared__ TimePre pre;
+    if (threadIdx.x == blockDim.x - 32)
+        pre = time_pre(ctl, tc, true);
+    __syncwarp();
     StepSums<T, AccT> ss;
 
+    // Rows of a strip cost 6 more at each range's start. A strip cut into equal
+    // ranges, or, where that leaves a longer chain (few warps a strip), one even
+    // split of all rows, whose ranges may lie in two strips (12 more). FP64,
+    // us a step with the even split and with ranges: 511 x 770 80 and 74 (85
+    // with neighbouring ranges in a block), 256 x 256 46 and 41, 16 x 16 39 and
+    // 31, 1000 x 1024 114 and 113. The bound is a row's chain of about 1500
+    // FP64 instructions a warp, not their rate: issue slots are half used.
     const int nr = g.nr, nc = g.nc;
     const int nstrips = (nc + G::OW - 1) / G::OW;
     const long long total = (long long)nstrips * nr;
-    long long w0 = total * wid / warps_total, w1 = total * (wid + 1) / warps_total;
+    const int segs = max(1, min(nr, warps_total / nstrips));
+    const bool even = (total + warps_total - 1) / warps_total + 6 <
+                      (long long)((nr + segs - 1) / segs) * ((nstrips * (long long)segs + warps_total - 1) / warps_total);
+    // positions w0 .. w1 of the strips laid end to end; by ranges, the next of a
+    // warp is warps_total on
+    long long u = wid, w0, w1;
+    const auto range = [&]() {
+        if (even) {
+            w0 = total * u / warps_total;
+            w1 = total * (u + 1) / warps_total;
+        } else {
+            const long long strip = u / segs;
+            const int q = (int)(u - strip * segs);
+            w0 = strip * nr + (long long)nr * q / segs;
+            w1 = strip * nr + (long long)nr * (q + 1) / segs;
+        }
+    };
+    const long long units = even ? warps_total : (long long)nstrips * segs;
     if (wid >= warps_total)
-        w0 = w1 = 0;
-
-    while (w0 < w1) {
-        const int strip = (int)(w0 / nr);
-        const int r0 = (int)(w0 % nr);
-        const int r1 = (int)min((long long)nr, (long long)r0 + (w1 - w0));
-        w0 += r1 - r0;
-        sweep_segment<T, AccT, K, CPL, MATH, RAINF, LANDONLY>(g, rk, sv, strip, r0, r1, lane, ss);
+        u = units;
+    for (; u < units; u += warps_total) {
+        range();
+        while (w0 < w1) {
+            const int strip = (int)(w0 / nr);
+            const int r0 = (int)(w0 % nr);
+            const int r1 = (int)min((long long)nr, (long long)r0 + (w1 - w0));
+            w0 += r1 - r0;
+            sweep_segment<T, AccT, K, CPL, MATH, RAINF, LANDONLY>(g, rk, sv, strip, r0, r1, lane, ss);
+        }
     }
 
     publish_sums<T, AccT, RAINF>(ss, sv, ctl, lane, wid & (NSLOT - 1));
-    step_tail<T, K, MATH>(g, rk, tc, ctl);
+    step_tail<T, K, MATH>(g, rk, tc, ctl, pre);
 }
 
 // --------------------------------------------------------------------------

@@ -344,14 +344,28 @@ long long fcab::step_warps(const FcabConfig &c, int cpl, int nsm, int per_sm, in
     const long long strips = (c.ncols + ow - 1) / ow;
     const long long total = strips * c.nrows;
     const long long max_warps = (long long)nsm * (per_sm > 0 ? per_sm : 1) * wpb;
-    // rows per warp: enough warps to fill the resident slots, but at least 4
-    // rows per warp (each warp's segment costs 6 extra pipeline rows)
-    long long seg = c.seg_rows > 0 ? c.seg_rows : total / max_warps;
-    if (seg < 4)
-        seg = 4;
-    const long long want = (total + seg - 1) / seg;
-    const long long warps = want < max_warps ? want : max_warps;
-    return warps < 1 ? 1 : warps;
+    if (c.seg_rows > 0) {
+        const long long want = (total + c.seg_rows - 1) / c.seg_rows;
+        const long long warps = want < max_warps ? want : max_warps;
+        return warps < 1 ? 1 : warps;
+    }
+    if (strips >= max_warps)
+        return max_warps;
+    // Ranges per strip: a range of n rows is a chain of n + 6, each of which
+    // takes longer the more warps share a scheduler (FP64: 5.7 cycles an
+    // instruction alone, 7.7 with three others).
+    long long best = 1;
+    double best_cost = 1e300;
+    for (long long segs = 1; segs * strips <= max_warps && segs <= c.nrows; segs++) {
+        const long long per = (segs * strips + 4 * nsm - 1) / (4 * nsm);
+        const double cost = (double)((c.nrows + segs - 1) / segs + 6) * (5.1 + 0.65 * (double)per);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = segs;
+        }
+    }
+    // a strip of many rows: all warps, split evenly
+    return total / max_warps >= 32 ? max_warps : best * strips;
 }
 
 int fcab::blk_seg(const FcabConfig &c, int nsm, int per_sm)

@@ -119,3 +119,24 @@ def test_block_sweep_coast(size, K, rain_field):
     _check(dom, RunParams(K=K, steps=12, T_sim=1e6, boundary="closed",
                           inflow_cell=int(np.flatnonzero(dom.mask.ravel() == 0)[5]),
                           inflow_peak=50.0, inflow_t_peak=100.0, inflow_t_end=900.0))
+
+
+SCALAR = [(1, 1, 0), (3, 27, 0), (16, 16, 0), (37, 53, 5), (130, 59, 0), (67, 300, 17), (511, 130, 0),
+          (4, 63000, 0), (90, 31300, 0), (2600, 700, 0)]
+
+
+@pytest.mark.parametrize("nr,nc,seg", SCALAR)
+def test_row_sweep_ranges(nr, nc, seg):
+    """The row sweep (one column to a lane; FP64's) at every way its rows are
+    cut: ranges of one row, more strips than warps, an even split of long
+    strips, cuts asked for. FP32 equals the oracle bit for bit; FP64 depths,
+    each cell's own arithmetic, are the same however the rows are cut."""
+    steps = 20 if nr * nc < 200000 else 4
+    p = RunParams(steps=steps, T_sim=1e6, edges=(0, 1, 0, 1))
+    _check(_grid(nr, nc, nr + nc, True), p, seg_rows=seg, cols_per_lane=1)
+    dom = _grid(nr, nc, nr + 2 * nc, False)
+    a = run_session(dom, p, precision="f64", seg_rows=seg)
+    b = run_session(dom, p, precision="f64", seg_rows=nr)
+    assert a["t"] == b["t"]
+    for k in ("h", "hmax", "tmax"):
+        assert np.array_equal(a[k], b[k], equal_nan=True), k
