@@ -31,7 +31,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # parity build does on the host (-ffp-contract=off); explicit fmaf() calls
 # in the kernels are unaffected. It does not stop ptxas from fusing a packed
 # mul.rn.f32x2 into a following add.rn.f32x2 (nor does ptxas's own
-# --fmad=false); the pair sweep forms such products with scalar mul.rn.
+# --fmad=false); the block sweep forms such products with scalar mul.rn.
 NVFLAGS = ["-std=c++17", "-O3", "-lineinfo", "--fmad=false",
            "-Xcompiler", "-fPIC",
            "-Xcompiler", "-fvisibility=hidden", "-I", str(INCLUDE), "-I", str(CSRC),

@@ -37,8 +37,8 @@
 
 namespace fcab {
 
-constexpr int PADR = 8;   // padded rows above and below the grid (the pair sweep
-                          // starts up to six rows above a segment)
+constexpr int PADR = 8;   // padded rows above and below the grid (a range of
+                          // rows starts up to six rows above its first)
 constexpr int PADC = 4;   // padded columns left of the grid
 constexpr int NSLOT = 32; // accumulator slots (spread the atomics)
 constexpr double PAD_Z = 1e30;   // padding elevation of all-LAND grids
@@ -61,8 +61,8 @@ struct GridD {
     long long pitch;
     int nr, nc;
     int r_lo, r_hi;             // rows of real cells: [0, nr), or with a slab's halo rows
-    // row-tile tensor maps of z, n, h0, h1 (device memory) for the TMA row
-    // source of the FP32 pair sweep, or nullptr (plain loads)
+    // tile tensor maps of z, n, h0, h1, hmax (device memory) for the block
+    // sweep, or nullptr
     const CUtensorMap *tmap = nullptr;
 };
 

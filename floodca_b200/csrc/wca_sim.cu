@@ -1486,13 +1486,13 @@ __global__ void k_math_probe(int which, const float *x, const float *y, float *o
         else if (which == 8)
             r = __fsqrt_rn(x[i]);
         else if (which == 10) {
-            // the pair sweep's cube root: its value where it decides the
+            // the block sweep's cube root: its value where it decides the
             // rounding itself, NaN where it defers to the exact evaluation
             bool u0, u1;
             const f2 c = cbrt_sq2(mk2(x[i], x[i]), u0, u1);
             r = u0 ? __int_as_float(0x7fc00000) : lo2(c);
         } else if (which == 11) {
-            // the pair sweep's product then packed sum: two roundings,
+            // the block sweep's product then packed sum: two roundings,
             // RN(RN(x*y) + g)
             r = lo2(add2(mul2_sep(mk2(x[i], x[i]), mk2(y[i], y[i])), bc2(g)));
         } else

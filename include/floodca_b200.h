@@ -186,10 +186,9 @@ typedef struct FcabConfig {
     double inflow_peak;       /* triangular hydrograph: 0 at t=0, peak (m^3/s) at */
     double inflow_t_peak;     /*   inflow_t_peak, 0 at inflow_t_end; added after  */
     double inflow_t_end;      /*   the clamp, before hmax                         */
-    int cols_per_lane;        /* 0 = autotuned (1 or 2); else 1, 2 or 4 (FP32 all-LAND
-                                 grids: 2 runs the packed pair sweep, 4 with K = 4 two
-                                 pairs per lane; padded fields beyond 2^31 elements run 1) */
-    int seg_rows;             /* 0 = autotuned; rows per warp segment */
+    int cols_per_lane;        /* 0, 2 or 4: FP32 runs the block sweep; 1: the row sweep, one
+                                 column to a lane (what padded fields beyond 2^31 elements run) */
+    int seg_rows;             /* 0 = chosen; rows of a unit (block sweep) or of a warp's range */
 } FcabConfig;
 
 typedef struct FcabStats {
@@ -220,7 +219,7 @@ typedef struct FcabPoll {
 typedef struct FcabInfo {
     int cols_per_lane, grid, warps, ctas_per_sm, rain_field, land_only;
     long long land_cells, faces_per_step, pitch;
-    int tma_rows;             /* 1: the pair sweep reads rows by TMA (FCAB_ROW_SOURCE=tma) */
+    int tma_rows;             /* 1: rows come by TMA (the block sweep) */
 } FcabInfo;
 
 typedef struct FcabSim FcabSim;
@@ -417,8 +416,8 @@ FCAB_API int fcab_run_noalloc(const FcabConfig *cfg, const float *z, const float
  * hf^(2/3); 1: min(x, RN(sqrt(g*y))); 2: the fast-mode hf^(2/3); 4/5/6: the
  * branch-free reciprocal, square root and Markstein quotient x/y; 7/8/9: the
  * IEEE reciprocal, square root and quotient they must equal; 10: the packed
- * pair sweep's hf^(2/3), NaN where it defers to the exact evaluation; 11: the
- * pair sweep's product then packed sum, RN(RN(x*y) + g), rounded twice. */
+ * block sweep's hf^(2/3), NaN where it defers to the exact evaluation; 11: the
+ * block sweep's product then packed sum, RN(RN(x*y) + g), rounded twice. */
 FCAB_API int fcab_math_probe(int which, const float *x, const float *y, float *out, long long n,
                              float g);
 
