@@ -52,12 +52,13 @@ constexpr int BLK_THREADS = 32 * BLK_ROWS;
 constexpr int BLK_STAGES = 3;               // tile stages: the pass at work and those ahead
 constexpr uint32_t BLK_ROW_B = 256;         // bytes of a strip row
 // Cells up to which the step's last CTA does a missed seed's velocity pass
-// alone: it reads the depths (4 B a cell, about 100 us for 2^20 cells) and
-// evaluates the few cells deep enough to matter. One step in a hundred needs
-// it; a kernel that could launch the pass costs 1.3 us more to launch every
-// step, cannot overlap its start with the step before, and its graph takes 4
-// ms more to build and free.
-constexpr long long BLK_SOLO = 1ll << 20;
+// alone: it reads the depths and evaluates the cells deep enough to matter, a
+// few as a rule, but all wet ones after a sharp fall of the maximum: 10 ns a
+// cell (3809 x 132 masked with a point inflow, two such passes in 169 steps:
+// 15.5 ms a run with a limit of 2^20 cells, 5.6 with the pass launched). One
+// step in a hundred needs it; a kernel that could launch the pass costs 1.3 us
+// more to launch every step and cannot overlap its start with the step before.
+constexpr long long BLK_SOLO = 1ll << 16;
 
 // Shared memory, in bytes from a 128-byte boundary. Tile stage: rows
 // first-2 .. first+7 of z, h, n and rows first-2 .. first+5 of hmax, so that a

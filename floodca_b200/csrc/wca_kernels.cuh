@@ -1335,7 +1335,7 @@ __device__ __forceinline__ T velocity_at(const GridD<T> &g, const RunK<T> &rk, c
 // instead of launching it, and a step starts while the one before it ends:
 // its barriers are set up and its first tiles of z and n on their way before
 // it waits for that one. Measured, us a step: 61 x 93 14.5 -> 9.0, 256^2
-// 18.2 -> 11.1, 512^2 19.3 -> 14.3, 1024^2 27.8 -> 25.2.
+// 18.2 -> 11.1.
 template <typename AccT, int K, int MATH, bool RAINF, bool GEN, bool TAILV>
 __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
     k_step_blk(GridD<float> g, RunK<float> rk, TimeCfg tc, Ctl *ctl, int seg)
