@@ -415,12 +415,14 @@ __device__ __forceinline__ void open_sides(int r, int c, int nr, int nc, int r_l
              : 0;
 }
 
-// Cells that are not LAND: elevation and level of SEA cells (z = -PAD_Z) are
+// Cells that are not LAND (n NaN; a LAND cell may have any finite elevation,
+// a raster's -3.4e38 too): elevation and level of SEA cells (z = -PAD_Z) are
 // the sea level, the level of WALL cells their elevation PAD_Z.
 __device__ __forceinline__ void sea_levels(f2 &z, f2 &L, f2 n, float zs)
 {
-    z = sel2(lo2(z) < -1e29f, hi2(z) < -1e29f, bc2(zs), z);
-    L = sel2(lo2(n) != lo2(n), hi2(n) != hi2(n), z, L);
+    const bool o0 = lo2(n) != lo2(n), o1 = hi2(n) != hi2(n);
+    z = sel2(o0 && lo2(z) < -1e29f, o1 && hi2(z) < -1e29f, bc2(zs), z);
+    L = sel2(o0, o1, z, L);
 }
 // Sum of two cells' Manning n for their mean; a cell that is not LAND (NaN)
 // takes the other's.
@@ -965,8 +967,9 @@ struct BlockSweep {
                         const f2 z = sld(tb + BLK_Z);
                         const int cbase = column();
                         const bool own = own2 && out_lane;
-                        const bool sea0 = own && lo2(z) < -1e29f && cbase >= 0 && cbase < nc;
-                        const bool sea1 = own && hi2(z) < -1e29f && cbase + 1 >= 0 &&
+                        const bool sea0 = own && !l0 && lo2(z) < -1e29f && cbase >= 0 &&
+                                          cbase < nc;
+                        const bool sea1 = own && !l1 && hi2(z) < -1e29f && cbase + 1 >= 0 &&
                                           cbase + 1 < nc;
                         AccT sea = 0;
                         const float dt = FCAB_SV(dt);

@@ -121,6 +121,19 @@ def test_block_sweep_coast(size, K, rain_field):
                           inflow_peak=50.0, inflow_t_peak=100.0, inflow_t_end=900.0))
 
 
+@pytest.mark.parametrize("K", [4, 8])
+@pytest.mark.parametrize("zz", [-9e28, -1e30, -3.4028235e38, 3e29])
+def test_block_sweep_coast_extreme_land_elevations(zz, K):
+    """LAND cells with a raster's nodata as elevation, in rows with SEA and
+    WALL cells and beside both: only the mask says which cells are SEA."""
+    dom = _grid(40, 70, 3, False, h0=0.5)
+    dom.mask[10:12, 20:24] = 1
+    dom.mask[20, 30:40] = 2
+    for r, c in ((11, 24), (12, 21), (11, 40), (20, 40), (20, 43), (30, 60)):
+        dom.z[r, c] = np.float32(zz)
+    _check(dom, RunParams(K=K, steps=20, T_sim=1e6, edges=(1, 0, 0, 0)))
+
+
 SCALAR = [(1, 1, 0), (3, 27, 0), (16, 16, 0), (37, 53, 5), (130, 59, 0), (67, 300, 17), (511, 130, 0),
           (4, 63000, 0), (90, 31300, 0), (2600, 700, 0)]
 
