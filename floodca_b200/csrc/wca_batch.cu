@@ -25,7 +25,8 @@ __global__ void k_gather_active(const MemberD<float> *members, int n, int *flags
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m < n) {
         const Ctl *c = members[m].ctl;
-        flags[m] = c->active ? 1 : (c->done ? 0 : 2);   // 1 running, 2 paused, 0 done
+        // 1 running, 2 paused, 0 done; 3 a step of it left an error
+        flags[m] = c->err ? 3 : c->active ? 1 : (c->done ? 0 : 2);
     }
 }
 
@@ -347,7 +348,8 @@ static int window_graph(FcabBatch *b, int steps, double window_s)
     return 0;
 }
 
-// Members running / paused at a window end, and the window loop's passes.
+// Members running / paused at a window end, and the window loop's passes; an
+// error if a step of a member left one.
 static int poll_members(FcabBatch *b, int *running, int *paused, unsigned long long *passes)
 {
     k_gather_active<<<(b->n + 127) / 128, 128, 0, b->stream>>>(b->d_members, b->n, b->d_flags);
@@ -365,6 +367,12 @@ static int poll_members(FcabBatch *b, int *running, int *paused, unsigned long l
         return bfail(FCAB_ERR_CUDA, cudaGetErrorString(e));
     *running = *paused = 0;
     for (int i = 0; i < b->n; i++) {
+        if (b->h_flags[i] == 3) {
+            char msg[96];
+            snprintf(msg, sizeof(msg),
+                     "batch member %d: a row tile of a step did not arrive: its depths are not valid", i);
+            return bfail(FCAB_ERR_CUDA, msg);
+        }
         *running += b->h_flags[i] == 1;
         *paused += b->h_flags[i] == 2;
     }

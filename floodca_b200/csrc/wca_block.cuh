@@ -721,7 +721,7 @@ struct BlockSweep {
             if (t.sv.want_v && t.vmax)
                 atomicMax(&ctl->vmax_bits, (unsigned long long)t.vmax);
             if (t.bad)
-                ctl->err = 3;       // a row tile never arrived; the host reports it
+                ctl->err = CTL_LOST_TILE;
         }
     }
 

@@ -87,7 +87,7 @@ struct Ctl {
     // prepared for the next step by the previous step's last CTA
     double t, dt, F, tmax_val, inflow_dh, t_next, dt_base;
     int step, hit, active, h_cur, want_v, done, pause, force_day;
-    int err, n_force_days;
+    int n_force_days;
     int fin_pending;            // slab runs: 1 after a step, 2 after the first velocity pass
     int inflow_off;             // 1: the inflow cell is not LAND (no inflow volume)
     long long dt_min_hits;
@@ -107,7 +107,9 @@ struct Ctl {
     double accd[4][NSLOT];      // V_rain, clamp, V_sea, V_bnd (double accumulation)
     float accf[4][NSLOT];       // same, FP32 accumulation
     unsigned long long cap[NSLOT];
+    int err;                    // CTL_*: what the host has to report; cleared by an upload
 };
+constexpr int CTL_LOST_TILE = 3;    // a row tile did not arrive within its wait's limit
 
 // Event and forcing parameters for the device-side step control.
 struct TimeCfg {
@@ -1275,8 +1277,8 @@ __device__ __forceinline__ void step_tail(const GridD<T> &g, const RunK<T> &rk, 
                 if (tc.tail_vpass && ctl->need_v) {
                     k_init_dt<T, K, MATH><<<VPASS_GRID, 256, 0, cudaStreamTailLaunch>>>(g, rk, tc,
                                                                                       ctl, 1);
-                    if (cudaGetLastError() != cudaSuccess)
-                        ctl->err = 2;   // the host's poll runs the pass instead
+                    // where that fails need_v stays set and the host's poll runs the pass
+                    (void)cudaGetLastError();
                 }
             }
         }
@@ -1425,8 +1427,7 @@ __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
                     if constexpr (TAILV) {
                         k_init_dt<float, K, MATH>
                             <<<VPASS_GRID, 256, 0, cudaStreamTailLaunch>>>(g, rk, tc, ctl, 1);
-                        if (cudaGetLastError() != cudaSuccess)
-                            ctl->err = 2;   // the host's poll runs the pass instead
+                        (void)cudaGetLastError();   // as in step_tail
                     } else {
                         solo = 1;
                         T.tail()->vmax = vbits;

@@ -733,6 +733,7 @@ static int upload_common(FcabSim *s, const void *z, const void *h, const void *n
         s->rkf.has_sea = has_sea;
     }
     s->tc.inflow_ok = inflow_ok;
+    CUDA_TRY(cudaMemsetAsync(&s->ctl->err, 0, sizeof(int), s->stream));
     s->uploaded = true;
     s->h_cur_host = 0;
     return fcab_sim_reset_time(s, 0.0, 0, 0.0, -1);
@@ -897,7 +898,8 @@ extern "C" int fcab_sim_reset_time(FcabSim *s, double t, int step, double dt_bas
     c.force_day = force_day;
     c.h_cur = s->h_cur_host;
     s->step0 = step;
-    CUDA_TRY(cudaMemcpyAsync(s->ctl, &c, sizeof(Ctl), cudaMemcpyHostToDevice, s->stream));
+    // all but err, which stands until the fields are uploaded again
+    CUDA_TRY(cudaMemcpyAsync(s->ctl, &c, offsetof(Ctl, err), cudaMemcpyHostToDevice, s->stream));
     // V0 = LAND volume of the current depth
     double *vol = (double *)s->scratch;
     CUDA_TRY(cudaMemsetAsync(vol, 0, sizeof(double), s->stream));
@@ -967,6 +969,15 @@ extern "C" int fcab_sim_advance(FcabSim *s, int nsteps)
     return 0;
 }
 
+// The error a step left in the control block: the depths are not those of the
+// run, so everything that reads its state fails.
+static int step_error(int err)
+{
+    if (err == CTL_LOST_TILE)
+        return fail(FCAB_ERR_CUDA, "a row tile of a step did not arrive: the depths are not valid");
+    return 0;
+}
+
 // Runs the guarded full velocity pass from the host (it does nothing unless
 // a step left its dt deferred).
 static int settle_deferred_dt(FcabSim *s)
@@ -1009,7 +1020,7 @@ extern "C" int fcab_sim_poll(FcabSim *s, FcabPoll *p)
     p->pause = c->pause;
     p->force_day = c->force_day;
     s->h_cur_host = c->h_cur;
-    return 0;
+    return step_error(c->err);
 }
 
 extern "C" int fcab_sim_resume(FcabSim *s, int force_day)
@@ -1100,7 +1111,7 @@ extern "C" int fcab_sim_stats(FcabSim *s, FcabStats *st)
                       st->clamp_err) /
                  den;
     s->h_cur_host = c->h_cur;
-    return 0;
+    return step_error(c->err);
 }
 
 extern "C" int fcab_sim_download(FcabSim *s, void *h, void *hmax, void *tmax)
@@ -1109,6 +1120,8 @@ extern "C" int fcab_sim_download(FcabSim *s, void *h, void *hmax, void *tmax)
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     const Ctl *c = (const Ctl *)s->ctl_host;
     s->h_cur_host = c->h_cur;
+    if (int rc = step_error(c->err))
+        return rc;
     fcab::RowCopy f[3];
     int nf = 0;
     auto own_rows = [&](void *dst, void *src) {
@@ -1239,6 +1252,7 @@ extern "C" int fcab_sim_upload_state(FcabSim *s, const void *h, const void *hmax
     if (tmax)
         f[nf++] = whole_field(s, s->tmax, tmax, s->esize);
     CUDA_TRY(put_fields(s, f, nf, cudaMemcpyHostToDevice));
+    CUDA_TRY(cudaMemsetAsync(&s->ctl->err, 0, sizeof(int), s->stream));
     if (!hmax || hmax == h)     // the padding of both is zeros
         CUDA_TRY(cudaMemcpyAsync(s->hmax, s->h0, s->nelem * s->esize, cudaMemcpyDeviceToDevice,
                                  s->stream));
@@ -1315,13 +1329,27 @@ extern "C" int fcab_sim_count_flooded(FcabSim *s, int nthr, const double *thr, u
     CUDA_TRY(cudaGetLastError());
     s->launches += 1;
     unsigned long long h[5];
+    int err = 0;
     CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
+    CUDA_TRY(cudaMemcpyAsync(&err, &s->ctl->err, sizeof(err), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
+    if (int rc = step_error(err))
+        return rc;
     for (int j = 0; j < nthr; j++)
         flooded[j] = (long long)h[j];
     double mx;
     memcpy(&mx, &h[4], sizeof(double));
     *max_depth = mx;
+    return 0;
+}
+
+extern "C" int fcab_sim_lost_tile_probe(FcabSim *s)
+{
+    if (!s->inited)
+        return fail(FCAB_ERR_STATE, "lost_tile_probe before upload");
+    const int err = CTL_LOST_TILE;
+    CUDA_TRY(cudaMemcpyAsync(&s->ctl->err, &err, sizeof(err), cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
     return 0;
 }
 

@@ -267,7 +267,11 @@ FCAB_API int fcab_sim_run(FcabSim *s);
  * fcab_sim_upload calls it with zeros. */
 FCAB_API int fcab_sim_reset_time(FcabSim *s, double t, int step, double dt_base, int force_day);
 
-/* Waits for the queued steps and reads the device step control. */
+/* Waits for the queued steps and reads the device step control. Returns
+ * FCAB_ERR_CUDA, as do run, stats, download, count_flooded, layout and
+ * fcab_batch_run, once a row tile of a step has not arrived within the step's
+ * bounded wait: the depths are then not those of the run, until the fields
+ * are uploaded again. */
 FCAB_API int fcab_sim_poll(FcabSim *s, FcabPoll *p);
 
 /* Clears a pause (forcing day changed, or a progress point), recording the
@@ -420,6 +424,10 @@ FCAB_API int fcab_run_noalloc(const FcabConfig *cfg, const float *z, const float
  * block sweep's product then packed sum, RN(RN(x*y) + g), rounded twice. */
 FCAB_API int fcab_math_probe(int which, const float *x, const float *y, float *out, long long n,
                              float g);
+
+/* Test hook: leaves in the session's control block what a step leaves whose
+ * row tile did not arrive (see fcab_sim_poll). */
+FCAB_API int fcab_sim_lost_tile_probe(FcabSim *s);
 
 /* Waits, then fills st (computes the LAND volume V). */
 FCAB_API int fcab_sim_stats(FcabSim *s, FcabStats *st);
