@@ -5,6 +5,8 @@
 // and with it into libfloodca_b200_f64.so, matching the caller's build.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -102,24 +104,32 @@ int load_rday(FcaGrid *g, const char *path, real lambda)
 }
 
 // Drives a session to the end of the run, serving pauses: forcing-day
-// reloads, progress lines and the ensemble poll hook.
+// reloads, progress lines and the ensemble poll hook. pause_every: steps
+// between its pauses (fcab_sim_set_pause_every), 0 for none.
 int drive(FcabSim *s, FcaGrid *g, const FcaRunCfg *cfg, FcaAcc *acc, FcaTimers *tm,
-          void (*poll)(void *), void *pctx, int poll_every, double t_wall0)
+          void (*poll)(void *), void *pctx, int poll_every, int pause_every, double t_wall0)
 {
-    int chunk = 32, taken = acc->step;
-    for (;;) {
-        // a run of a fixed number of steps goes out whole (a pause only makes
-        // what was sent past it do nothing)
-        const int left = cfg->steps > 0 ? cfg->steps - taken : 0;
-        const int most = cfg->n_force_days > 0 || poll || cfg->progress_every > 0 ? 256 : 1 << 16;
-        if (fcab_sim_advance(s, left > 0 && left < most ? left : left > 0 ? most : chunk) != 0)
+    FcabPoll p;
+    p.t = acc->t;
+    p.step = acc->step;
+    p.force_day = acc->force_day;
+    const int days = cfg->n_force_days;
+    const auto day_of = [&](double t) { return t < 0.0 ? 0 : std::min((int)(t / FCA_DAY_S), days - 1); };
+    for (int chunk = 32;;) {
+        // where the run ends or pauses for another forcing day, at the earliest
+        // (a run whose first day is not loaded begins with that pause)
+        double t_end = (double)cfg->T_sim;
+        if (days > 0 && day_of(p.t) != p.force_day)
+            t_end = p.t;
+        else if (days > 0 && day_of(p.t) < days - 1)
+            t_end = std::min(t_end, (day_of(p.t) + 1) * FCA_DAY_S);
+        if (fcab_sim_advance(s, fcab_steps_ahead(cfg->steps, p.step, p.t, t_end,
+                                                 (double)cfg->phys.dt_max, pause_every, chunk)) != 0)
             return -2;
-        FcabPoll p;
         if (fcab_sim_poll(s, &p) != 0)
             return -2;
         if (p.done)
             return 0;
-        taken = p.step;
         if (!p.pause) {
             if (chunk < 256)
                 chunk *= 2;
@@ -127,10 +137,8 @@ int drive(FcabSim *s, FcaGrid *g, const FcaRunCfg *cfg, FcaAcc *acc, FcaTimers *
         }
         chunk = 32;
         int day = p.force_day;
-        if (cfg->n_force_days > 0) {
-            int d = p.t < 0.0 ? 0 : (int)(p.t / FCA_DAY_S);
-            if (d >= cfg->n_force_days)
-                d = cfg->n_force_days - 1;
+        if (days > 0) {
+            const int d = day_of(p.t);
             if (d != p.force_day) {
                 const double ti = now_s();
                 if (load_rday(g, cfg->force_files[d], cfg->lambda) != 0) {
@@ -160,6 +168,7 @@ int drive(FcabSim *s, FcaGrid *g, const FcaRunCfg *cfg, FcaAcc *acc, FcaTimers *
         }
         if (fcab_sim_resume(s, day) != 0)
             return -2;
+        p.force_day = day;
     }
 }
 
@@ -238,7 +247,7 @@ extern "C" int fca_cuda_run(FcaGrid *g, FcaRunCfg *cfg, FcaAcc *acc, FcaTimers *
 
     const int step0 = acc->step;
     const double t_wall0 = now_s();
-    int rc = drive(s, g, cfg, acc, tm, nullptr, nullptr, 0, t_wall0);
+    int rc = drive(s, g, cfg, acc, tm, nullptr, nullptr, 0, cfg->progress_every, t_wall0);
     if (rc < 0) {
         report("run");
         fcab_sim_destroy(s);
@@ -332,7 +341,8 @@ extern "C" int fca_cuda_ens_run(FcaCudaEns *e, FcaGrid *g, const FcaRunCfg *cfg,
     tm->t_dt = tm->t_flux = tm->t_limiter = tm->t_update = -1;
     const int step0 = acc->step;
     const double t_wall0 = now_s();
-    const int rc = drive(e->s, g, cfg, acc, tm, poll, pctx, poll_every, t_wall0);
+    const int rc = drive(e->s, g, cfg, acc, tm, poll, pctx, poll_every, poll ? poll_every : 0,
+                         t_wall0);
     if (rc < 0) {
         report("ens_run");
         return -2;

@@ -898,6 +898,8 @@ extern "C" int fcab_sim_reset_time(FcabSim *s, double t, int step, double dt_bas
     c.force_day = force_day;
     c.h_cur = s->h_cur_host;
     s->step0 = step;
+    s->t0 = t;
+    s->stepped = false;
     // all but err, which stands until the fields are uploaded again
     CUDA_TRY(cudaMemcpyAsync(s->ctl, &c, offsetof(Ctl, err), cudaMemcpyHostToDevice, s->stream));
     // V0 = LAND volume of the current depth
@@ -952,6 +954,7 @@ extern "C" int fcab_sim_advance(FcabSim *s, int nsteps)
     int rc = resolve_variant(s);
     if (rc)
         return rc;
+    s->stepped = true;
     if (nsteps >= GRAPH_STEPS) {
         rc = ensure_graph(s);
         if (rc)
@@ -1037,15 +1040,31 @@ extern "C" int fcab_sim_resume(FcabSim *s, int force_day)
     return 0;
 }
 
+extern "C" int fcab_steps_ahead(int max_steps, int step, double t, double t_end, double dt_max,
+                                int pause_every, int chunk)
+{
+    int n = chunk;
+    if (max_steps > 0) {
+        const double sure = (t_end - t) / dt_max;
+        n = std::max(n, sure < 65536.0 ? (int)std::max(sure, 0.0) : 65536);
+        n = std::min(n, max_steps - step);
+    }
+    if (pause_every > 0)
+        n = std::min(n, pause_every - step % pause_every);
+    return std::max(n, 1);
+}
+
 extern "C" int fcab_sim_run(FcabSim *s)
 {
     FcabPoll p;
-    int chunk = GRAPH_STEPS, done_steps = s->step0;
-    for (;;) {
-        // a run of a fixed number of steps goes out whole, whatever it is
-        // (steps past the end do nothing, but cost a launch each)
-        const int left = s->cfg.max_steps > 0 ? s->cfg.max_steps - done_steps : 0;
-        int rc = fcab_sim_advance(s, left > 0 ? std::min(left, 1 << 16) : chunk);
+    p.t = s->t0;
+    p.step = s->step0;
+    if (s->stepped)     // since the clock was set
+        if (int rc = fcab_sim_poll(s, &p))
+            return rc;
+    for (int chunk = GRAPH_STEPS;;) {
+        int rc = fcab_sim_advance(s, fcab_steps_ahead(s->cfg.max_steps, p.step, p.t, s->cfg.T_sim,
+                                                      s->cfg.dt_max, s->tc.progress_every, chunk));
         if (rc)
             return rc;
         rc = fcab_sim_poll(s, &p);
@@ -1055,7 +1074,6 @@ extern "C" int fcab_sim_run(FcabSim *s)
             return 0;
         if (p.pause)
             return fail(FCAB_ERR_STATE, "run paused (forcing or progress); use the drop-in loop");
-        done_steps = p.step;
         if (chunk < 8 * GRAPH_STEPS)
             chunk *= 2;
     }

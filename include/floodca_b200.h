@@ -259,6 +259,14 @@ FCAB_API int fcab_sim_set_rain(FcabSim *s, const void *C, const void *Rday);
  * after the end of the run (T_sim or max_steps) do nothing. */
 FCAB_API int fcab_sim_advance(FcabSim *s, int nsteps);
 
+/* How many steps a run loop sends from (t, step) before it polls again: chunk,
+ * or for a fixed step count (max_steps > 0) as many as are sure to be taken
+ * before t_end, dt_max each at most; no more than are left, nor than there are
+ * to the next pause (pause_every > 0). Steps sent past the end of a run or past
+ * a pause do nothing but cost a launch each: at most chunk of them. */
+FCAB_API int fcab_steps_ahead(int max_steps, int step, double t, double t_end, double dt_max,
+                              int pause_every, int chunk);
+
 /* Runs to the end of the run (T_sim or max_steps) and waits. */
 FCAB_API int fcab_sim_run(FcabSim *s);
 
