@@ -241,8 +241,16 @@ __device__ __noinline__ float pair_velocity(float vm, bool x0, bool x1, f2 mo, f
     return vm;
 }
 
-// hf^(2/3) per half as cbrt_sq2; `unsure` is raised when either half needs
-// the exact scalar function (cbrt_sq_rn).
+// hf^(2/3) = RN(cbrt(hf*hf)) per half, without the exactness fix-up: the
+// cube root u of hf by one Newton step on a log2/exp2 estimate u0
+// (u = u0 - (u0^3 - hf)/(3 u0^2), the residual taken exactly by fused
+// multiply-adds), then u^2 as the float pair s_hi + t, t = s_lo - 2 u0 corr,
+// rounded to y with its rounding error e (Fast2Sum). The value y + e is
+// within about 2^-40 relative of cbrt(hf^2) for hf in [2^-20, 2^20].
+// `unsure` is raised when that is not enough to decide the rounding of either
+// half: |e| within 2^-11 of half an ulp of y (tested as fma(e, 1 + 2^-11, y)
+// != y, which also covers the halved gap below a power of two), or hf outside
+// [2^-20, 2^20]; the caller then evaluates the pair exactly (cbrt_sq_rn).
 __device__ __forceinline__ f2 cbrt_sq2n(f2 hf, bool &unsure)
 {
     const f2 l = lg2_2(hf);

@@ -163,36 +163,4 @@ __device__ __forceinline__ f2 sqrt2_nr(f2 x)
     return fma2(r, h, s);
 }
 
-// hf^(2/3) = RN(cbrt(hf*hf)) per half, without the exactness fix-up: the
-// cube root u of hf by one Newton step on a log2/exp2 estimate u0
-// (u = u0 - (u0^3 - hf)/(3 u0^2), the residual taken exactly by fused
-// multiply-adds), then u^2 as the float pair s_hi + t, t = s_lo - 2 u0 corr,
-// rounded to y with its rounding error e (Fast2Sum). The value y + e is
-// within about 2^-40 relative of cbrt(hf^2) for hf in [2^-20, 2^20].
-// `unsure` (per half) is set when that is not enough to decide the rounding:
-// |e| within 2^-11 of half an ulp of y (tested as fma(e, 1 + 2^-11, y) != y,
-// which also covers the halved gap below a power of two), or hf outside
-// [2^-20, 2^20]; the caller then evaluates those halves exactly.
-__device__ __forceinline__ f2 cbrt_sq2(f2 hf, bool &unsure0, bool &unsure1)
-{
-    const f2 l = lg2_2(hf);
-    const f2 u0 = ex2_2(mul2(l, bc2(0.333333343f)));
-    const f2 s_hi = mul2_sep(u0, u0);
-    const f2 s_lo = fma2(u0, u0, neg2(s_hi));
-    const f2 r1 = fma2(s_hi, u0, neg2(hf));
-    const f2 r = fma2(s_lo, u0, r1);                        // u0^3 - hf
-    const f2 c2 = mul2(r, rcp_2(mul2(bc2(1.5f), s_hi)));    // 2 (u0 - u)
-    const f2 t = fma2(u0, neg2(c2), s_lo);
-    const f2 y = add2(s_hi, t);
-    const f2 e = add2(sub2(s_hi, y), t);
-    const f2 chk = fma2(e, bc2(1.00048828125f), y);
-    float l0, l1, y0, y1, k0, k1;
-    sp2(l, l0, l1);
-    sp2(y, y0, y1);
-    sp2(chk, k0, k1);
-    unsure0 = k0 != y0 || !(fabsf(l0) <= 20.0f);
-    unsure1 = k1 != y1 || !(fabsf(l1) <= 20.0f);
-    return y;
-}
-
 }  // namespace fcab

@@ -1532,15 +1532,33 @@ __global__ void k_math_probe(int which, const float *x, const float *y, float *o
         else if (which == 8)
             r = __fsqrt_rn(x[i]);
         else if (which == 10) {
-            // the block sweep's cube root: its value where it decides the
-            // rounding itself, NaN where it defers to the exact evaluation
-            bool u0, u1;
-            const f2 c = cbrt_sq2(mk2(x[i], x[i]), u0, u1);
-            r = u0 ? __int_as_float(0x7fc00000) : lo2(c);
+            // the block sweep's cube root of the pair (x, y): x's value where it
+            // decides the roundings itself, NaN where it defers to the exact evaluation
+            bool unsure = false;
+            const f2 c = cbrt_sq2n(mk2(x[i], y ? y[i] : x[i]), unsure);
+            r = unsure ? __int_as_float(0x7fc00000) : lo2(c);
         } else if (which == 11) {
             // the block sweep's product then packed sum: two roundings,
             // RN(RN(x*y) + g)
             r = lo2(add2(mul2_sep(mk2(x[i], x[i]), mk2(y[i], y[i])), bc2(g)));
+        } else if (which == 12) {
+            // the block sweep's critical velocity of the pair (y, x), likewise
+            // (each half decides for itself)
+            bool u0, u1;
+            const f2 c = vcrit2(bc2(g), mk2(y ? y[i] : x[i], x[i]), u0, u1);
+            r = u1 ? __int_as_float(0x7fc00000) : hi2(c);
+        } else if (which == 13) {
+            // the block sweep's sqrt(x/g) of a level difference x over a distance g
+            bool unsure = false;
+            r = lo2(blk_face_v<MATH_EXACT>(bc2(x[i]), bc2(0.0f), bc2(0.0f), bc2(0.0f), bc2(1.0f),
+                                           bc2(g), bc2(-__frcp_rn(g)), 0.0f, 0.0f, unsure)
+                        .rs);
+        } else if (which == 14) {
+            // its reciprocal of the mean Manning n x/2, held to 1e-12
+            bool unsure = false;
+            r = lo2(blk_face_v<MATH_EXACT>(bc2(1.0f), bc2(0.0f), bc2(0.0f), bc2(0.0f), bc2(x[i]),
+                                           bc2(1.0f), bc2(-1.0f), 0.0f, 0.0f, unsure)
+                        .v);
         } else
             r = __fdiv_rn(x[i], y[i]);
         out[i] = r;
@@ -1553,6 +1571,9 @@ extern "C" int fcab_math_probe(int which, const float *x, const float *y, float 
     float *dx = nullptr, *dy = nullptr, *dout = nullptr;
     const size_t b = (size_t)n * sizeof(float);
     int rc = 0;
+    if (!x || !out || which < 0 || which > 14 ||
+        (!y && (which == 1 || which == 6 || which == 9 || which == 11)))
+        return fail(FCAB_ERR_ARG, "math_probe: no such function, or no second input");
     if (cudaMalloc(&dx, b) != cudaSuccess || cudaMalloc(&dy, b) != cudaSuccess ||
         cudaMalloc(&dout, b) != cudaSuccess) {
         rc = fail(FCAB_ERR_CUDA, "math_probe alloc");
@@ -1563,7 +1584,7 @@ extern "C" int fcab_math_probe(int which, const float *x, const float *y, float 
         rc = fail(FCAB_ERR_CUDA, "math_probe copy");
         goto done;
     }
-    k_math_probe<<<1024, 256>>>(which, dx, dy, dout, n, g);
+    k_math_probe<<<1024, 256>>>(which, dx, y ? dy : nullptr, dout, n, g);
     if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
         cudaMemcpy(out, dout, b, cudaMemcpyDeviceToHost) != cudaSuccess)
         rc = fail(FCAB_ERR_CUDA, "math_probe run");

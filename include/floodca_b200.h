@@ -427,9 +427,11 @@ FCAB_API int fcab_run_noalloc(const FcabConfig *cfg, const float *z, const float
  * host outputs. which = 0: RN(cbrt(x*x)) as the exact mode computes
  * hf^(2/3); 1: min(x, RN(sqrt(g*y))); 2: the fast-mode hf^(2/3); 4/5/6: the
  * branch-free reciprocal, square root and Markstein quotient x/y; 7/8/9: the
- * IEEE reciprocal, square root and quotient they must equal; 10: the packed
- * block sweep's hf^(2/3), NaN where it defers to the exact evaluation; 11: the
- * block sweep's product then packed sum, RN(RN(x*y) + g), rounded twice. */
+ * IEEE reciprocal, square root and quotient they must equal; and what the block
+ * sweep evaluates: 10: hf^(2/3) of x beside y (NULL: x) in the other half of the
+ * pair, NaN where it defers to the exact evaluation of both; 11: the product
+ * then packed sum RN(RN(x*y) + g), rounded twice; 12: RN(sqrt(g*x)) beside y,
+ * NaN where it defers; 13: RN(sqrt(RN(x/g))); 14: 1 / max(x/2, 1e-12). */
 FCAB_API int fcab_math_probe(int which, const float *x, const float *y, float *out, long long n,
                              float g);
 
