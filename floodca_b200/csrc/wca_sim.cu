@@ -150,7 +150,8 @@ __global__ void k_encode_mask(const uint8_t *m, float *z, float *n, long long pi
 // last row and column, and with a slab's halo rows; SEA cells; values other
 // than LAND, SEA, WALL; whether cell `cell` of the uploaded rows is LAND.
 struct MaskStats {
-    unsigned int land, land_up, sea, other, north, south, west, east, inflow_land;
+    unsigned long long land, land_up, sea, other;
+    unsigned int north, south, west, east, inflow_land;
 };
 
 __global__ void k_mask_stats(const uint8_t *m, long long pitch, int nr, int nc, int hn, int hs,
@@ -180,17 +181,20 @@ __global__ void k_mask_stats(const uint8_t *m, long long pitch, int nr, int nc, 
         if (i == cell && is_land)
             out->inflow_land = 1u;
     }
+    // a warp's counts fit 32 bits (2^40 cells over 4096 warps)
     land = __reduce_add_sync(0xffffffffu, land);
     up = __reduce_add_sync(0xffffffffu, up);
     sea = __reduce_add_sync(0xffffffffu, sea);
     other = __reduce_add_sync(0xffffffffu, other);
     if ((threadIdx.x & 31) == 0) {
-        if (land) atomicAdd(&out->land, land);
-        if (up) atomicAdd(&out->land_up, up);
-        if (sea) atomicAdd(&out->sea, sea);
-        if (other) atomicAdd(&out->other, other);
+        if (land) atomicAdd(&out->land, (unsigned long long)land);
+        if (up) atomicAdd(&out->land_up, (unsigned long long)up);
+        if (sea) atomicAdd(&out->sea, (unsigned long long)sea);
+        if (other) atomicAdd(&out->other, (unsigned long long)other);
     }
 }
+
+constexpr int MASK_STATS_GRID = 512;     // of 256 threads
 
 size_t esize_of(int prec) { return prec == FCAB_PREC_F64 ? 8 : 4; }
 
@@ -694,7 +698,7 @@ static int upload_common(FcabSim *s, const void *z, const void *h, const void *n
     memset(&ms, 0, sizeof(ms));
     static_assert(sizeof(MaskStats) <= 64, "session scratch");
     CUDA_TRY(cudaMemsetAsync(s->scratch, 0, sizeof(MaskStats), s->stream));
-    k_mask_stats<<<512, 256, 0, s->stream>>>(s->m, s->pitch, c.nrows, c.ncols, s->hn, s->hs,
+    k_mask_stats<<<MASK_STATS_GRID, 256, 0, s->stream>>>(s->m, s->pitch, c.nrows, c.ncols, s->hn, s->hs,
                                              c.inflow_cell >= 0 && c.inflow_cell < Nup
                                                  ? c.inflow_cell
                                                  : -1,
@@ -1593,6 +1597,29 @@ done:
     cudaFree(dy);
     cudaFree(dout);
     return rc;
+}
+
+extern "C" int fcab_mask_probe(const uint8_t *mask, long long pitch, int nrows, int ncols,
+                               long long counts[4])
+{
+    MaskStats ms, *d = nullptr;
+    if (!mask || !counts || nrows < 1 || ncols < 1)
+        return fail(FCAB_ERR_ARG, "mask_probe: no mask or an empty grid");
+    CUDA_TRY(cudaMalloc(&d, sizeof(ms)));
+    cudaError_t e = cudaMemset(d, 0, sizeof(ms));
+    if (e == cudaSuccess) {
+        k_mask_stats<<<MASK_STATS_GRID, 256>>>(mask, pitch, nrows, ncols, 0, 0, -1, d);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess)
+        e = cudaMemcpy(&ms, d, sizeof(ms), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    CUDA_TRY(e);
+    counts[0] = (long long)ms.land;
+    counts[1] = (long long)ms.land_up;
+    counts[2] = (long long)ms.sea;
+    counts[3] = (long long)ms.other;
+    return 0;
 }
 
 namespace fcab {

@@ -435,6 +435,13 @@ FCAB_API int fcab_run_noalloc(const FcabConfig *cfg, const float *z, const float
 FCAB_API int fcab_math_probe(int which, const float *x, const float *y, float *out, long long n,
                              float g);
 
+/* Test hook: what an upload counts over its mask, a device array in a session's
+ * padded layout (8 rows above, 4 columns left): LAND cells, the same with halo
+ * rows, SEA cells, and values that are neither LAND, SEA nor WALL. With pitch 0
+ * all rows are one. */
+FCAB_API int fcab_mask_probe(const uint8_t *mask, long long pitch, int nrows, int ncols,
+                             long long counts[4]);
+
 /* Test hook: leaves in the session's control block what a step leaves whose
  * row tile did not arrive (see fcab_sim_poll). */
 FCAB_API int fcab_sim_lost_tile_probe(FcabSim *s);
