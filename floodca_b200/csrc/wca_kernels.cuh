@@ -121,8 +121,6 @@ struct TimeCfg {
     int vseed_on;               // seed the dt pruning (a missed seed needs the full pass)
     int split;                  // slab of a row-split domain: the step control waits for
                                 // the velocity maximum reduced over all slabs
-    int tail_vpass;             // the step kernel itself tail-launches the full velocity
-                                // pass when its seed missed (else the launcher adds it)
 };
 
 // --------------------------------------------------------------------------
@@ -1274,7 +1272,7 @@ __device__ __forceinline__ void step_tail(const GridD<T> &g, const RunK<T> &rk, 
                 // a missed seed defers this step's dt to the full velocity
                 // pass: launched from here into the tail of the stream, so
                 // it runs before the next step and only when needed
-                if (tc.tail_vpass && ctl->need_v) {
+                if (ctl->need_v) {
                     k_init_dt<T, K, MATH><<<VPASS_GRID, 256, 0, cudaStreamTailLaunch>>>(g, rk, tc,
                                                                                       ctl, 1);
                     // where that fails need_v stays set and the host's poll runs the pass

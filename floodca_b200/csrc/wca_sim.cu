@@ -520,7 +520,7 @@ extern "C" int fcab_sim_create(FcabSim **out, const FcabConfig *cfg, void *strea
     tc.time_f32 = p == FCAB_PREC_F32_ALL;
     tc.prec_f64 = p == FCAB_PREC_F64;
     tc.vseed_on = 1;        // seeded dt pruning; a missed seed is settled by the full
-    tc.tail_vpass = 1;      // velocity pass, which the step kernel launches itself
+                            // velocity pass, which the step kernel does or launches itself
     *out = s;
     return 0;
 }
@@ -856,35 +856,18 @@ static void grid_view(FcabSim *s, GridD<T> &g)
     g.tmap = s->L.blk ? static_cast<const CUtensorMap *>(s->tmaps) : nullptr;
 }
 
-// Host launches per step: the step; with seeded dt pruning and no tail
-// launch, also the guarded full velocity pass (it returns at once unless the
-// step deferred its dt). A tail-launched pass runs only when the seed missed
-// (FcabStats.dt_full_passes counts those).
-static int launches_per_step(const FcabSim *s)
-{
-    return s->tc.vseed_on && !s->tc.tail_vpass ? 2 : 1;
-}
-
+// One launch a step; the step itself does or launches the full velocity pass
+// when its seed missed (FcabStats.dt_full_passes counts those).
 static cudaError_t launch_one(FcabSim *s)
 {
-    const int full_grid = 2 * 148 * 4;
-    cudaError_t e;
     if (s->esize == 8) {
         GridD<double> g;
         grid_view(s, g);
-        e = s->L.step(&g, &s->rkd, s->tc, s->ctl, s->split, s->grid, s->stream,
-                      s->L.smem);
-        if (e == cudaSuccess && s->tc.vseed_on && !s->tc.tail_vpass)
-            e = s->L.init(&g, &s->rkd, s->tc, s->ctl, full_grid, s->stream, 1);
-        return e;
+        return s->L.step(&g, &s->rkd, s->tc, s->ctl, s->split, s->grid, s->stream, s->L.smem);
     }
     GridD<float> g;
     grid_view(s, g);
-    e = s->L.step(&g, &s->rkf, s->tc, s->ctl, s->split, s->grid, s->stream,
-                  s->L.smem);
-    if (e == cudaSuccess && s->tc.vseed_on && !s->tc.tail_vpass)
-        e = s->L.init(&g, &s->rkf, s->tc, s->ctl, full_grid, s->stream, 1);
-    return e;
+    return s->L.step(&g, &s->rkf, s->tc, s->ctl, s->split, s->grid, s->stream, s->L.smem);
 }
 
 extern "C" int fcab_sim_reset_time(FcabSim *s, double t, int step, double dt_base, int force_day)
@@ -966,12 +949,12 @@ extern "C" int fcab_sim_advance(FcabSim *s, int nsteps)
     }
     while (nsteps >= GRAPH_STEPS) {
         CUDA_TRY(cudaGraphLaunch(s->graph, s->stream));
-        s->launches += GRAPH_STEPS * launches_per_step(s);
+        s->launches += GRAPH_STEPS;
         nsteps -= GRAPH_STEPS;
     }
     for (; nsteps > 0; nsteps--) {
         CUDA_TRY(launch_one(s));
-        s->launches += launches_per_step(s);
+        s->launches += 1;
     }
     return 0;
 }
@@ -1242,7 +1225,6 @@ extern "C" int fcab_sim_set_config(FcabSim *s, const FcabConfig *cfg)
     tc.U = cfg->U > 0 ? cfg->U : 1;
     tc.inflow_ok = inflow_ok;
     tc.vseed_on = 1;
-    tc.tail_vpass = 1;
     s->cpl = cfg->cols_per_lane ? pick_cpl(*cfg) : keep_cpl;
     s->variant_dirty = true;
     return 0;
