@@ -8,7 +8,7 @@ Outputs (next to this file):
 Run `python -m floodca_b200.build` (or `__graft_entry__.build()`). Objects
 go to _build/ at the repository root. Sources are rebuilt only when newer
 than their object. FCAB_NVCC_FLAGS adds nvcc flags (for example the launch
-shape macro -DFCAB_PAIR_WARPS=12); changing it needs a clean _build/.
+shape macro -DFCAB_BLK_CTAS=3); changing it needs a clean _build/.
 """
 from __future__ import annotations
 

@@ -100,13 +100,6 @@ __device__ __forceinline__ f2 abs2(f2 a)
     r.u = a.u & 0x7fffffff7fffffffull;
     return r;
 }
-// magnitude of a with the sign of s, per half
-__device__ __forceinline__ f2 copysign2(f2 a, f2 s)
-{
-    f2 r;
-    r.u = (a.u & 0x7fffffff7fffffffull) | (s.u & 0x8000000080000000ull);
-    return r;
-}
 __device__ __forceinline__ f2 sel2(bool p0, bool p1, f2 a, f2 b)
 {
     return mk2(p0 ? lo2(a) : lo2(b), p1 ? hi2(a) : hi2(b));
@@ -152,15 +145,6 @@ __device__ __forceinline__ f2 rcp2_nr(f2 x)
     const f2 y = rcp_2(x);
     const f2 e = fma2(neg2(x), y, bc2(1.0f));
     return fma2(e, y, y);
-}
-// RN(sqrt(x)) per half, x normal and positive (see sqrt_nr).
-__device__ __forceinline__ f2 sqrt2_nr(f2 x)
-{
-    const f2 y = rsqrt_2(x);
-    const f2 s = mul2(x, y);
-    const f2 h = mul2(bc2(0.5f), y);
-    const f2 r = fma2(neg2(s), s, x);
-    return fma2(r, h, s);
 }
 
 }  // namespace fcab

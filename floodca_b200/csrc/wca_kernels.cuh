@@ -41,7 +41,7 @@ constexpr int PADR = 8;   // padded rows above and below the grid (a range of
                           // rows starts up to six rows above its first)
 constexpr int PADC = 4;   // padded columns left of the grid
 constexpr int NSLOT = 32; // accumulator slots (spread the atomics)
-constexpr double PAD_Z = 1e30;   // padding elevation of all-LAND grids
+constexpr double PAD_Z = 1e30;   // padding elevation
 
 template <int CPL>
 struct Geom {
@@ -51,8 +51,8 @@ struct Geom {
 };
 
 // Device view of the padded grid. Element (r, c) of the nrows x ncols grid is
-// at index (r + PADR) * pitch + (c + PADC); padding cells are WALL with zero
-// z, h and n.
+// at index (r + PADR) * pitch + (c + PADC); padding cells are WALL with
+// elevation PAD_Z and zero h and n.
 template <typename T>
 struct GridD {
     const T *z, *n, *cr;        // cr: per-cell C*Rday, or nullptr
@@ -1567,7 +1567,7 @@ struct BatchQ {
 };
 
 template <typename T, typename AccT, int K, int CPL, int MATH, bool RAINF, bool LANDONLY>
-__global__ void __launch_bounds__(128, CPL == 2 ? 4 : 1)
+__global__ void __launch_bounds__(128, 1)
 k_step_batch(const MemberD<T> *members,
                                                     const int *unit_member, int total_units,
                                                     BatchQ *q, int *need_list)
