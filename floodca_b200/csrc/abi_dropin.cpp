@@ -105,9 +105,10 @@ int load_rday(FcaGrid *g, const char *path, real lambda)
 
 // Drives a session to the end of the run, serving pauses: forcing-day
 // reloads, progress lines and the ensemble poll hook. pause_every: steps
-// between its pauses (fcab_sim_set_pause_every), 0 for none.
+// between its pauses (fcab_sim_set_pause_every), 0 for none; one_run: the
+// session serves this run alone.
 int drive(FcabSim *s, FcaGrid *g, const FcaRunCfg *cfg, FcaAcc *acc, FcaTimers *tm,
-          void (*poll)(void *), void *pctx, int poll_every, int pause_every, double t_wall0)
+          void (*poll)(void *), void *pctx, int poll_every, int pause_every, bool one_run, double t_wall0)
 {
     FcabPoll p;
     p.t = acc->t;
@@ -123,6 +124,16 @@ int drive(FcabSim *s, FcaGrid *g, const FcaRunCfg *cfg, FcaAcc *acc, FcaTimers *
             t_end = p.t;
         else if (days > 0 && day_of(p.t) < days - 1)
             t_end = std::min(t_end, (day_of(p.t) + 1) * FCA_DAY_S);
+        if (one_run) {
+            // the steps left: at the rate so far, or of dt_max each
+            const double rest = (double)cfg->T_sim - p.t;
+            double left = p.step > acc->step && p.t > acc->t
+                              ? rest * (p.step - acc->step) / (p.t - acc->t)
+                              : rest / (double)cfg->phys.dt_max;
+            if (cfg->steps > 0)
+                left = std::min(left, (double)(cfg->steps - p.step));
+            fcab_sim_expect_steps(s, (long long)std::max(0.0, std::min(left, 1e15)));
+        }
         if (fcab_sim_advance(s, fcab_steps_ahead(cfg->steps, p.step, p.t, t_end,
                                                  (double)cfg->phys.dt_max, pause_every, chunk)) != 0)
             return -2;
@@ -247,7 +258,7 @@ extern "C" int fca_cuda_run(FcaGrid *g, FcaRunCfg *cfg, FcaAcc *acc, FcaTimers *
 
     const int step0 = acc->step;
     const double t_wall0 = now_s();
-    int rc = drive(s, g, cfg, acc, tm, nullptr, nullptr, 0, cfg->progress_every, t_wall0);
+    int rc = drive(s, g, cfg, acc, tm, nullptr, nullptr, 0, cfg->progress_every, true, t_wall0);
     if (rc < 0) {
         report("run");
         fcab_sim_destroy(s);
@@ -342,7 +353,7 @@ extern "C" int fca_cuda_ens_run(FcaCudaEns *e, FcaGrid *g, const FcaRunCfg *cfg,
     const int step0 = acc->step;
     const double t_wall0 = now_s();
     const int rc = drive(e->s, g, cfg, acc, tm, poll, pctx, poll_every, poll ? poll_every : 0,
-                         t_wall0);
+                         false, t_wall0);
     if (rc < 0) {
         report("ens_run");
         return -2;

@@ -57,7 +57,11 @@ constexpr uint32_t BLK_ROW_B = 256;         // bytes of a strip row
 // cell (3809 x 132 masked with a point inflow, two such passes in 169 steps:
 // 15.5 ms a run with a limit of 2^20 cells, 5.6 with the pass launched). One
 // step in a hundred needs it; a kernel that could launch the pass costs 1.3 us
-// more to launch every step and cannot overlap its start with the step before.
+// more to launch every step and cannot overlap its start with the step before,
+// and a graph of such kernels takes 3.5 ms more to build and free. What the
+// grids between pay for that worst case: 300 steps of 733 x 1101 9.9 ms with
+// this limit, 9.1 with 2^20; a call of fca_cuda_run of 400 steps at 1024^2
+// 17.0 ms (20.5 with a graph built for it) against 16.0.
 constexpr long long BLK_SOLO = 1ll << 16;
 
 // Shared memory, in bytes from a 128-byte boundary. Tile stage: rows

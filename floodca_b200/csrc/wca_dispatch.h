@@ -34,6 +34,7 @@ struct Launchers {
     int threads;           // threads per CTA of the step kernel
     int smem;              // dynamic shared memory of the step kernel
     int blk;               // the block sweep: `grid` CTAs share the rows
+    int nested;            // the step kernel holds a device-side launch
 };
 
 // Batched-ensemble launchers (FP32 state, FP64 accumulation).
@@ -119,6 +120,7 @@ Launchers make_launchers()
     L.threads = step_threads<CPL, MATH>();
     L.smem = 0;
     L.blk = 0;
+    L.nested = 1;
     return L;
 }
 
@@ -135,8 +137,9 @@ cudaError_t launch_step_blk(const void *g, const void *rk, const TimeCfg &tc, Ct
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     c.attrs = at;
-    // only where both launches fit on the GPU (two CTAs of each per SM):
-    // measured 3 to 9 % faster up to 512^2, 3 % slower at 733 x 1101
+    // only where both launches fit on the GPU (two CTAs of each per SM of the
+    // B200's 148): measured 3 to 9 % faster up to 512^2, 3 % slower at 733 x
+    // 1101. Kernels that hold a launch (above BLK_SOLO cells) have none.
     c.numAttrs = !TAILV && grid <= 2 * 148 ? 1 : 0;
     return cudaLaunchKernelEx(&c, &k_step_blk<AccT, K, MATH, RAINF, GEN, TAILV>,
                               *static_cast<const GridD<float> *>(g),
@@ -153,6 +156,7 @@ Launchers make_launchers_blk()
     L.threads = BLK_THREADS;
     L.smem = blk_smem_bytes<K>();
     L.blk = 1;
+    L.nested = TAILV;
     return L;
 }
 

@@ -41,6 +41,7 @@ struct FcabSim {
     int step0 = 0;
     double t0 = 0.0;
     bool stepped = false;        // steps were sent since reset_time set t0 and step0
+    long long expect = -1;       // fcab_sim_expect_steps
     double V0 = 0.0;
     long long land_cells = 0, open_faces = 0, faces_per_step = 0;
     // slab of a row-split domain: halo rows above (hn) and below (hs) the

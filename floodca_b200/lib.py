@@ -71,6 +71,7 @@ def core() -> C.CDLL:
         "fcab_sim_rows_get": (C.c_int, [_P, _I, _I, _P]),
         "fcab_sim_rows_put": (C.c_int, [_P, _I, _I, _P]),
         "fcab_sim_destroy": (None, [_P]),
+        "fcab_sim_expect_steps": (C.c_int, [_P, _LL]),
         "fcab_steps_ahead": (C.c_int, [_I, _I, C.c_double, C.c_double, C.c_double, _I, _I]),
         "fcab_mask_probe": (C.c_int, [_P, C.c_longlong, _I, _I, C.POINTER(C.c_longlong)]),
         "fcab_sim_lost_tile_probe": (C.c_int, [_P]),

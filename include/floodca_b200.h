@@ -267,6 +267,10 @@ FCAB_API int fcab_sim_advance(FcabSim *s, int nsteps);
 FCAB_API int fcab_steps_ahead(int max_steps, int step, double t, double t_end, double dt_max,
                               int pause_every, int chunk);
 
+/* About how many steps the session still has to take (negative, the default:
+ * any number): it sends them as graphs only where building one pays. */
+FCAB_API int fcab_sim_expect_steps(FcabSim *s, long long nsteps);
+
 /* Runs to the end of the run (T_sim or max_steps) and waits. */
 FCAB_API int fcab_sim_run(FcabSim *s);
 

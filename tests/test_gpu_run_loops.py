@@ -5,7 +5,7 @@ import ctypes as C
 import pytest
 
 from floodca_b200 import synth
-from floodca_b200.lib import dropin
+from floodca_b200.lib import check, core, dropin
 from floodca_b200.sim import DropinGrid, RunParams, Session
 from oracle import pyoracle
 
@@ -49,6 +49,29 @@ def test_dropin_capped_run_equals_the_run_by_time():
     assert a.run() == 0 and b.run() == 0
     ra, rb = a.result(), b.result()
     assert ra["step"] == rb["step"] and (ra["h"] == rb["h"]).all()
+
+
+@pytest.mark.parametrize("precision,nr,nc", [("f32", 260, 270), ("f64", 70, 65), ("f32", 40, 50)])
+@pytest.mark.parametrize("expect", [-1, 0, 4095, 4096])
+def test_steps_sent_with_and_without_a_graph(precision, nr, nc, expect):
+    """Kernels with a device-side launch (FP32 above 2^16 cells, FP64) and
+    without: sent one by one or as graphs, and changing over in the middle, the
+    run is the same."""
+    dom = synth.make_terrain(synth.TerrainSpec(nr, nc, seed=2))
+    dom.h[:] = 0.02
+    p = RunParams(steps=150, T_sim=1e6)
+    want = pyoracle.run(dom, p, double=precision == "f64")
+    with Session(dom, p, precision=precision) as s:
+        check(core().fcab_sim_expect_steps(s.h, expect), "expect_steps")
+        s.advance(70)
+        check(core().fcab_sim_expect_steps(s.h, 10**6), "expect_steps")
+        s.run()
+        assert s.stats()["step"] == 150
+        h = s.download()[0]
+    if precision == "f32":
+        assert (h == want["h"]).all()
+    else:
+        assert abs(h - want["h"]).max() <= 1e-12
 
 
 @pytest.mark.parametrize("every", [1, 10, 37, 100])
