@@ -59,7 +59,7 @@ def measured_peaks() -> dict:
 
 
 def profile_traffic() -> float | None:
-    """DRAM bytes per k_step launch from the committed ncu summary, if any."""
+    """DRAM bytes per step launch from the committed ncu summary, if any."""
     f = ROOT / "profiles" / "k_step_traffic.json"
     try:
         return float(json.loads(f.read_text())["dram_bytes_per_launch_4096"])
@@ -404,12 +404,13 @@ def main() -> int:
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak or 6650.0, "unit": "GB/s",
             "frac": achieved / (peak or 6650.0), "traffic": profile_traffic(),
             "peak_source": "measured" if peak else "fallback",
-            "bytes_per_cell": bytes_per_cell, "kernel": "k_step",
-            "time": "CUDA events around the timed steps on the session stream: one k_step "
+            "bytes_per_cell": bytes_per_cell,
+            "kernel": "k_step_blk" if info["tma_rows"] else "k_step",
+            "time": "CUDA events around the timed steps on the session stream: one step-kernel "
                     "launch per step; the only other kernel in the region is the full velocity "
-                    "pass that k_step tail-launches on a step whose dt seed missed "
+                    "pass that the step tail-launches when its dt seed missed "
                     "(full_velocity_passes of them, about 0.2 ms each), so achieved "
-                    "understates k_step's own rate by that share",
+                    "understates the step kernel's own rate by that share",
             "full_velocity_passes": int(full_passes)}
 
     out = {"metric": METRIC, "value": value, "unit": "Gcell/s", "n_gpus": world,

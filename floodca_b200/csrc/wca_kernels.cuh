@@ -1334,8 +1334,8 @@ __device__ __forceinline__ T velocity_at(const GridD<T> &g, const RunK<T> &rk, c
 // (TAILV = false) the last CTA does a missed seed's velocity pass itself
 // instead of launching it, and a step starts while the one before it ends:
 // its barriers are set up and its first tiles of z and n on their way before
-// it waits for that one. Measured, us a step: 61 x 93 14.5 -> 9.0, 256^2
-// 18.2 -> 11.1.
+// it waits for that one. Measured, us a step of this sweep without all that and
+// with it: 61 x 93 14.5 and 9.0, 256^2 18.2 and 11.1 (10.5 with what came later).
 template <typename AccT, int K, int MATH, bool RAINF, bool GEN, bool TAILV>
 __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
     k_step_blk(GridD<float> g, RunK<float> rk, TimeCfg tc, Ctl *ctl, int seg)
