@@ -22,7 +22,8 @@ struct VariantKey {
 
 // Type-erased launchers; `g`, `rk` point at GridD<T>/RunK<T> of the variant's T.
 struct Launchers {
-    // split: warps of the whole grid (sweeps by warp), or rows of a unit (block sweep)
+    // split: ranges of a strip, 0 for an even split (sweeps by warp); rows of a
+    // unit (block sweep)
     cudaError_t (*step)(const void *g, const void *rk, const TimeCfg &tc, Ctl *ctl, int split,
                         int grid, cudaStream_t s, int smem);
     // full velocity pass + step control: the first step's dt, or
@@ -92,11 +93,11 @@ bool lookup_f64(const VariantKey &k, Launchers *out);
 
 template <typename T, typename AccT, int K, int CPL, int MATH, bool RAINF, bool LAND>
 cudaError_t launch_step(const void *g, const void *rk, const TimeCfg &tc, Ctl *ctl,
-                        int warps_total, int grid, cudaStream_t s, int smem)
+                        int segs, int grid, cudaStream_t s, int smem)
 {
     k_step<T, AccT, K, CPL, MATH, RAINF, LAND><<<grid, step_threads<CPL, MATH>(), smem, s>>>(
         *static_cast<const GridD<T> *>(g), *static_cast<const RunK<T> *>(rk), tc, ctl,
-        warps_total);
+        segs);
     return cudaGetLastError();
 }
 

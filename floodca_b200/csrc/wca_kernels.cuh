@@ -1480,7 +1480,7 @@ __global__ void __launch_bounds__(BLK_THREADS, blk_ctas_per_sm<K>())
 template <typename T, typename AccT, int K, int CPL, int MATH, bool RAINF, bool LANDONLY>
 __global__ void __launch_bounds__(step_threads<CPL, MATH>(),
                                   step_min_blocks<K, CPL, MATH>()) k_step(GridD<T> g, RunK<T> rk, TimeCfg tc, Ctl *ctl,
-                                              int warps_total)
+                                              int segs)
 {
     using G = Geom<CPL>;
     if (ctl->active == 0)
@@ -1496,45 +1496,42 @@ __global__ void __launch_bounds__(step_threads<CPL, MATH>(),
     __syncwarp();
     StepSums<T, AccT> ss;
 
-    // Rows of a strip cost 6 more at each range's start. A strip cut into equal
-    // ranges, or, where that leaves a longer chain (few warps a strip), one even
-    // split of all rows, whose ranges may lie in two strips (12 more). FP64,
-    // us a step with the even split and with ranges: 511 x 770 80 and 74 (85
-    // with neighbouring ranges in a block), 256 x 256 46 and 41, 16 x 16 39 and
-    // 31, 1000 x 1024 114 and 113. The bound is a row's chain of about 1500
-    // FP64 instructions a warp, not their rate: issue slots are half used.
+    // Rows of a strip cost 6 more at each range's start. A strip is cut into
+    // `segs` equal ranges, or (0), all rows of the strips laid end to end are
+    // split evenly over the warps (row_ranges says when).
     const int nr = g.nr, nc = g.nc;
     const int nstrips = (nc + G::OW - 1) / G::OW;
-    const long long total = (long long)nstrips * nr;
-    const int segs = max(1, min(nr, warps_total / nstrips));
-    const bool even = (total + warps_total - 1) / warps_total + 6 <
-                      (long long)((nr + segs - 1) / segs) * ((nstrips * (long long)segs + warps_total - 1) / warps_total);
-    // positions w0 .. w1 of the strips laid end to end; by ranges, the next of a
-    // warp is warps_total on
-    long long u = wid, w0, w1;
-    const auto range = [&]() {
-        if (even) {
-            w0 = total * u / warps_total;
-            w1 = total * (u + 1) / warps_total;
+    const int warps_total = (int)(gridDim.x * (blockDim.x >> 5));
+    int u = wid;                            // the next range, warps_total apart for a warp
+    int per = 0, more = 0;                  // rows of a range, one more in the first `more`
+    long long w0 = 0, w1 = 0;               // the even split's positions
+    if (segs > 0) {
+        per = nr / segs;
+        more = nr - per * segs;
+    } else {
+        const long long total = (long long)nstrips * nr;
+        w0 = total * wid / warps_total;
+        w1 = total * (wid + 1) / warps_total;
+    }
+    for (;;) {
+        int strip, r0, r1;
+        if (segs > 0) {
+            if (u >= nstrips * segs)
+                break;
+            strip = u / segs;
+            const int q = u - strip * segs;
+            r0 = q * per + min(q, more);
+            r1 = r0 + per + (q < more ? 1 : 0);
+            u += warps_total;
         } else {
-            const long long strip = u / segs;
-            const int q = (int)(u - strip * segs);
-            w0 = strip * nr + (long long)nr * q / segs;
-            w1 = strip * nr + (long long)nr * (q + 1) / segs;
-        }
-    };
-    const long long units = even ? warps_total : (long long)nstrips * segs;
-    if (wid >= warps_total)
-        u = units;
-    for (; u < units; u += warps_total) {
-        range();
-        while (w0 < w1) {
-            const int strip = (int)(w0 / nr);
-            const int r0 = (int)(w0 % nr);
-            const int r1 = (int)min((long long)nr, (long long)r0 + (w1 - w0));
+            if (w0 >= w1)
+                break;
+            strip = (int)(w0 / nr);
+            r0 = (int)(w0 % nr);
+            r1 = (int)min((long long)nr, (long long)r0 + (w1 - w0));
             w0 += r1 - r0;
-            sweep_segment<T, AccT, K, CPL, MATH, RAINF, LANDONLY>(g, rk, sv, strip, r0, r1, lane, ss);
         }
+        sweep_segment<T, AccT, K, CPL, MATH, RAINF, LANDONLY>(g, rk, sv, strip, r0, r1, lane, ss);
     }
 
     publish_sums<T, AccT, RAINF>(ss, sv, ctl, lane, wid & (NSLOT - 1));

@@ -250,6 +250,7 @@ extern "C" int fcab_run_noalloc(const FcabConfig *cfg, const float *z, const flo
     NA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, L.step_fn, L.threads, 0));
     const int wpb = L.threads / 32;
     const int grid = (int)((step_warps(*cfg, key.cpl, nsm, per_sm, wpb) + wpb - 1) / wpb);
+    const int segs = row_ranges(*cfg, key.cpl, (long long)grid * wpb);
 
     if (stats) {   // V0, the LAND volume of the initial depth
         k_volume<float><<<256, 256, 0, s>>>(g, ctl, rk.k.A, vol);
@@ -257,7 +258,7 @@ extern "C" int fcab_run_noalloc(const FcabConfig *cfg, const float *z, const flo
     }
     NA_TRY(L.init(&g, &rk, tc, ctl, nsm * 4, s, 0));
     for (int k = 0; k < cfg->max_steps; k++)
-        NA_TRY(L.step(&g, &rk, tc, ctl, grid * wpb, grid, s, 0));
+        NA_TRY(L.step(&g, &rk, tc, ctl, segs, grid, s, 0));
     k_unpack<<<512, 256, 0, s>>>(g, ctl, h, hmax, tmax);
     NA_TRY(cudaGetLastError());
 

@@ -378,6 +378,22 @@ long long fcab::step_warps(const FcabConfig &c, int cpl, int nsm, int per_sm, in
     return total / max_warps >= 32 ? max_warps : best * strips;
 }
 
+int fcab::row_ranges(const FcabConfig &c, int cpl, long long warps)
+{
+    // Ranges of a strip, unless that leaves a longer chain (few warps a strip)
+    // than the even split, whose ranges may lie in two strips (12 rows more).
+    // FP64, us a step with the even split and with ranges: 511 x 770 80 and 74
+    // (85 with neighbouring ranges in a block), 256 x 256 46 and 41, 16 x 16 39
+    // and 31, 1000 x 1024 114 and 113. The bound is a row's chain of about 1500
+    // FP64 instructions a warp, not their rate: issue slots are half used.
+    const int ow = 32 * cpl - 2 * (cpl == 1 ? 3 : 4);
+    const long long strips = (c.ncols + ow - 1) / ow, nr = c.nrows;
+    const long long segs = std::max(1ll, std::min(nr, warps / strips));
+    const bool even = (strips * nr + warps - 1) / warps + 6 <
+                      ((nr + segs - 1) / segs) * ((strips * segs + warps - 1) / warps);
+    return even ? 0 : (int)segs;
+}
+
 int fcab::blk_seg(const FcabConfig &c, int nsm, int per_sm)
 {
     if (c.seg_rows > 0)
@@ -828,7 +844,7 @@ static int resolve_variant(FcabSim *s)
         s->grid = (int)std::min<long long>(units, (long long)nsm * per_sm);
     } else {
         s->grid = (int)((step_warps(s->cfg, s->cpl, nsm, per_sm, wpb) + wpb - 1) / wpb);
-        s->split = s->grid * wpb;
+        s->split = row_ranges(s->cfg, s->cpl, (long long)s->grid * wpb);
     }
     s->warps_total = s->grid * wpb;
     s->occupancy = per_sm;

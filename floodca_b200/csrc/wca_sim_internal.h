@@ -60,6 +60,9 @@ int pick_cpl(const FcabConfig &c);
 // per_sm CTAs of wpb warps) with segments of cfg.seg_rows rows when set,
 // else an even split, at least 4 rows per warp (wca_sim.cu).
 long long step_warps(const FcabConfig &c, int cpl, int nsm, int per_sm, int wpb);
+// How the row sweep cuts the rows over that many warps: equal ranges per strip,
+// or 0: all strips' rows split evenly.
+int row_ranges(const FcabConfig &c, int cpl, long long warps);
 // Whether a session's fields suit the block sweep: FP32 with row maps, all LAND
 // or with its mask coded in z and n, tau_h > 0, 32-bit element offsets.
 bool runs_block_sweep(const FcabSim *s);
